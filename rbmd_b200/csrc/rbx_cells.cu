@@ -7,13 +7,13 @@
 // sort: atomic histogram, one-block scan, atomic scatter, then a per-cell
 // bitonic sort.  Inside a cell atoms are ordered by a 4x4x4 Morton sub-cell
 // code, then by old index (deterministic), so consecutive atoms are close in
-// space: 32-atom chunks have small bounding boxes for the list builder.
+// space: chunks of them have small bounding boxes for the list builder.
 //
 // The candidate list replaces Estimate/GenerateFullNeighborListOp
-// (src/neighbor_list/src/op/rocm/full_neighbor_list_op.hip.cu:177-288): one
-// warp per 32 centre atoms (one per lane) streams the chunks of the 27
-// stencil cells that survive a bounding-box cull through shared memory and
-// screens them in FP32; only pairs inside a guard band around the cutoff are
+// (src/neighbor_list/src/op/rocm/full_neighbor_list_op.hip.cu:177-288): a
+// block per 32 centre atoms stages the four-atom chunks of the 27 stencil
+// cells that survive a bounding-box cull in shared memory and screens them in
+// FP32; only pairs inside a guard band around the cutoff are
 // settled with the reference's FP64 predicate, so the list is bit-identical
 // (as a set) to the FP64 reference list.  Rows come out in stencil order,
 // then in cell order.
@@ -210,232 +210,397 @@ k_cell_segsort(int ncell, int n, const int* __restrict__ start, const unsigned* 
 }
 
 // ---------------------------------------------------------------------------
-// Candidate list.  Atoms of a cell are cut into 32-atom chunks; chunk k of
-// cell c sits at table index (cell_start[c] >> 5) + c + k, which is unique
-// and needs no scan (the indices of consecutive cells never overlap), and the
-// few indices between two cells are marked empty.  k_chunk_boxes writes each
-// chunk's bounding box, rounded outwards to FP32, and its cell.
+// Candidate list.  A block of eight warps builds the rows of one group of up
+// to 32 consecutive centre atoms of a cell, four atoms a warp.
 //
-// k_full_list runs one warp per chunk of centre atoms, one centre atom per
-// lane.  For each of the 27 stencil cells it culls the cell's chunks against
-// the group's box (directed rounding: a lower bound of the true box distance,
-// so no pair within the cutoff is ever culled), then streams each surviving
-// chunk through a 32-slot shared buffer as {v, |v|^2}, FP32 coordinates
+// The atoms of a cell are also cut into chunks of four (consecutive in the
+// cell's Morton order); chunk k of cell c sits at table index
+// (cell_start[c] >> 2) + c + k, which is unique and needs no scan (the
+// indices of consecutive cells never overlap).  k_chunk_boxes writes each
+// chunk's bounding box, rounded outwards to FP32.  Groups are numbered the
+// same way with 32 in place of four; a group index between two cells has
+// group_cell -1.
+//
+// Level 1: the block culls the chunks of the 27 stencil cells against the
+// box of its centre atoms (directed rounding: a lower bound of the true box
+// distance, so no pair within the cutoff is ever culled); the survivors, in
+// stencil order, are staged in shared memory as {v, |v|^2}, FP32 coordinates
 // relative to the centre cell's centre with the periodic image applied.
-// Lane u tests slot v as |v|^2 - 2 u.v < C - |u|^2: three FMAs per pair.
-// Pairs inside a guard band around the cutoff are settled with the
-// reference's FP64 predicate, so the list equals the FP64 reference list as a
-// set; rows come out in stencil order, then in cell order.
+// Level 2: each warp culls the staged chunks against the box of its own four
+// centre atoms.  Then a lane takes one staged atom (eight chunks an
+// iteration) and tests it against the four centres as |v|^2 - 2 u.v <
+// C - |u|^2: three FMAs per pair.  Pairs inside a guard band around the
+// cutoff are settled with the reference's FP64 predicate, so the list equals
+// the FP64 reference list as a set; hits are appended through a ballot
+// prefix, so rows come out in stencil order, then in cell order.
 //
-// Split rows (RBL engines in the mixed form): a pair whose build distance is
-// certainly at least r_near = r_core + skin cannot come within r_core before
-// the next rebuild (no atom moves more than skin/2 before one), so the fused
-// RBL kernel tests it with its batch hash first.  Such far pairs are written from the end of the
-// row backwards; every other candidate from the front.  count[i] is the
-// number of candidates (above cap: overflow), far[i] the number written to
-// the back; the front holds min(count, cap) - far[i] entries, all written.
+// Split rows (RBL engines): a pair whose build distance is certainly at
+// least r_near = r_core + skin cannot come within r_core before the next
+// rebuild (no atom moves more than skin/2 before one), so the fused RBL
+// kernel tests it with its batch hash first.  Such far pairs are written from
+// the end of the row backwards; every other candidate from the front.
+// count[i] is the number of candidates (above cap: overflow), far[i] the
+// number of far ones; a row that overflows holds some cap of its candidates.
+//
+// Bound by instruction issue.  Four centres a warp and four-atom chunks leave
+// about 1,400 tested slots an atom at rho* = 0.8, cutoff 5.3 (499 hits),
+// against 3,700 when one warp tests 32-atom chunks against 32 centres, one a
+// lane, as an earlier builder did; and a small box fills the chip (that
+// builder ran one warp per 32 atoms through all 27 cells).  Measured, B200,
+// rho* = 0.8, cutoff 5.3, that builder and this one: 200,000 atoms 660 and
+// 456 us (split rows 915 and 600), 20,000 atoms split 214 and 84, 4,000 atoms
+// split 171 and 42.
 // ---------------------------------------------------------------------------
-constexpr int NL_BLOCK = 128;
-constexpr int NL_WARPS = NL_BLOCK / 32;
+constexpr int NL_WARPS = 8;                // warps of a block
+constexpr int NL_BLOCK = 32 * NL_WARPS;
+constexpr int NL_CH = 4;                   // atoms of a chunk, centre atoms of a warp
+constexpr int NL_GROUP = NL_CH * NL_WARPS; // centre atoms of a block
+constexpr int NL_BATCH = 448;              // chunks staged at a time
+constexpr int NL_WORDS = 256;              // 32-chunk cull words handled at a time
 
-__device__ __forceinline__ int chunk_base(int c, int cs) { return (cs >> 5) + c; }
+__device__ __forceinline__ int chunk_base(int c, int cs) { return cs / NL_CH + c; }
+__device__ __forceinline__ int group_base(int c, int cs) { return cs / NL_GROUP + c; }
 
-int full_list_table_size(int n, int ncell) { return (n >> 5) + ncell; }
+static size_t full_list_groups(int n, int ncell) { return (size_t)(n / NL_GROUP) + ncell; }
+static size_t full_list_chunks(int n, int ncell) { return (size_t)(n / NL_CH) + ncell; }
+
+// Device scratch of one list build.
+struct ListTables {
+  float4* rel;      // per atom: FP32 position relative to its cell's centre
+  float4 *lo, *hi;  // per chunk: its box relative to its cell's centre, rounded outwards
+  int* group_cell;  // per group: its cell, -1 for an index between two cells
+};
 
 __global__ void __launch_bounds__(128)
-k_chunk_boxes(const double* __restrict__ x, const double* __restrict__ y,
-              const double* __restrict__ z, const int* __restrict__ cell_start,
-              float4* __restrict__ box_lo, float4* __restrict__ box_hi, int* __restrict__ cell_of) {
+k_chunk_boxes(DBox b, int dimx, int dimy, int dimz, const double* __restrict__ x,
+              const double* __restrict__ y, const double* __restrict__ z,
+              const int* __restrict__ cell_start, ListTables T) {
   const int c = blockIdx.x;
   const int cs = cell_start[c], ce = cell_start[c + 1];
-  const int nch = (ce - cs + 31) >> 5;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int base = chunk_base(c, cs);
-  for (int k = warp; k < nch; k += 4) {
-    const int a = cs + 32 * k + lane;
+  const int cz = c / (dimx * dimy), cy = (c / dimx) % dimy, cx = c % dimx;
+  const double o[3] = {b.lo[0] + (cx + 0.5) * (b.len[0] / dimx),
+                       b.lo[1] + (cy + 0.5) * (b.len[1] / dimy),
+                       b.lo[2] + (cz + 0.5) * (b.len[2] / dimz)};
+  // a lane an atom, a chunk four neighbouring lanes
+  for (int a0 = cs; a0 < ce; a0 += blockDim.x) {
+    const int a = a0 + threadIdx.x;
     const bool ok = a < ce;
+    const double p[3] = {ok ? x[a] : 0.0, ok ? y[a] : 0.0, ok ? z[a] : 0.0};
     float lo[3], hi[3];
-    const double* p[3] = {x, y, z};
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      const double v = ok ? p[d][a] : 0.0;
-      lo[d] = ok ? __double2float_rd(v) : INFINITY;
-      hi[d] = ok ? __double2float_ru(v) : -INFINITY;
-    }
+      lo[d] = ok ? __double2float_rd(__dsub_rd(p[d], o[d])) : INFINITY;
+      hi[d] = ok ? __double2float_ru(__dsub_ru(p[d], o[d])) : -INFINITY;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-        hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+      for (int s = 1; s < NL_CH; s <<= 1) {
+        lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], s));
+        hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], s));
       }
-    if (lane == 0) {
-      box_lo[base + k] = make_float4(lo[0], lo[1], lo[2], 0.f);
-      box_hi[base + k] = make_float4(hi[0], hi[1], hi[2], 0.f);
-      cell_of[base + k] = c;
+    }
+    if (!ok) continue;
+    T.rel[a] = make_float4((float)(p[0] - o[0]), (float)(p[1] - o[1]), (float)(p[2] - o[2]), 0.f);
+    if (threadIdx.x % NL_CH == 0) {
+      const int k = base + (a - cs) / NL_CH;
+      T.lo[k] = make_float4(lo[0], lo[1], lo[2], 0.f);
+      T.hi[k] = make_float4(hi[0], hi[1], hi[2], 0.f);
     }
   }
-  const int next = chunk_base(c + 1, ce);  // first index of the next cell
-  for (int t = base + nch + threadIdx.x; t < next; t += blockDim.x) cell_of[t] = -1;
+  const int g0 = group_base(c, cs), ng = (ce - cs + NL_GROUP - 1) / NL_GROUP;
+  const int g1 = group_base(c + 1, ce);  // first index of the next cell
+  for (int g = g0 + threadIdx.x; g < g1; g += blockDim.x) T.group_cell[g] = g < g0 + ng ? c : -1;
 }
+
+// A store under a predicate, without a branch around it.
+__device__ __forceinline__ void store_if(bool take, int* p, int v) {
+  asm volatile(
+      "{\n\t.reg .pred t;\n\tsetp.ne.u32 t, %0, 0;\n\t@t st.global.u32 [%1], %2;\n\t}" ::"r"(
+          (unsigned)take),
+      "l"(p), "r"(v)
+      : "memory");
+}
+
+struct FullListSmem {
+  float4 atom[(NL_BATCH + 1) * NL_CH];  // staged chunks; the last one is empty
+  float2 bx[NL_BATCH], by[NL_BATCH], bz[NL_BATCH];  // {lo, hi} of a staged chunk
+  int first[NL_BATCH + 1];              // its first atom
+  unsigned short meta[NL_BATCH];        // stencil cell | atoms << 8
+  unsigned short pick[NL_WARPS][NL_BATCH + 8];  // a warp's surviving chunks
+  float4 shift[27];                     // centre of a stencil cell's image, relative to the
+  float shl[27][3], shh[27][3];         // centre cell's; and rounded down and up
+  int cs[27], ce[27], cb[27];           // atom range and first chunk index of a stencil cell
+  int word0[28];                        // first cull word of a stencil cell
+  unsigned mask[NL_WORDS];              // surviving chunks of a word
+  int off[NL_WORDS + 1];                // survivors before it
+};
 
 // SPLIT: RBL rows with a far segment; without it (Verlet lists) no far test.
 template <bool SPLIT>
-__global__ void __launch_bounds__(NL_BLOCK, 5)
+__global__ void __launch_bounds__(NL_BLOCK, 4)
 k_full_list(DBox b, int dimx, int dimy, int dimz, double cut2, float cut2_up, float lo_band,
-            float hi_band, int nidx, const double* __restrict__ x, const double* __restrict__ y,
-            const double* __restrict__ z, const int* __restrict__ cell_start,
-            const float4* __restrict__ box_lo, const float4* __restrict__ box_hi,
-            const int* __restrict__ cell_of, int cap, int* __restrict__ count,
-            int* __restrict__ nbrs, int* __restrict__ overflow, float near2,
-            int* __restrict__ far, long long* __restrict__ total) {
-  __shared__ float4 buf[NL_WARPS][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int w = blockIdx.x * NL_WARPS + warp;
-  if (w >= nidx) return;
-  const int c = cell_of[w];
+            float hi_band, const double* __restrict__ x, const double* __restrict__ y,
+            const double* __restrict__ z, const int* __restrict__ cell_start, ListTables T,
+            int cap, int* __restrict__ count, int* __restrict__ nbrs, int* __restrict__ overflow,
+            float near2, int* __restrict__ far, long long* __restrict__ total) {
+  extern __shared__ __align__(16) unsigned char s_list[];
+  FullListSmem& S = *reinterpret_cast<FullListSmem*>(s_list);
+  const int c = T.group_cell[blockIdx.x];
   if (c < 0) return;  // an index between two cells
+  // the warp's index through a shuffle, so that the compiler knows the loops
+  // below to be uniform over the warp
+  const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+  const unsigned lt = (1u << lane) - 1u;
   const int cs = cell_start[c], ce = cell_start[c + 1];
-  const int g = w - chunk_base(c, cs);
-  const int cz = c / (dimx * dimy), cy = (c / dimx) % dimy, cx = c % dimx;
-  const double ox = b.lo[0] + (cx + 0.5) * (b.len[0] / dimx);
-  const double oy = b.lo[1] + (cy + 0.5) * (b.len[1] / dimy);
-  const double oz = b.lo[2] + (cz + 0.5) * (b.len[2] / dimz);
-  const bool live = cs + g * 32 + lane < ce;
-  const int i = live ? cs + g * 32 + lane : cs + g * 32;
-  const double xi = x[i], yi = y[i], zi = z[i];
-  const float ux = (float)(xi - ox), uy = (float)(yi - oy), uz = (float)(zi - oz);
-  const float uu = fmaf(ux, ux, fmaf(uy, uy, uz * uz));
-  const float ax = live ? -2.f * ux : 0.f, ay = live ? -2.f * uy : 0.f,
-              az = live ? -2.f * uz : 0.f;
-  const float lo_i = live ? lo_band - uu : -INFINITY;
-  const float hi_i = live ? hi_band - uu : -INFINITY;
-  // far pairs: d above this
-  const float near_i = live ? near2 - uu : INFINITY;
-  // box of the group's centre atoms relative to the cell centre, rounded outwards
-  float glo[3], ghi[3];
-  {
-    const double p[3] = {xi, yi, zi}, o[3] = {ox, oy, oz};
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      glo[d] = live ? __double2float_rd(__dsub_rd(p[d], o[d])) : INFINITY;
-      ghi[d] = live ? __double2float_ru(__dsub_ru(p[d], o[d])) : -INFINITY;
-    }
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1)
+  const int g = (int)blockIdx.x - group_base(c, cs);
+  const int i0 = cs + NL_GROUP * g + NL_CH * warp;  // this warp's first centre atom
+  if (warp == 0) {  // the stencil cells, and their cull words
+    const int cz = c / (dimx * dimy), cy = (c / dimx) % dimy, cx = c % dimx;
+    int words = 0;
+    if (lane < 27) {
+      // stencil order of ComputeFullNeighborStencilCellOnTheFly:
+      // offsets (s%3-1, (s/3)%3-1, s/9-1); the image's centre lies that many
+      // cell edges away
+      const int o[3] = {lane % 3 - 1, (lane / 3) % 3 - 1, lane / 9 - 1};
+      const int dim[3] = {dimx, dimy, dimz}, at[3] = {cx + o[0], cy + o[1], cz + o[2]};
+      int w[3];
+      float sh[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        glo[d] = fminf(glo[d], __shfl_xor_sync(0xffffffffu, glo[d], s));
-        ghi[d] = fmaxf(ghi[d], __shfl_xor_sync(0xffffffffu, ghi[d], s));
+        w[d] = at[d] < 0 ? at[d] + dim[d] : (at[d] >= dim[d] ? at[d] - dim[d] : at[d]);
+        const double e = o[d] * (b.len[d] / dim[d]);
+        sh[d] = (float)e;
+        // one FP64 rounding of the edge and of the two centres: 4 ulp of the
+        // box's extent cover them
+        const double slack = 1e-15 * (fabs(b.lo[d]) + b.len[d]);
+        S.shl[lane][d] = __double2float_rd(__dsub_rd(e, slack));
+        S.shh[lane][d] = __double2float_ru(__dadd_ru(e, slack));
       }
-  }
-  int cnt = 0, nback = 0;  // candidates found, entries written to the back
-  int* row = nbrs + (size_t)i * cap;
-  for (int s = 0; s < 27; ++s) {
-    // stencil order of ComputeFullNeighborStencilCellOnTheFly:
-    // offsets (s%3-1, (s/3)%3-1, s/9-1)
-    int nx = cx + s % 3 - 1, ny = cy + (s / 3) % 3 - 1, nz = cz + s / 9 - 1;
-    double shx = 0.0, shy = 0.0, shz = 0.0;
-    if (nx < 0) { nx += dimx; shx = -b.len[0]; } else if (nx >= dimx) { nx -= dimx; shx = b.len[0]; }
-    if (ny < 0) { ny += dimy; shy = -b.len[1]; } else if (ny >= dimy) { ny -= dimy; shy = b.len[1]; }
-    if (nz < 0) { nz += dimz; shz = -b.len[2]; } else if (nz >= dimz) { nz -= dimz; shz = b.len[2]; }
-    const int nc = (nz * dimy + ny) * dimx + nx;
-    const int ncs = cell_start[nc], nce = cell_start[nc + 1];
-    const int nch = (nce - ncs + 31) >> 5;
-    const int nb = chunk_base(nc, ncs);
-    const double dx = shx - ox, dy = shy - oy, dz = shz - oz;
-    const double dxl = __dsub_rd(shx, ox), dyl = __dsub_rd(shy, oy), dzl = __dsub_rd(shz, oz);
-    const double dxh = __dsub_ru(shx, ox), dyh = __dsub_ru(shy, oy), dzh = __dsub_ru(shz, oz);
-    for (int kb = 0; kb < nch; kb += 32) {
-      bool near = false;
-      if (kb + lane < nch) {  // lower bound of the box-box distance
-        const float4 bl = box_lo[nb + kb + lane], bh = box_hi[nb + kb + lane];
-        const float clx = __double2float_rd(__dadd_rd((double)bl.x, dxl));
-        const float cly = __double2float_rd(__dadd_rd((double)bl.y, dyl));
-        const float clz = __double2float_rd(__dadd_rd((double)bl.z, dzl));
-        const float chx = __double2float_ru(__dadd_ru((double)bh.x, dxh));
-        const float chy = __double2float_ru(__dadd_ru((double)bh.y, dyh));
-        const float chz = __double2float_ru(__dadd_ru((double)bh.z, dzh));
-        const float gx = fmaxf(0.f, fmaxf(__fsub_rd(clx, ghi[0]), __fsub_rd(glo[0], chx)));
-        const float gy = fmaxf(0.f, fmaxf(__fsub_rd(cly, ghi[1]), __fsub_rd(glo[1], chy)));
-        const float gz = fmaxf(0.f, fmaxf(__fsub_rd(clz, ghi[2]), __fsub_rd(glo[2], chz)));
-        const float d2 = __fadd_rd(__fadd_rd(__fmul_rd(gx, gx), __fmul_rd(gy, gy)), __fmul_rd(gz, gz));
-        near = d2 < cut2_up;
-      }
-      unsigned m = __ballot_sync(0xffffffffu, near);
-      while (m) {
-        const int k = kb + __ffs(m) - 1;
-        m &= m - 1;
-        const int first = ncs + 32 * k;
-        float4 v = make_float4(0.f, 0.f, INFINITY, INFINITY);  // empty slot: never a hit
-        if (first + lane < nce) {
-          const int a = first + lane;
-          v.x = (float)(x[a] + dx);
-          v.y = (float)(y[a] + dy);
-          v.z = (float)(z[a] + dz);
-          v.w = fmaf(v.x, v.x, fmaf(v.y, v.y, v.z * v.z));
-        }
-        __syncwarp();  // the previous chunk's readers are done
-        buf[warp][lane] = v;
-        __syncwarp();
-        unsigned acc = 0, maybe = 0, farm = 0;  // farm: build distance certainly >= r_near
+      S.shift[lane] = make_float4(sh[0], sh[1], sh[2], 0.f);
+      const int nc = (w[2] * dimy + w[1]) * dimx + w[0];
+      S.cs[lane] = cell_start[nc];
+      S.ce[lane] = cell_start[nc + 1];
+      S.cb[lane] = chunk_base(nc, S.cs[lane]);
+      words = (S.ce[lane] - S.cs[lane] + 32 * NL_CH - 1) / (32 * NL_CH);
+    }
+    int incl = words;
 #pragma unroll
-        for (int t = 0; t < 32; ++t) {
-          const float4 q = buf[warp][t];  // broadcast
-          const float d = fmaf(ax, q.x, fmaf(ay, q.y, fmaf(az, q.z, q.w)));
-          acc |= d < lo_i ? 1u << t : 0u;
-          maybe |= d < hi_i ? 1u << t : 0u;
-          if (SPLIT) farm |= d > near_i ? 1u << t : 0u;
-        }
-        if (nc == c && k == g) {  // the centre atom itself
-          acc &= ~(1u << lane);
-          maybe &= ~(1u << lane);
-        }
-        unsigned unsure = maybe & ~acc;
-        if (__any_sync(0xffffffffu, unsure != 0)) {  // rare: the FP64 predicate decides
-          while (unsure) {
-            const int t = __ffs(unsure) - 1;
-            unsure &= unsure - 1;
-            const int j = first + t;
-            if (dist2_list(b, xi, yi, zi, x[j], y[j], z[j]) < cut2) acc |= 1u << t;
-          }
-        }
-        if (cnt + __popc(acc) <= cap) {
-          // every hit of the chunk fits: next front and back slots as offsets,
-          // the counts recovered after the loop
-          int foff = cnt - nback, boff = cap - 1 - nback;
-          while (acc) {  // hits in cell order, each lane into its own row
-            const int t = __ffs(acc) - 1;
-            acc &= acc - 1;
-            const bool to_back = SPLIT && ((farm >> t) & 1u);
-            row[to_back ? boff : foff] = first + t;
-            boff -= to_back;
-            foff += !to_back;
-          }
-          nback = cap - 1 - boff;
-          cnt = foff + nback;
-        }
-        while (acc) {  // the row fills up: stop storing at cap entries
-          const int t = __ffs(acc) - 1;
-          acc &= acc - 1;
-          // one store to the front or the back of the row (no branch)
-          const bool to_back = SPLIT && ((farm >> t) & 1u);
-          if (cnt < cap) row[to_back ? cap - 1 - nback : cnt - nback] = first + t;
-          nback += (cnt < cap) & to_back;
-          ++cnt;
-        }
+    for (int k = 1; k < 32; k <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, k);
+      if (lane >= k) incl += t;
+    }
+    if (lane < 27) S.word0[lane + 1] = incl;
+    if (lane == 0) S.word0[0] = 0;
+  }
+  if (threadIdx.x < NL_CH) S.atom[NL_BATCH * NL_CH + threadIdx.x] =
+      make_float4(0.f, 0.f, 0.f, INFINITY);  // an empty slot: never a hit
+  if (threadIdx.x == NL_CH) S.first[NL_BATCH] = 0;
+  // this warp's centres i0 + q: their tests and their box (it is their chunk's)
+  float ax[NL_CH], ay[NL_CH], az[NL_CH], lo_i[NL_CH], hi_i[NL_CH], near_i[NL_CH];
+#pragma unroll
+  for (int q = 0; q < NL_CH; ++q) {
+    const bool live = i0 + q < ce;
+    const float4 u = T.rel[live ? i0 + q : cs];
+    const float uu = fmaf(u.x, u.x, fmaf(u.y, u.y, u.z * u.z));
+    ax[q] = live ? -2.f * u.x : 0.f;
+    ay[q] = live ? -2.f * u.y : 0.f;
+    az[q] = live ? -2.f * u.z : 0.f;
+    lo_i[q] = live ? lo_band - uu : -INFINITY;
+    hi_i[q] = live ? hi_band - uu : -INFINITY;
+    near_i[q] = near2 - uu;  // far pairs: d above this
+  }
+  const int own = chunk_base(c, cs) + (int)NL_WARPS * g;  // the group's first chunk
+  float ulo[3], uhi[3], glo[3], ghi[3];                   // boxes of the group, of the warp
+  {
+    const bool ok = lane < NL_WARPS && cs + NL_GROUP * g + NL_CH * lane < ce;
+    const float4 l = T.lo[ok ? own + lane : own], h = T.hi[ok ? own + lane : own];
+    const float ll[3] = {l.x, l.y, l.z}, hh[3] = {h.x, h.y, h.z};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      glo[d] = __shfl_sync(0xffffffffu, ll[d], warp);
+      ghi[d] = __shfl_sync(0xffffffffu, hh[d], warp);
+      ulo[d] = ll[d];  // lanes without a chunk repeat the first
+      uhi[d] = hh[d];
+#pragma unroll
+      for (int s = 1; s < NL_WARPS; s <<= 1) {
+        ulo[d] = fminf(ulo[d], __shfl_xor_sync(0xffffffffu, ulo[d], s));
+        uhi[d] = fmaxf(uhi[d], __shfl_xor_sync(0xffffffffu, uhi[d], s));
       }
+      ulo[d] = __shfl_sync(0xffffffffu, ulo[d], 0);
+      uhi[d] = __shfl_sync(0xffffffffu, uhi[d], 0);
     }
   }
-  if (live) {
-    count[i] = cnt;
-    if (SPLIT) far[i] = nback;
-    if (cnt > cap) atomicOr(overflow, 1);
+  int nfront[NL_CH], nback[NL_CH];
+#pragma unroll
+  for (int q = 0; q < NL_CH; ++q) nfront[q] = nback[q] = 0;
+  int* const row = nbrs + (size_t)i0 * cap;  // NL_CH rows, back to back
+  __syncthreads();
+
+  // the box of chunk k of stencil cell s relative to the centre cell's centre
+  auto chunk_box = [&](int s, int k, float rl[3], float rh[3]) {
+    const float4 bl = T.lo[S.cb[s] + k], bh = T.hi[S.cb[s] + k];
+    const float l[3] = {bl.x, bl.y, bl.z}, h[3] = {bh.x, bh.y, bh.z};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      rl[d] = __fadd_rd(l[d], S.shl[s][d]);
+      rh[d] = __fadd_ru(h[d], S.shh[s][d]);
+    }
+  };
+  // lower bound of the squared distance of boxes [al, ah] and [bl, bh]
+  auto gap2 = [](const float al[3], const float ah[3], const float bl[3], const float bh[3]) {
+    float e[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      e[d] = fmaxf(0.f, fmaxf(__fsub_rd(bl[d], ah[d]), __fsub_rd(al[d], bh[d])));
+    return __fadd_rd(__fadd_rd(__fmul_rd(e[0], e[0]), __fmul_rd(e[1], e[1])),
+                     __fmul_rd(e[2], e[2]));
+  };
+  // stencil cell of cull word w
+  auto word_cell = [&](int w) {
+    return __popc(__ballot_sync(0xffffffffu, lane < 27 && S.word0[min(lane, 27)] <= w)) - 1;
+  };
+
+  const int nwords = S.word0[27];
+  for (int wb = 0; wb < nwords; wb += NL_WORDS) {
+    const int nw = min(NL_WORDS, nwords - wb);
+    for (int w = warp; w < nw; w += NL_WARPS) {  // level 1
+      const int s = word_cell(wb + w);
+      const int k = (wb + w - S.word0[s]) * 32 + lane;
+      bool near = false;
+      if (k * NL_CH < S.ce[s] - S.cs[s]) {
+        float rl[3], rh[3];
+        chunk_box(s, k, rl, rh);
+        near = gap2(ulo, uhi, rl, rh) < cut2_up;
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, near);
+      if (lane == 0) S.mask[w] = m;
+    }
+    __syncthreads();
+    if (warp == 0) {  // survivors before each word
+      int carry = 0;
+      for (int w0 = 0; w0 < nw; w0 += 32) {
+        const int v = w0 + lane < nw ? __popc(S.mask[w0 + lane]) : 0;
+        int incl = v;
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, incl, k);
+          if (lane >= k) incl += t;
+        }
+        if (w0 + lane < nw) S.off[w0 + lane] = carry + incl - v;
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+      }
+      if (lane == 0) S.off[nw] = carry;
+    }
+    __syncthreads();
+    const int found = S.off[nw];
+    for (int b0 = 0; b0 < found; b0 += NL_BATCH) {
+      const int nb = min(NL_BATCH, found - b0);
+      for (int w = warp; w < nw; w += NL_WARPS) {  // the batch's chunks
+        if (S.off[w + 1] <= b0 || S.off[w] >= b0 + NL_BATCH) continue;
+        const int s = word_cell(wb + w);
+        const unsigned m = S.mask[w];
+        const int slot = S.off[w] + __popc(m & lt) - b0;
+        if (((m >> lane) & 1u) && slot >= 0 && slot < NL_BATCH) {
+          const int k = (wb + w - S.word0[s]) * 32 + lane;
+          float rl[3], rh[3];
+          chunk_box(s, k, rl, rh);
+          S.bx[slot] = make_float2(rl[0], rh[0]);
+          S.by[slot] = make_float2(rl[1], rh[1]);
+          S.bz[slot] = make_float2(rl[2], rh[2]);
+          const int a = S.cs[s] + NL_CH * k;
+          S.first[slot] = a;
+          S.meta[slot] = (unsigned short)(s | min(NL_CH, S.ce[s] - a) << 8);
+        }
+      }
+      __syncthreads();
+#pragma unroll 4
+      for (int t = threadIdx.x; t < nb * NL_CH; t += NL_BLOCK) {  // its atoms
+        const int slot = t / NL_CH, u = t % NL_CH;
+        const int meta = S.meta[slot];
+        const float4 sh = S.shift[meta & 255];
+        float4 v = make_float4(0.f, 0.f, 0.f, INFINITY);
+        if (u < meta >> 8) {
+          const float4 r = T.rel[S.first[slot] + u];
+          v.x = r.x + sh.x;
+          v.y = r.y + sh.y;
+          v.z = r.z + sh.z;
+          v.w = fmaf(v.x, v.x, fmaf(v.y, v.y, v.z * v.z));
+        }
+        S.atom[t] = v;
+      }
+      __syncthreads();
+      if (i0 < ce) {
+        unsigned short* const pick = S.pick[warp];
+        int np = 0;
+        for (int k0 = 0; k0 < nb; k0 += 32) {  // level 2
+          const int k = min(k0 + lane, nb - 1);
+          const float2 vx = S.bx[k], vy = S.by[k], vz = S.bz[k];
+          const float rl[3] = {vx.x, vy.x, vz.x}, rh[3] = {vx.y, vy.y, vz.y};
+          const bool near = (gap2(glo, ghi, rl, rh) < cut2_up) & (k0 + lane < nb);
+          const unsigned m = __ballot_sync(0xffffffffu, near);
+          if (near) pick[np + __popc(m & lt)] = (unsigned short)k;
+          np += __popc(m);
+        }
+        if (lane < 8) pick[np + lane] = NL_BATCH;  // pad with the empty chunk
+        __syncwarp();
+        const int u = lane % NL_CH;
+        for (int t = 0; t < np; t += 32 / NL_CH) {
+          const int ch = pick[t + lane / NL_CH];
+          const float4 v = S.atom[ch * NL_CH + u];
+          const int j = S.first[ch] + u;
+          float d[NL_CH];
+          bool in[NL_CH];
+          // the warp's own chunk (its lanes meet themselves) and pairs in the
+          // guard band are settled one by one
+          bool odd = (unsigned)(j - i0) < (unsigned)NL_CH;
+#pragma unroll
+          for (int q = 0; q < NL_CH; ++q) {
+            d[q] = fmaf(ax[q], v.x, fmaf(ay[q], v.y, fmaf(az[q], v.z, v.w)));
+            in[q] = d[q] < lo_i[q];
+            odd |= in[q] ^ (d[q] < hi_i[q]);
+          }
+          if (__any_sync(0xffffffffu, odd)) {
+#pragma unroll
+            for (int q = 0; q < NL_CH; ++q) {
+              const int i = i0 + q;
+              if (in[q] != (d[q] < hi_i[q]))  // the FP64 predicate decides
+                in[q] = dist2_list(b, x[i], y[i], z[i], x[j], y[j], z[j]) < cut2;
+              in[q] = in[q] && j != i;
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < NL_CH; ++q) {
+            if (SPLIT) {
+              const bool bk = in[q] & (d[q] > near_i[q]);
+              const unsigned mb = __ballot_sync(0xffffffffu, bk);
+              const unsigned mf = __ballot_sync(0xffffffffu, in[q]) ^ mb;
+              const int pos = (bk ? nback[q] : nfront[q]) + __popc((bk ? mb : mf) & lt);
+              store_if(in[q] & (pos < cap), row + (q * cap + (bk ? cap - 1 - pos : pos)), j);
+              nback[q] += __popc(mb);
+              nfront[q] += __popc(mf);
+            } else {
+              const unsigned m = __ballot_sync(0xffffffffu, in[q]);
+              const int pos = nfront[q] + __popc(m & lt);
+              store_if(in[q] & (pos < cap), row + (q * cap + pos), j);
+              nfront[q] += __popc(m);
+            }
+          }
+        }
+      }
+      __syncthreads();  // the next batch overwrites this one
+    }
   }
-  if (total) {  // the warp's rows (cnt is 0 on lanes without a centre atom)
-    const int s = __reduce_add_sync(0xffffffffu, cnt);
-    if (lane == 0) atomicAdd((unsigned long long*)total, (unsigned long long)s);
+  int sum = 0;
+#pragma unroll
+  for (int q = 0; q < NL_CH; ++q) {
+    const int n = nfront[q] + nback[q];
+    if (i0 + q < ce && lane == q) {
+      count[i0 + q] = n;
+      if (SPLIT) far[i0 + q] = nback[q];
+      if (n > cap) atomicOr(overflow, 1);
+    }
+    sum += n;
   }
+  if (total && lane == 0 && i0 < ce) atomicAdd((unsigned long long*)total, (unsigned long long)sum);
 }
 
 // ---------------------------------------------------------------------------
@@ -795,10 +960,17 @@ int launch_cells_sort(const DBox& b, const int dims[3], int n, const double* x, 
   return check_launch("cells_sort");
 }
 
-size_t full_list_scratch_bytes(int n, int ncell) {
-  const size_t t = (size_t)full_list_table_size(n, ncell);
+static size_t list_pieces(int n, int ncell, size_t piece[4]) {
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
-  return al(sizeof(float4) * t) * 2 + al(sizeof(int) * t);
+  piece[0] = al(sizeof(float4) * (size_t)n);
+  piece[1] = piece[2] = al(sizeof(float4) * full_list_chunks(n, ncell));
+  piece[3] = al(sizeof(int) * full_list_groups(n, ncell));
+  return piece[0] + piece[1] + piece[2] + piece[3];
+}
+
+size_t full_list_scratch_bytes(int n, int ncell) {
+  size_t piece[4];
+  return list_pieces(n, ncell, piece);
 }
 
 int launch_full_list(const DBox& b, const int dims[3], double cutoff, int n, const double* x,
@@ -813,36 +985,39 @@ int launch_full_list(const DBox& b, const int dims[3], double cutoff, int n, con
   const double cut2 = cutoff * cutoff;
   double emax = 0.0;
   for (int d = 0; d < 3; ++d) emax = fmax(emax, b.len[d] / dims[d]);
-  // FP32 screening error of |v|^2 - 2 u.v against C - |u|^2, with u (|u_d| <=
-  // e/2) and v (|v_d| <= 3e/2) rounded once to FP32 relative to the centre
-  // cell's centre: coordinate rounding moves |d|^2 by at most
-  // 4 sqrt(3) r e 2^-24, and the roundings of |v|^2, the three FMAs, |u|^2 and
-  // C - |u|^2 by at most (60 e^2 + 3 r^2) 2^-24 (e = largest cell edge,
-  // r = cutoff).  Pairs within twice that of the cutoff take the FP64 path.
+  // FP32 screening error of |v|^2 - 2 u.v against C - |u|^2.  u (|u_d| <= e/2)
+  // is rounded once relative to its cell's centre, v (|v_d| <= 3e/2) once
+  // relative to its own cell's centre (e/2), in the image's offset (e) and in
+  // their sum (3e/2), so a coordinate of v - u is off by at most 3.5 e 2^-24,
+  // which moves |d|^2 by at most 7 sqrt(3) r e 2^-24 (e = largest cell edge,
+  // r = cutoff); the roundings of |v|^2, the three FMAs, |u|^2 and C - |u|^2
+  // add at most (60 e^2 + 3 r^2) 2^-24.  Pairs within twice that of the cutoff
+  // take the FP64 path.
   const double err =
-      (4.0 * sqrt(3.0) * cutoff * emax + 60.0 * emax * emax + 3.0 * cut2) / 16777216.0;
+      (7.0 * sqrt(3.0) * cutoff * emax + 60.0 * emax * emax + 3.0 * cut2) / 16777216.0;
   const double band = 2.0 * err;
   const float lo_band = (float)(cut2 - band), hi_band = (float)(cut2 + band);
   float cut2_up = (float)cut2;  // rounded up
   if ((double)cut2_up < cut2) cut2_up = nextafterf(cut2_up, INFINITY);
-  const int t = full_list_table_size(n, ncell);
-  auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  size_t piece[4];
+  list_pieces(n, ncell, piece);
   char* p = (char*)scratch;
-  float4* box_lo = (float4*)p;
-  float4* box_hi = (float4*)(p + al(sizeof(float4) * t));
-  int* cell_of = (int*)(p + 2 * al(sizeof(float4) * t));
-  k_chunk_boxes<<<ncell, 128, 0, st>>>(x, y, z, cell_start, box_lo, box_hi, cell_of);
+  ListTables T;
+  T.rel = (float4*)p;
+  T.lo = (float4*)(p + piece[0]);
+  T.hi = (float4*)(p + piece[0] + piece[1]);
+  T.group_cell = (int*)(p + piece[0] + piece[1] + piece[2]);
+  k_chunk_boxes<<<ncell, 128, 0, st>>>(b, dims[0], dims[1], dims[2], x, y, z, cell_start, T);
   count_launch();
   // far threshold in r^2, raised by the FP32 error of the test value
   const float near2 = split ? (float)(split->r_near * split->r_near + band) : INFINITY;
-  if (split)
-    k_full_list<true><<<(t + NL_WARPS - 1) / NL_WARPS, NL_BLOCK, 0, st>>>(
-        b, dims[0], dims[1], dims[2], cut2, cut2_up, lo_band, hi_band, t, x, y, z, cell_start,
-        box_lo, box_hi, cell_of, cap, count, nbrs, overflow, near2, split->far, total);
-  else
-    k_full_list<false><<<(t + NL_WARPS - 1) / NL_WARPS, NL_BLOCK, 0, st>>>(
-        b, dims[0], dims[1], dims[2], cut2, cut2_up, lo_band, hi_band, t, x, y, z, cell_start,
-        box_lo, box_hi, cell_of, cap, count, nbrs, overflow, near2, nullptr, total);
+  const auto kern = split ? k_full_list<true> : k_full_list<false>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(FullListSmem)) != cudaSuccess)
+    return check_launch("full_list (shared memory)");
+  kern<<<(unsigned)full_list_groups(n, ncell), NL_BLOCK, sizeof(FullListSmem), st>>>(
+      b, dims[0], dims[1], dims[2], cut2, cut2_up, lo_band, hi_band, x, y, z, cell_start, T, cap,
+      count, nbrs, overflow, near2, split ? split->far : nullptr, total);
   count_launch();
   return check_launch("full_list");
 }
