@@ -288,7 +288,7 @@ int rbx_rbe_force(const rbx_box* box, int num_atoms, int p_number, double alpha,
     o.f_out_x = fx;
     o.f_out_y = fy;
     o.f_out_z = fz;
-    rc = launch_rbe_force_f64(num_atoms, p_number, tab, charge, px, py, pz, o, st);
+    rc = launch_rbe_force_f64(b, num_atoms, p_number, tab, charge, px, py, pz, o, st);
   }
   cudaFreeAsync(tab, st);
   return rc;
@@ -326,9 +326,11 @@ int rbx_ewald_force(const rbx_box* box, int num_atoms, const int kmax[3], double
   const int nk = (2 * kmax[0] + 1) * (2 * kmax[1] + 1) * (2 * kmax[2] + 1) - 1;
   if (nk <= 0) return RBX_OK;
   double *re = nullptr, *im = nullptr, *kv = nullptr;
+  KTab* tab = nullptr;
   RBX_TRY(async_alloc(&re, nk, st));
   RBX_TRY(async_alloc(&im, nk, st));
   RBX_TRY(async_alloc(&kv, (size_t)3 * nk, st));
+  RBX_TRY(async_alloc(&tab, nk, st));
   double qsq = 0.0;
   int rc = RBX_OK;
   if (energy && num_atoms > 0) {  // sum q^2 for the self-energy term
@@ -341,11 +343,12 @@ int rbx_ewald_force(const rbx_box* box, int num_atoms, const int kmax[3], double
   }
   const DBox b = make_dbox(*box);
   if (!rc)
-    rc = launch_ewald(b, num_atoms, kmax, alpha, qqr2e, qsq, charge, px, py, pz, re, im, kv, fx,
-                      fy, fz, energy, st);
+    rc = launch_ewald(b, num_atoms, kmax, alpha, qqr2e, qsq, charge, px, py, pz, re, im, kv, tab,
+                      fx, fy, fz, energy, st);
   cudaFreeAsync(re, st);
   cudaFreeAsync(im, st);
   cudaFreeAsync(kv, st);
+  cudaFreeAsync(tab, st);
   return rc;
 }
 
@@ -801,7 +804,7 @@ int rbx_rbsog_force(const rbx_box* box, int level, double cut_off, double qqr2e,
       o.f_out_x = fx;
       o.f_out_y = fy;
       o.f_out_z = fz;
-      rc = launch_rbe_force_f64(num_atoms, pt, tab, charge, px, py, pz, o, st);
+      rc = launch_rbe_force_f64(b, num_atoms, pt, tab, charge, px, py, pz, o, st);
     }
     if (!rc && energy) {
       cudaMemcpyAsync(energy, en, sizeof(double), cudaMemcpyDeviceToHost, st);

@@ -567,7 +567,7 @@ int rbx_engine::kspace_finish(bool kick, const int* epoch_dev) {
   if (mixed)
     ETRY(launch_rbe_force_mixed(n, Pk, tab, atoms, o, st, tun.frc_block));
   else
-    ETRY(launch_rbe_force_f64(n, Pk, tab, q, x, y, z, o, st, tun.frc_block));
+    ETRY(launch_rbe_force_f64(dbox, n, Pk, tab, q, x, y, z, o, st, tun.frc_block));
   return RBX_OK;
 }
 
@@ -692,7 +692,7 @@ int rbx_engine::autotune(bool force, rbx_tuning* out) {
         rc = time_it(
             [&]() {
               return mixed ? launch_rbe_force_mixed(n, Pk, tab, atoms, o, st, blk)
-                           : launch_rbe_force_f64(n, Pk, tab, q, x, y, z, o, st, blk);
+                           : launch_rbe_force_f64(dbox, n, Pk, tab, q, x, y, z, o, st, blk);
             },
             &ms);
         c.push_back({blk, 0, ms});
@@ -1357,9 +1357,8 @@ int rbx_engine::kspace_energy_exact(const int kmax[3], double* energy) {
     set_error("kspace_energy_exact: cudaMallocAsync failed");
     return RBX_ERR_NOMEM;
   }
-  const size_t N = (size_t)n;
   int rc = launch_ewald(dbox, n, kmax, prm.alpha, prm.qqr2e, qsq, q, x, y, z, buf, buf + nk,
-                        buf + 2 * (size_t)nk, stage, stage + N, stage + 2 * N,
+                        buf + 2 * (size_t)nk, nullptr, nullptr, nullptr, nullptr,
                         buf + 5 * (size_t)nk, st);
   if (!rc)
     rc = cuda_ok(cudaMemcpyAsync(energy, buf + 5 * (size_t)nk, sizeof(double),

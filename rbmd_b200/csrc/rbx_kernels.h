@@ -14,6 +14,7 @@ struct KTab {
   double kx, ky, kz;
   double a, b;  // coef * Re rho, coef * Im rho, coef = -4 pi qqr2e S / (P V k^2)
   int m[4];     // integer m (mixed form)
+  double md[3]; // m as given (FP64 form)
 };
 
 // Destinations of the RBE force pass.
@@ -71,9 +72,9 @@ int launch_rbe_finalize(const DBox& b, int p, int nparts, const double* part_re,
                         unsigned* sum_ctr = nullptr);
 // kterm: scratch of 8 p doubles for the per-k energy/virial terms (parallel
 // finalize); when null and energy is requested, one block does the finalize.
-int launch_rbe_force_f64(int n, int p, const KTab* tab, const double* q, const double* x,
-                         const double* y, const double* z, const RbeForceOut& out,
-                         cudaStream_t st, int block = 256);
+int launch_rbe_force_f64(const DBox& b, int n, int p, const KTab* tab, const double* q,
+                         const double* x, const double* y, const double* z,
+                         const RbeForceOut& out, cudaStream_t st, int block = 256);
 int launch_rbe_force_mixed(int n, int p, const KTab* tab, const uint4* atoms,
                            const RbeForceOut& out, cudaStream_t st, int block = 256);
 // step_dev (may be null): read the step from device memory (step graphs).
@@ -82,10 +83,11 @@ int launch_rbe_sample(int p, const double* tables, const int cnt[3], const doubl
                       double* mz, int* mi, int* status, cudaStream_t st);
 int launch_m_to_int(int p, const double* mx, const double* my, const double* mz, int* mi,
                     cudaStream_t st);
+// Forces only with tab (nk entries of scratch).
 int launch_ewald(const DBox& b, int n, const int kmax[3], double alpha, double qqr2e,
                  double qsq, const double* q, const double* x, const double* y, const double* z,
-                 double* re, double* im, double* kvec, double* fx, double* fy, double* fz,
-                 double* energy, cudaStream_t st);
+                 double* re, double* im, double* kvec, KTab* tab, double* fx, double* fy,
+                 double* fz, double* energy, cudaStream_t st);
 
 // Host-side sampler tables (order m = 0, +1, -1, ...), identical to the oracle's.
 int rbe_axis_table(double L, double alpha, double* w, int max_entries, double* total);

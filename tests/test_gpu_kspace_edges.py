@@ -1,0 +1,106 @@
+"""The k-space passes over charged atoms only: no charge at all, a few charged
+atoms (threads share an atom's k-vectors), mostly charged tiles, all charged;
+ragged atom and k counts, more k-vectors than one staged table.
+
+Reference: direct FP64 sums in numpy over every atom.  FP64 tolerance: the
+phase of |m| <= 40 turns carries 40 * 2^-53 * 2 pi = 3e-14 at most, amplified
+by nothing in the sums, and a sum of N terms adds sqrt(N) 2^-53: 1e-12 covers
+both.  Float: the coordinate's own rounding times |m|, 40 * 2^-24 = 2.4e-6 of
+a turn, 1.5e-5 rad; the reference takes the same float coordinates, so only the
+fixed-point step 2^-32 and the FP32 sine remain: 5e-6 as the golden tests use.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+CASES = [(257, 33, 0.0), (1000, 100, 0.03), (1003, 64, 0.4), (999, 129, 0.7), (512, 600, 1.0),
+         (40001, 100, 0.1)]
+
+
+def _system(n, p, share, seed):
+    rng = np.random.default_rng(seed)
+    lo, hi = np.array([0.0, 0.0, 0.0]), np.array([21.0, 18.5, 24.0])
+    pos = rng.uniform(0, 1, (n, 3)) * (hi - lo)
+    q = np.where(rng.uniform(size=n) < share, rng.choice([-1.0, 1.0, 0.5], n), 0.0)
+    m = rng.integers(-12, 13, (3, p)).astype(float)
+    m[0, (m == 0).all(0)] = 1.0
+    return lo, hi, pos, q, m
+
+
+def _direct(L, pos, q, m, S, p):
+    k = 2 * np.pi * m / L[:, None]
+    ph = pos @ k
+    re, im = (q[:, None] * np.cos(ph)).sum(0), (q[:, None] * np.sin(ph)).sum(0)
+    c = -4 * np.pi * S / (p * np.prod(L) * (k * k).sum(0))
+    f = (c * (np.cos(ph) * im - np.sin(ph) * re)) @ k.T * q[:, None]
+    return re, im, f
+
+
+def _close(got, want, tol):
+    scale = np.sqrt((want ** 2).mean())
+    assert np.sqrt(((got - want) ** 2).mean()) <= tol * scale
+    assert np.abs(got - want).max() <= 50 * tol * scale
+
+
+@pytest.mark.parametrize("n,p,share", CASES)
+@pytest.mark.parametrize("real", ["f64", "f32"])
+def test_kspace_charged_shares(cuda, rbx, n, p, share, real):
+    lo, hi, pos, q, m = _system(n, p, share, n + p)
+    if real == "f32":
+        pos, q = pos.astype(np.float32).astype(float), q.astype(np.float32).astype(float)
+    L = hi - lo
+    t = cuda.float64 if real == "f64" else cuda.float32
+    dev = lambda a: cuda.as_tensor(np.ascontiguousarray(a)).to("cuda", t)  # noqa: E731
+    box = rbx.Box.make(lo, hi)
+    S = rbx.rbe_gauss_sum(box, 0.16)
+    T = [dev(q), *(dev(v) for v in m), *(dev(pos[:, d]) for d in range(3))]
+    rho = [cuda.zeros(p, dtype=t, device="cuda") for _ in range(2)]
+    F = [cuda.full((n,), 7.0, dtype=t, device="cuda") for _ in range(3)]
+    sf, fc = ((rbx.rbe_structure_factor, rbx.rbe_force) if real == "f64" else
+              (rbx.rbe_structure_factor_f32, rbx.rbe_force_f32))
+    sf(box, *T, *rho)
+    fc(box, 0.16, S, 1.0, *rho, *T, *F)
+    cuda.cuda.synchronize()
+    re, im, f = _direct(L, pos, q, m, S, p)
+    tol = 1e-12 if real == "f64" else 5e-6
+    _close(np.stack([a.cpu().numpy() for a in rho]).astype(float), np.stack([re, im]), tol)
+    got = np.stack([a.cpu().numpy() for a in F], 1).astype(float)
+    _close(got, f, tol)
+    assert (got[q == 0] == 0).all()
+
+
+def test_kspace_fractional_k_and_far_positions(cuda, rbx):
+    """The FP64 functors take any real k-vector and positions outside the box."""
+    lo, hi, pos, q, m = _system(300, 40, 0.5, 3)
+    m = m + 0.25
+    pos = pos + 1000.0 * (hi - lo)
+    L = hi - lo
+    dev = lambda a: cuda.as_tensor(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    box = rbx.Box.make(lo, hi)
+    T = [dev(q), *(dev(v) for v in m), *(dev(pos[:, d]) for d in range(3))]
+    rho = [cuda.zeros(40, dtype=cuda.float64, device="cuda") for _ in range(2)]
+    F = [cuda.zeros(300, dtype=cuda.float64, device="cuda") for _ in range(3)]
+    rbx.rbe_structure_factor(box, *T, *rho)
+    rbx.rbe_force(box, 0.16, 50.0, 1.0, *rho, *T, *F)
+    cuda.cuda.synchronize()
+    re, im, f = _direct(L, pos, q, m, 50.0, 40)
+    # 36,750 turns at most: 36,750 * 2 pi * 2^-53 * 4 roundings = 1e-10
+    _close(np.stack([a.cpu().numpy() for a in rho]), np.stack([re, im]), 1e-10)
+    _close(np.stack([a.cpu().numpy() for a in F], 1), f, 1e-10)
+
+
+@pytest.mark.parametrize("n,kmax,share", [(300, (1, 1, 1), 1.0), (2000, (3, 2, 1), 0.1),
+                                          (70, (0, 4, 2), 0.0)])
+def test_ewald_blocks(cuda, rbx, oracle, n, kmax, share):
+    lo, hi, pos, q, _ = _system(n, 1, share, n)
+    dev = lambda a: cuda.as_tensor(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    cols = [np.ascontiguousarray(pos[:, d]) for d in range(3)]
+    f, e = oracle.ewald_force(oracle.Box.make(lo, hi), 0.16, 1.0, list(kmax), q, *cols)
+    F = [cuda.zeros(n, dtype=cuda.float64, device="cuda") for _ in range(3)]
+    en = cuda.zeros(1, dtype=cuda.float64, device="cuda")
+    rbx.ewald_force(rbx.Box.make(lo, hi), list(kmax), 0.16, 1.0, dev(q), *(dev(c) for c in cols),
+                    *F, energy=en)
+    cuda.cuda.synchronize()
+    _close(np.stack([a.cpu().numpy() for a in F], 1), f, 1e-12)
+    assert abs(en.item() - e) <= 1e-11 * abs(e)
