@@ -40,17 +40,19 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 
 // LJ 12-6 force/r (lj126_rs, src/force/src/lj_op/rocm/lj_op.hip.cu:40-54) in FP64.
 __device__ __forceinline__ double lj_f64(double eps_ij, double s6, double d2) {
-  const double d6 = d2 * d2 * d2;
-  const double sd6 = s6 / d6;
-  return -24.0 * eps_ij * ((2.0 * sd6 - 1.0) * sd6) / d2;
+  const double r2i = 1.0 / d2;
+  const double sd6 = s6 * (r2i * r2i * r2i);
+  return -24.0 * eps_ij * ((2.0 * sd6 - 1.0) * sd6) * r2i;
 }
 // erfc-Coulomb force/r (CoulCutForce_rs_fix, lj_cut_coul_kspace_op.hip.cu:134-161).
 __device__ __forceinline__ double coul_f64(double alpha, double sqrt_alpha, double qqr2e,
                                            double qq, double d2) {
-  const double dis = sqrt(d2);
-  const double g = erfc(sqrt_alpha * dis) / d2 +
-                   2.0 * sqrt_alpha * exp(-alpha * d2) / (1.7724538509055160273 * dis);
-  return -qqr2e * qq * g / dis;
+  const double rinv = rsqrt(d2), dis = d2 * rinv;
+  // erfc(x) = erfcx(x) exp(-x^2): one exponential serves both terms
+  const double ex = exp(-alpha * d2);
+  const double g = ex * (erfcx(sqrt_alpha * dis) * rinv +
+                         (2.0 / 1.7724538509055160273) * sqrt_alpha);
+  return -qqr2e * qq * g * (rinv * rinv);
 }
 __device__ __forceinline__ float lj_f32(float eps_ij, float s6, float d2) {
   const float d6 = d2 * d2 * d2;
@@ -200,9 +202,28 @@ __device__ __forceinline__ float fixed_d2_weighted(const PairParams& pp, const u
 // classification and the hash are branch-free, and force-carrying pairs are
 // appended to a per-warp queue (index plus two flag bits) that is drained 32
 // pairs at a time from its tail.
+//
+// Bound by the latency of the gathers and, above that, by integer issue, so
+// resident warps count more than registers: the mixed form fits eight blocks an
+// SM (32 registers, no spills), the FP64 form six (40, a few spilled words that
+// stay in L1).  What keeps the registers down is that the warp index comes
+// through a shuffle: atom, row and loop state are then uniform.  Queue pushes
+// are predicated stores at ballot prefixes; the far segment is read in full
+// 128-entry batches from the row's end, so only its front batch tests for
+// entries that are none.  Measured, B200, 200,000-atom LJ electrolyte: mixed
+// 464 -> 380 us (four blocks of 64 registers, per-thread state before; 415,
+// 397, 389, 381 at four to seven blocks), FP64 697 -> 554 us (three blocks
+// before; 608, 568 at four and five); water, 73,000 atoms: 271 -> 244 and
+// 523 -> 371 us.  A second queue that window-tests the selected far pairs
+// before they take a force slot was slower in the mixed form (+10 %), and split
+// rows with it slower than unsplit ones in FP64 (677 us then, 607 unsplit).
 // ---------------------------------------------------------------------------
-constexpr int RBL_NEAR_U = 3;  // 32-candidate chunks per near batch
-constexpr int RBL_QCAP = 32 + 32 * (RBL_NEAR_U > 4 ? RBL_NEAR_U : 4);  // far batches: 128
+// 32-candidate chunks per near batch: the mixed form's near segments (73
+// candidates on the LJ electrolyte) fit one batch of three; the FP64 form's
+// whole rows take two, whose registers leave room for a sixth block (2 / 3
+// chunks at five blocks: 568 / 601 us at 200,000 atoms)
+constexpr int RBL_NEAR_U_MIXED = 3, RBL_NEAR_U_F64 = 2;
+constexpr int RBL_QCAP = 32 + 128;  // force queue (a far batch is 128 entries)
 constexpr int QF_SHELL = (int)0x80000000;  // shell pair: force times freq
 constexpr int QF_CHECK = 0x40000000;       // far pair: shell window still to be tested
 constexpr int QF_INDEX = 0x3fffffff;       // atom index (n < 2^30)
@@ -212,6 +233,16 @@ __device__ __forceinline__ float lj_f32_fast(float eps_ij, float s6, float d2) {
   const float r2i = __fdividef(1.0f, d2);
   const float sd6 = s6 * (r2i * r2i * r2i);
   return -24.f * eps_ij * ((2.f * sd6 - 1.f) * sd6) * r2i;
+}
+
+// Append v at *p (shared memory, 32-bit address) under a predicate, without a
+// branch around the store.
+__device__ __forceinline__ void push_if(bool take, unsigned p, int v) {
+  asm volatile(
+      "{\n\t.reg .pred t;\n\tsetp.ne.u32 t, %0, 0;\n\t@t st.shared.u32 [%1], %2;\n\t}" ::"r"(
+          (unsigned)take),
+      "r"(p), "r"(v)
+      : "memory");
 }
 
 template <int SEL>
@@ -258,6 +289,7 @@ __device__ __forceinline__ void rbl_fused_body(
     const int* __restrict__ epoch_dev, const Rows& rows, double* __restrict__ fx,
     double* __restrict__ fy, double* __restrict__ fz, double* __restrict__ fpart, int bx,
     int gx) {
+  constexpr int NEAR_U = MIXED ? RBL_NEAR_U_MIXED : RBL_NEAR_U_F64;
   using T = typename std::conditional<MIXED, float, double>::type;
   const int epoch = epoch_dev ? *epoch_dev : epoch_arg;  // device copy inside a step graph
   __shared__ int s_q[PAIR_WARPS][RBL_QCAP];
@@ -265,7 +297,9 @@ __device__ __forceinline__ void rbl_fused_body(
   const TypeTables tt = load_type_tables(pp, MIXED);
   const float* const f_eps = tt.f_eps;
   const float* const f_s6 = tt.f_s6;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // the warp's index through a shuffle: uniform for the compiler, with all
+  // that follows from it (the atom, its row, the loops)
+  const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const unsigned lt = lanemask_lt();
   const unsigned long long fmask = (unsigned long long)(pp.freq - 1);
   const float alpha_f = (float)pp.alpha, sqa_f = (float)pp.sqrt_alpha, qqr2e_f = (float)pp.qqr2e;
@@ -274,6 +308,7 @@ __device__ __forceinline__ void rbl_fused_body(
   const int nt = pp.ntypes;
   const int wstride = gx * PAIR_WARPS;
   int* const wq = s_q[warp];
+  const unsigned wq_at = (unsigned)__cvta_generic_to_shared(wq);
   for (int i = bx * PAIR_WARPS + warp; i < n; i += wstride) {
     const uint4 ai = atoms[i];
     const double xi = x[i], yi = y[i], zi = z[i];
@@ -328,9 +363,11 @@ __device__ __forceinline__ void rbl_fused_body(
         const double d2 =
             __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
         const bool ok = !(c & QF_CHECK) || classify_exact(d2, pp).shell_window;
-        const double qq = (double)qi * __ldg(q + j);
         double f = lj_f64(tt.eps[ti * nt + tj], tt.s6[ti * nt + tj], d2);
-        if (qq != 0.0) f += coul_f64(pp.alpha, pp.sqrt_alpha, pp.qqr2e, qq, d2);
+        if (qi != (T)0) {  // the whole warp works on atom i
+          const double qq = (double)qi * __ldg(q + j);
+          if (qq != 0.0) f += coul_f64(pp.alpha, pp.sqrt_alpha, pp.qqr2e, qq, d2);
+        }
         if (c < 0) f *= (double)freq_t;
         f = ok ? f : 0.0;
         fxa -= (T)(f * dx);
@@ -348,24 +385,24 @@ __device__ __forceinline__ void rbl_fused_body(
     };
 
     // near segment: full classification
-    for (int k0 = 0; k0 < nf; k0 += 32 * RBL_NEAR_U) {
-      int jj[RBL_NEAR_U];
-      uint4 aa[RBL_NEAR_U];
-      unsigned long long kb[RBL_NEAR_U];
+    for (int k0 = 0; k0 < nf; k0 += 32 * NEAR_U) {
+      int jj[NEAR_U];
+      uint4 aa[NEAR_U];
+      unsigned long long kb[NEAR_U];
 #pragma unroll
-      for (int u = 0; u < RBL_NEAR_U; ++u) {
+      for (int u = 0; u < NEAR_U; ++u) {
         const int k = k0 + u * 32 + lane;
         jj[u] = k < nf ? __ldg(row + k) : i;
       }
 #pragma unroll
-      for (int u = 0; u < RBL_NEAR_U; ++u) {
+      for (int u = 0; u < NEAR_U; ++u) {
         aa[u] = __ldg(atoms + jj[u]);
         kb[u] = __ldg(key_b + jj[u]);
       }
       unsigned core_bits = 0, shell_bits = 0, sel_bits = 0, unsure_bits = 0;
 #pragma unroll
-      for (int u = 0; u < RBL_NEAR_U; ++u) {
-        const bool valid = jj[u] != i;
+      for (int u = 0; u < NEAR_U; ++u) {
+        const bool valid = k0 + u * 32 + lane < nf;
         bool unsure;
         const Classified c = classify_screen(
             pp, CUBIC ? fixed_d2(ai, aa[u]) : fixed_d2_weighted(pp, ai, aa[u]), &unsure);
@@ -377,7 +414,7 @@ __device__ __forceinline__ void rbl_fused_body(
       }
       if (__any_sync(0xffffffffu, unsure_bits != 0)) {  // rare: FP64 predicate decides
 #pragma unroll
-        for (int u = 0; u < RBL_NEAR_U; ++u) {
+        for (int u = 0; u < NEAR_U; ++u) {
           if (unsure_bits & (1u << u)) {
             const Classified c = classify_exact(exact_d2(pp, x, y, z, i, jj[u]), pp);
             core_bits = (core_bits & ~(1u << u)) | ((unsigned)c.core_active << u);
@@ -387,47 +424,52 @@ __device__ __forceinline__ void rbl_fused_body(
       }
       const unsigned push_bits = core_bits | (shell_bits & sel_bits);
 #pragma unroll
-      for (int u = 0; u < RBL_NEAR_U; ++u) {
+      for (int u = 0; u < NEAR_U; ++u) {
         const bool push = (push_bits >> u) & 1u;
         const unsigned m = __ballot_sync(0xffffffffu, push);
-        if (push) wq[qn + __popc(m & lt)] = ((core_bits >> u) & 1u) ? jj[u] : (jj[u] | QF_SHELL);
+        push_if(push, wq_at + 4 * (qn + __popc(m & lt)),
+                ((core_bits >> u) & 1u) ? jj[u] : (jj[u] | QF_SHELL));
         qn += __popc(m);
       }
       drain_full();
     }
 
-    // far segment: batch hash first; selected pairs are queued with the
-    // window test still to do.  The segment is read from the 16-byte boundary
-    // at or below its start, four entries a lane (one 128-entry batch per
-    // warp load); entries before the segment start are skipped.
+    // far segment: batch hash first; selected pairs are queued with the window
+    // test still to do
+    // 128 entries, four a lane (e); lanes' entries below `skip` are not in the
+    // segment
+    auto far_batch = [&](int4 e, int skip) {
+      const int jj[4] = {e.x, e.y, e.z, e.w};
+      unsigned long long kb[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) kb[u] = __ldg(key_b + jj[u]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool sel = batch_selected<SEL>(ea ^ kb[u], fmask, pp.div) & (u >= skip);
+        const unsigned m = __ballot_sync(0xffffffffu, sel);
+        push_if(sel, wq_at + 4 * (qn + __popc(m & lt)), jj[u] | (QF_SHELL | QF_CHECK));
+        qn += __popc(m);
+      }
+      drain_full();
+    };
     {
+      // full batches from the row's end (rows start on 128-byte lines and
+      // cap % 32 == 0, so every lane's four entries are 16-byte aligned), then
+      // the ragged front one
+      int p0 = rows.cap - 128;
       const int fs = rows.cap - nb;  // first far entry
-      const int fb = fs & ~3;        // rows start on 128-byte lines (cap % 32 == 0)
-      const int4* f4 = reinterpret_cast<const int4*>(row + fb);
-      for (int k0 = 0; fb + k0 < rows.cap; k0 += 128) {
-        const int p0 = fb + k0 + 4 * lane;  // row position of this lane's first entry
+      for (; p0 >= fs; p0 -= 128)
+        far_batch(__ldg(reinterpret_cast<const int4*>(row + p0) + lane), 0);
+      const int skip = fs - (p0 + 4 * lane);  // of this lane's entries
+      if (p0 + 128 > fs) {
         int4 e = make_int4(i, i, i, i);
-        if (p0 < rows.cap) e = __ldg(f4 + (k0 >> 2) + lane);
-        const int jj[4] = {p0 >= fs ? e.x : i, p0 + 1 >= fs ? e.y : i, p0 + 2 >= fs ? e.z : i,
-                           p0 + 3 >= fs ? e.w : i};
-        unsigned long long kb[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) kb[u] = __ldg(key_b + jj[u]);
-        unsigned sb = 0;
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          sb |= (unsigned)((jj[u] != i) & batch_selected<SEL>(ea ^ kb[u], fmask, pp.div)) << u;
-        // queue slots: exclusive prefix over lanes of the per-lane counts (0..4)
-        const unsigned c = __popc(sb);
-        const unsigned b0 = __ballot_sync(0xffffffffu, c & 1u),
-                       b1 = __ballot_sync(0xffffffffu, c & 2u),
-                       b2 = __ballot_sync(0xffffffffu, c & 4u);
-        int pos = qn + __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt);
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if ((sb >> u) & 1u) wq[pos++] = jj[u] | QF_SHELL | QF_CHECK;
-        qn += __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
-        drain_full();
+        if (skip < 4) {
+          e = __ldg(reinterpret_cast<const int4*>(row + p0 + 4 * lane));
+          if (skip > 0) e.x = i;  // what lies before the segment is no entry
+          if (skip > 1) e.y = i;
+          if (skip > 2) e.z = i;
+        }
+        far_batch(e, skip);
       }
     }
     if (lane < qn) pair_force(lane);
@@ -452,7 +494,7 @@ __device__ __forceinline__ void rbl_fused_body(
 }
 
 template <bool MIXED, int SEL, bool CUBIC>
-__global__ void __launch_bounds__(PAIR_BLOCK, MIXED ? 4 : 3)  // no spills in either form
+__global__ void __launch_bounds__(PAIR_BLOCK, MIXED ? 8 : 6)
 k_rbl_fused(PairParams pp, int n, const uint4* __restrict__ atoms, const double* __restrict__ x,
             const double* __restrict__ y, const double* __restrict__ z,
             const double* __restrict__ q, const int* __restrict__ type,
@@ -465,9 +507,11 @@ k_rbl_fused(PairParams pp, int n, const uint4* __restrict__ atoms, const double*
 }
 
 // The batched form holds its replica's pointers in registers (the single
-// form reads them from the constant bank): one resident block fewer, no spills.
+// form reads them from the constant bank), so it fits fewer blocks: five in the
+// mixed form (a phased step of 48 replicas, 4,448 atoms on average: 1066, 940,
+// 952, 1046 us at three, five, six and eight).
 template <bool MIXED, int SEL, bool CUBIC>
-__global__ void __launch_bounds__(PAIR_BLOCK, MIXED ? 3 : 2)
+__global__ void __launch_bounds__(PAIR_BLOCK, MIXED ? 5 : 2)
 k_rbl_fused_batch(const RblArgs* __restrict__ a, const int* __restrict__ start, int nrep) {
   // the replica's arguments in shared memory: read where used, not held in registers
   static_assert(sizeof(RblArgs) % 4 == 0 && sizeof(RblArgs) <= 4 * PAIR_BLOCK, "RblArgs size");
