@@ -200,7 +200,7 @@ int rbx_engine::init() {
   ETRY(alloc(&cell_start, (size_t)ncell + 1));
   ETRY(alloc(&cell_scratch, cells_scratch_bytes(n, ncell)));
   ETRY(alloc(&list_scratch, full_list_scratch_bytes(n, ncell)));
-  ETRY(alloc(&dflags, 12));  // [8], [9]: block counters of the drift and the RBE finalize
+  ETRY(alloc(&dflags, 12));  // [8]: block counter of the drift
   ETRY(cuda_ok(cudaMemsetAsync(dflags, 0, sizeof(int) * 12, st), "memset"));
   ETRY(alloc(&max_d2, 1));
   ETRY(alloc(&cand_total, 1));
@@ -532,18 +532,18 @@ int rbx_engine::kspace_finish(bool kick, const int* epoch_dev) {
   const bool mixed = prm.precision == RBX_MIXED;
   const bool rbl = prm.neighbor_type == RBX_NEIGHBOR_RBL;
   const int mean_parts = rbl ? nrbl + (spec_natoms ? SPEC_PARTS : 0) : 0;
+  RbeForceOut o;  // the force launch also sums the energy and virial terms
   if (sog) {
     const SogVirial sv{P, sog_mult, sog_wv, kterm + 2 * (size_t)Pk, virk};
     ETRY(launch_rbsog_finalize(dbox, Pk, nparts, part_re, part_im, mx, my, mz, sog_w, rho_re,
                                rho_im, tab, kterm, -sog_self * qsq * prm.qqr2e, ek, mean_parts,
-                               fpart, n, rbl ? mean : nullptr, st, &sv));
+                               fpart, n, rbl ? mean : nullptr, st, &sv, &o.job));
   } else
     ETRY(launch_rbe_finalize(dbox, P, P > 0 ? nparts : 0, part_re, part_im, mx, my, mz,
                              prm.alpha, S, prm.qqr2e, qsq, qsum, P > 0 ? rho_re : nullptr,
                              rho_im, P > 0 ? ek : nullptr, virk, P > 0 ? tab : nullptr,
                              mean_parts, fpart, n, rbl ? mean : nullptr, kterm, st,
-                             (unsigned*)(dflags + 9)));
-  RbeForceOut o;
+                             &o.job));
   o.f_pair_x = fpx;
   o.f_pair_y = fpy;
   o.f_pair_z = fpz;

@@ -17,6 +17,20 @@ struct KTab {
   double md[3]; // m as given (FP64 form)
 };
 
+// Energy and virial from the per-k terms of a finalize: one warp adds them in
+// increasing k.  Given to a force pass, it runs as one more block of that
+// launch, beside the forces, which do not need it.
+struct EnergyJob {
+  enum Kind { NONE, RBE, RBSOG } kind = NONE;
+  int p = 0;
+  const double* kterm = nullptr;  // RBE [p][8]; RBSOG [p]
+  const double* vterm = nullptr;  // RBSOG [p][6]
+  double alpha = 0, V = 0, qqr2e = 0, qsq = 0, qsum = 0;  // RBE
+  double self_energy = 0;                                // RBSOG
+  double* energy = nullptr;
+  double* virial = nullptr;
+};
+
 // Destinations of the RBE force pass.
 struct RbeForceOut {
   const double* f_pair_x = nullptr;  // add real-space force (combine), or null
@@ -35,6 +49,7 @@ struct RbeForceOut {
   const int* type = nullptr;
   const double* inv_mass = nullptr;
   double half_dt = 0.0;
+  EnergyJob job;
 };
 
 // ---- k-space (rbx_rbe.cu) ----
@@ -69,9 +84,11 @@ int launch_rbe_finalize(const DBox& b, int p, int nparts, const double* part_re,
                         double qsum, double* rho_re, double* rho_im, double* energy,
                         double* virial, KTab* tab, int mean_parts, const double* fpart,
                         int n_atoms, double* mean_out, double* kterm, cudaStream_t st,
-                        unsigned* sum_ctr = nullptr);
+                        EnergyJob* job = nullptr);
 // kterm: scratch of 8 p doubles for the per-k energy/virial terms (parallel
 // finalize); when null and energy is requested, one block does the finalize.
+// job: the sum over k is not launched here but described for the force pass.
+int launch_energy_sum(const EnergyJob& job, cudaStream_t st);
 int launch_rbe_force_f64(const DBox& b, int n, int p, const KTab* tab, const double* q,
                          const double* x, const double* y, const double* z,
                          const RbeForceOut& out, cudaStream_t st, int block = 256);
@@ -325,7 +342,8 @@ int launch_rbsog_finalize(const DBox& b, int p, int nparts, const double* part_r
                           const double* mz, const double4* w, double* rho_re, double* rho_im,
                           KTab* tab, double* kterm, double self_energy, double* energy,
                           int mean_parts, const double* fpart, int n_atoms, double* mean_out,
-                          cudaStream_t st, const SogVirial* vir = nullptr);
+                          cudaStream_t st, const SogVirial* vir = nullptr,
+                          EnergyJob* job = nullptr);
 // The NPT gather chain of RBSOGSampleKSpace over the p samples: one block;
 // r_i = G_npt(m_i) |k_i|^4 / (G(m_i) |k_i|^2) and a Philox uniform u_i per
 // sample, then idx_0 = 0, idx_i = i when u_i r_(idx_(i-1)) < r_i else

@@ -463,38 +463,52 @@ k_rbe_finalize(int p, int nparts, const double* __restrict__ part_re,
 // strided order, then a fixed tree) and writes rho(k), the force table entry
 // and its seven energy/virial terms to kterm[k][0..6]; blocks p..p+2 reduce
 // the per-block pair-force sums into the mean force.  The per-k terms are then
-// added in increasing k by one warp in a fixed order: k_rbe_energy_sum, or,
-// with es.ctr, the last block of this kernel to finish.
+// added in increasing k by one warp in a fixed order (energy_job): in
+// k_energy_sum, or in an extra block of the force pass that follows, where
+// nothing waits for it (as the finalize's last block, behind a fence and a
+// counter, it was 2 us of a 6 us launch that the forces wait for).
 constexpr int FK_BLOCK = 128;
 
-struct EnergySum {
-  unsigned* ctr;  // block counter, zero before the launch; cleared again by the last block
-  double alpha, V, qqr2e, qsq, qsum;
-  double* energy;
-  double* virial;
-};
-
-__device__ __forceinline__ void rbe_energy_sum_warp(int p, const double* __restrict__ kterm,
-                                                    const EnergySum& es, bool coherent) {
-  const int lane = threadIdx.x & 31;
+__device__ __forceinline__ void energy_job(const EnergyJob& job) {
+  const int lane = threadIdx.x & 31, p = job.p;
   double t[7] = {0, 0, 0, 0, 0, 0, 0};
-  // each lane adds its k in increasing order; the seven loads of a k are independent
-  for (int k = lane; k < p; k += 32) {
-    const double* r = kterm + (size_t)k * 8;
+  if (job.kind == EnergyJob::RBE) {
+    // each lane adds its k in increasing order; the seven loads of a k are independent
+    for (int k = lane; k < p; k += 32)
 #pragma unroll
-    for (int c = 0; c < 7; ++c) t[c] += coherent ? __ldcg(r + c) : r[c];
+      for (int c = 0; c < 7; ++c) t[c] += job.kterm[(size_t)k * 8 + c];
+  } else {
+    for (int k = lane; k < p; k += 32) {
+      if (job.energy) t[0] += job.kterm[k];
+      if (job.vterm)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) t[1 + c] += job.vterm[6 * (size_t)k + c];
+    }
   }
 #pragma unroll
   for (int c = 0; c < 7; ++c)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t[c] += __shfl_down_sync(0xffffffffu, t[c], o);
-  if (lane == 0) {
+  if (lane != 0) return;
+  if (job.kind == EnergyJob::RBE) {
     const double MY_PIS = 1.77245385090551602729, MY_PI2 = 1.57079632679489661923;
-    const double etot =
-        t[0] - (sqrt(es.alpha) * es.qsq / MY_PIS + MY_PI2 * es.qsum * es.qsum / (es.alpha * es.V));
-    *es.energy = etot * es.qqr2e;
-    for (int c = 0; c < 6; ++c) es.virial[c] = t[1 + c] * es.qqr2e;
+    const double etot = t[0] - (sqrt(job.alpha) * job.qsq / MY_PIS +
+                                MY_PI2 * job.qsum * job.qsum / (job.alpha * job.V));
+    *job.energy = etot * job.qqr2e;
+    for (int c = 0; c < 6; ++c) job.virial[c] = t[1 + c] * job.qqr2e;
+  } else {
+    if (job.energy) *job.energy = t[0] + job.self_energy;
+    if (job.vterm)
+      for (int c = 0; c < 6; ++c) job.virial[c] = t[1 + c];
   }
+}
+
+__global__ void __launch_bounds__(32) k_energy_sum(EnergyJob job) { energy_job(job); }
+
+int launch_energy_sum(const EnergyJob& job, cudaStream_t st) {
+  k_energy_sum<<<1, 32, 0, st>>>(job);
+  count_launch();
+  return check_launch("energy_sum");
 }
 
 __device__ void rbe_finalize_one(int k, int p, int nparts, const double* __restrict__ part_re,
@@ -516,11 +530,10 @@ struct FinalizeArgs {
   const double* fpart;
   double n_atoms;
   double* mean_out;
-  EnergySum es;
 };
 
-// Block blk of a grid of gx blocks.
-__device__ __forceinline__ void finalize_k_body(const FinalizeArgs& A, int blk, int gx) {
+// Block blk.
+__device__ __forceinline__ void finalize_k_body(const FinalizeArgs& A, int blk) {
   const int p = A.p, nparts = A.nparts, mean_parts = A.mean_parts;
   const double* __restrict__ part_re = A.part_re;
   const double* __restrict__ part_im = A.part_im;
@@ -528,41 +541,38 @@ __device__ __forceinline__ void finalize_k_body(const FinalizeArgs& A, int blk, 
   double* __restrict__ kterm = A.kterm;
   double* __restrict__ mean_out = A.mean_out;
   const double n_atoms = A.n_atoms;
-  const EnergySum& es = A.es;
-  __shared__ double sh[FK_BLOCK / 32];
-  __shared__ bool s_last;
+  __shared__ double sh[2 * FK_BLOCK / 32];
   if (blk >= p) {  // mean of the pair-force block sums, one component per block
     const int d = blk - p;
     double s = 0.0;
-    for (int b = threadIdx.x; b < mean_parts; b += FK_BLOCK) s += fpart[(size_t)b * 3 + d];
+    constexpr int U = 16;  // loads in flight per thread
+    for (int b0 = threadIdx.x; b0 < mean_parts; b0 += U * FK_BLOCK) {
+      double v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int b = b0 + u * FK_BLOCK;
+        v[u] = b < mean_parts ? fpart[(size_t)b * 3 + d] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) s += v[u];
+    }
     s = block_sum_det<FK_BLOCK>(s, sh);
     if (threadIdx.x == 0) mean_out[d] = s / n_atoms;
   } else {
     rbe_finalize_one(blk, p, nparts, part_re, part_im, A.mx, A.my, A.mz, A.Lx, A.Ly, A.Lz,
                      A.alpha, A.S, A.qqr2e, A.rho_re, A.rho_im, A.tab, kterm, sh);
   }
-  if (!es.ctr) return;
-  if (threadIdx.x == 0) {
-    __threadfence();
-    s_last = atomicAdd(es.ctr, 1u) == (unsigned)gx - 1;
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  if (threadIdx.x < 32) rbe_energy_sum_warp(p, kterm, es, true);
-  if (threadIdx.x == 0) *es.ctr = 0u;
 }
 
 __global__ void __launch_bounds__(FK_BLOCK) k_rbe_finalize_k(FinalizeArgs a) {
-  finalize_k_body(a, blockIdx.x, gridDim.x);
+  finalize_k_body(a, blockIdx.x);
 }
 
 __global__ void __launch_bounds__(FK_BLOCK)
 k_rbe_finalize_k_batch(const FinalizeArgs* __restrict__ a, const int* __restrict__ start,
                        int nrep) {
   const int r = batch_replica(start, nrep, blockIdx.x);
-  const int b0 = __ldg(start + r);
-  finalize_k_body(a[r], blockIdx.x - b0, __ldg(start + r + 1) - b0);
+  finalize_k_body(a[r], blockIdx.x - __ldg(start + r));
 }
 
 // Block k's part of the finalize (all threads of the block call it).
@@ -573,29 +583,57 @@ __device__ void rbe_finalize_one(int k, int p, int nparts, const double* __restr
                                  double qqr2e, double* __restrict__ rho_re,
                                  double* __restrict__ rho_im, KTab* __restrict__ tab,
                                  double* __restrict__ kterm, double* sh) {
+  // a chain of latencies: every load is issued before the sums, the per-k
+  // constants (their FP64 divides) are formed while the loads are in flight,
+  // and one barrier serves both sums
+  constexpr int U = 8;
   double r = 0.0, im = 0.0;
   const double* pr = part_re + (size_t)k * nparts;
   const double* pi = part_im + (size_t)k * nparts;
-  for (int b = threadIdx.x; b < nparts; b += FK_BLOCK) {
-    r += pr[b];
-    im += pi[b];
-  }
-  r = block_sum_det<FK_BLOCK>(r, sh);
-  im = block_sum_det<FK_BLOCK>(im, sh);
-  if (threadIdx.x != 0) return;
-  if (rho_re) {
-    rho_re[k] = r;
-    rho_im[k] = im;
+  for (int b0 = threadIdx.x; b0 < nparts; b0 += U * FK_BLOCK) {
+    double vr[U], vi[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int b = b0 + u * FK_BLOCK;
+      vr[u] = b < nparts ? pr[b] : 0.0;
+      vi[u] = b < nparts ? pi[b] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      r += vr[u];
+      im += vi[u];
+    }
   }
   const double V = Lx * Ly * Lz;
   const double kx = 2 * RBX_PI * mx[k] / Lx;
   const double ky = 2 * RBX_PI * my[k] / Ly;
   const double kz = 2 * RBX_PI * mz[k] / Lz;
   const double k2 = kx * kx + ky * ky + kz * kz;
+  const double c = (-4 * RBX_PI * qqr2e * S / p) / (V * k2);
+  const double e_scale = (2 * RBX_PI * S) / (p * V) / k2;
+  const double inner = (1.0 / (4 * alpha)) + (1.0 / k2);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    r += __shfl_down_sync(0xffffffffu, r, o);
+    im += __shfl_down_sync(0xffffffffu, im, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    sh[threadIdx.x >> 5] = r;
+    sh[FK_BLOCK / 32 + (threadIdx.x >> 5)] = im;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+#pragma unroll
+  for (int w = 1; w < FK_BLOCK / 32; ++w) {
+    r += sh[w];
+    im += sh[FK_BLOCK / 32 + w];
+  }
+  if (rho_re) {
+    rho_re[k] = r;
+    rho_im[k] = im;
+  }
   if (kterm) {
-    const double coef = (2 * RBX_PI * S) / (p * V);
-    const double base = coef * (r * r + im * im) / k2;
-    const double inner = (1.0 / (4 * alpha)) + (1.0 / k2);
+    const double base = e_scale * (r * r + im * im);
     double* t = kterm + (size_t)k * 8;
     t[0] = base;
     t[1] = base * (1.0 - 2 * kx * kx * inner);
@@ -606,7 +644,6 @@ __device__ void rbe_finalize_one(int k, int p, int nparts, const double* __restr
     t[6] = base * (-2 * ky * kz * inner);
   }
   if (tab) {
-    const double c = (-4 * RBX_PI * qqr2e * S / p) / (V * k2);
     KTab t;
     t.kx = kx;
     t.ky = ky;
@@ -622,11 +659,6 @@ __device__ void rbe_finalize_one(int k, int p, int nparts, const double* __restr
     t.md[2] = mz[k];
     tab[k] = t;
   }
-}
-
-__global__ void __launch_bounds__(32)
-k_rbe_energy_sum(int p, const double* __restrict__ kterm, EnergySum es) {
-  rbe_energy_sum_warp(p, kterm, es, false);
 }
 
 // ---------------------------------------------------------------------------
@@ -655,6 +687,7 @@ struct ForceEpilogue {
   const int* type;
   const double* inv_mass;  // per type
   double half_dt;
+  EnergyJob job;           // the launch's last block, when there is one
 };
 
 __device__ __forceinline__ void force_epilogue(const ForceEpilogue& ep, int i, double fx,
@@ -726,6 +759,10 @@ __global__ void __launch_bounds__(FB)
 k_rbe_force_f64(int n, int p, double Lx, double Ly, double Lz, const KTab* __restrict__ tab,
                 const double* __restrict__ q, const double* __restrict__ x,
                 const double* __restrict__ y, const double* __restrict__ z, ForceEpilogue ep) {
+  if (ep.job.kind != EnergyJob::NONE && blockIdx.x == gridDim.x - 1) {
+    if (threadIdx.x < 32) energy_job(ep.job);
+    return;
+  }
   __shared__ KTabD s_tab[FRC_TABLE];
   __shared__ double s_x[FB], s_y[FB], s_z[FB];  // positions in quarter turns, then forces
   __shared__ unsigned short s_list[FB];
@@ -801,8 +838,13 @@ struct ForceMixedArgs {
   ForceEpilogue ep;
 };
 
+// Block bx of a grid of gx blocks.
 template <int FB>
-__device__ __forceinline__ void force_mixed_body(const ForceMixedArgs& A, int bx) {
+__device__ __forceinline__ void force_mixed_body(const ForceMixedArgs& A, int bx, int gx) {
+  if (A.ep.job.kind != EnergyJob::NONE && bx == gx - 1) {
+    if (threadIdx.x < 32) energy_job(A.ep.job);
+    return;
+  }
   const int n = A.n, p = A.p;
   const KTab* __restrict__ tab = A.tab;
   const uint4* __restrict__ atoms = A.atoms;
@@ -880,7 +922,7 @@ __device__ __forceinline__ void force_mixed_body(const ForceMixedArgs& A, int bx
 
 template <int FB>
 __global__ void __launch_bounds__(FB) k_rbe_force_mixed(ForceMixedArgs a) {
-  force_mixed_body<FB>(a, blockIdx.x);
+  force_mixed_body<FB>(a, blockIdx.x, gridDim.x);
 }
 
 template <int FB>
@@ -888,7 +930,8 @@ __global__ void __launch_bounds__(FB)
 k_rbe_force_mixed_batch(const ForceMixedArgs* __restrict__ a, const int* __restrict__ start,
                         int nrep) {
   const int r = batch_replica(start, nrep, blockIdx.x);
-  force_mixed_body<FB>(a[r], blockIdx.x - __ldg(start + r));
+  const int b0 = __ldg(start + r);
+  force_mixed_body<FB>(a[r], blockIdx.x - b0, __ldg(start + r + 1) - b0);
 }
 
 // ---------------------------------------------------------------------------
@@ -1145,7 +1188,7 @@ int launch_rbe_finalize(const DBox& b, int p, int nparts, const double* part_re,
                         double qsum, double* rho_re, double* rho_im, double* energy,
                         double* virial, KTab* tab, int mean_parts, const double* fpart,
                         int n_atoms, double* mean_out, double* kterm, cudaStream_t st,
-                        unsigned* sum_ctr) {
+                        EnergyJob* job) {
   if (energy && !kterm) {  // no per-k scratch: one block does it all
     k_rbe_finalize<<<1, FIN_WIDE, 0, st>>>(p, nparts, part_re, part_im, mx, my, mz, b.len[0],
                                             b.len[1], b.len[2], alpha, S, qqr2e, qsq, qsum,
@@ -1155,9 +1198,20 @@ int launch_rbe_finalize(const DBox& b, int p, int nparts, const double* part_re,
     return check_launch("rbe_finalize");
   }
   const int grid = p + (mean_out ? 3 : 0);
-  EnergySum es{nullptr, alpha, b.len[0] * b.len[1] * b.len[2], qqr2e, qsq, qsum, energy, virial};
-  // the energy sum in the finalize's last block when a counter is given
-  const bool fold = energy && sum_ctr && grid > 0 && p > 0;
+  EnergyJob sum;
+  if (energy) {
+    sum.kind = EnergyJob::RBE;
+    sum.p = p;
+    sum.kterm = kterm;
+    sum.alpha = alpha;
+    sum.V = b.len[0] * b.len[1] * b.len[2];
+    sum.qqr2e = qqr2e;
+    sum.qsq = qsq;
+    sum.qsum = qsum;
+    sum.energy = energy;
+    sum.virial = virial;
+  }
+  if (job) *job = sum;
   if (grid > 0) {
     FinalizeArgs a;
     a.p = p;
@@ -1181,11 +1235,9 @@ int launch_rbe_finalize(const DBox& b, int p, int nparts, const double* part_re,
     a.fpart = fpart;
     a.n_atoms = (double)n_atoms;
     a.mean_out = mean_out;
-    a.es = es;
-    a.es.ctr = fold ? sum_ctr : nullptr;
     if (batch_recorder()) {
-      if (energy && !fold) {
-        set_error("rbe_finalize: a batched finalize needs the energy sum folded in");
+      if (energy && !job) {
+        set_error("rbe_finalize: a batched finalize leaves the energy sum to the force pass");
         return RBX_ERR_INVALID;
       }
       return record_phase(PH_FINALIZE, 0, grid, FK_BLOCK, 0, &a, sizeof a);
@@ -1195,11 +1247,7 @@ int launch_rbe_finalize(const DBox& b, int p, int nparts, const double* part_re,
     const int rc = check_launch("rbe_finalize_k");
     if (rc) return rc;
   }
-  if (energy && !fold) {
-    k_rbe_energy_sum<<<1, 32, 0, st>>>(p, kterm, es);
-    count_launch();
-  }
-  return check_launch("rbe_energy_sum");
+  return energy && !job ? launch_energy_sum(sum, st) : RBX_OK;
 }
 
 static ForceEpilogue make_ep(const RbeForceOut& o) {
@@ -1220,6 +1268,7 @@ static ForceEpilogue make_ep(const RbeForceOut& o) {
   ep.type = o.type;
   ep.inv_mass = o.inv_mass;
   ep.half_dt = o.half_dt;
+  ep.job = o.job;
   return ep;
 }
 
@@ -1227,24 +1276,22 @@ static ForceEpilogue make_ep(const RbeForceOut& o) {
 int launch_rbe_force_f64(const DBox& b, int n, int p, const KTab* tab, const double* q,
                          const double* x, const double* y, const double* z,
                          const RbeForceOut& out, cudaStream_t st, int block) {
-  if (n <= 0) return RBX_OK;
+  const int extra = out.job.kind != EnergyJob::NONE;  // the energy's block
+  if (n <= 0) return extra ? launch_energy_sum(out.job, st) : RBX_OK;
   const ForceEpilogue ep = make_ep(out);
-  if (block == 128)
-    k_rbe_force_f64<128><<<(n + 127) / 128, 128, 0, st>>>(n, p, b.len[0], b.len[1], b.len[2], tab, q,
-                                                        x, y, z, ep);
-  else if (block == 512)
-    k_rbe_force_f64<512><<<(n + 511) / 512, 512, 0, st>>>(n, p, b.len[0], b.len[1], b.len[2], tab, q,
-                                                        x, y, z, ep);
-  else
-    k_rbe_force_f64<256><<<(n + 255) / 256, 256, 0, st>>>(n, p, b.len[0], b.len[1], b.len[2], tab, q,
-                                                        x, y, z, ep);
+  if (block != 128 && block != 512) block = 256;
+  const auto kern = block == 128 ? k_rbe_force_f64<128>
+                                 : (block == 512 ? k_rbe_force_f64<512> : k_rbe_force_f64<256>);
+  kern<<<(n + block - 1) / block + extra, block, 0, st>>>(n, p, b.len[0], b.len[1], b.len[2], tab,
+                                                          q, x, y, z, ep);
   count_launch();
   return check_launch("rbe_force_f64");
 }
 
 int launch_rbe_force_mixed(int n, int p, const KTab* tab, const uint4* atoms,
                            const RbeForceOut& out, cudaStream_t st, int block) {
-  if (n <= 0) return RBX_OK;
+  const int extra = out.job.kind != EnergyJob::NONE;  // the energy's block
+  if (n <= 0) return extra ? launch_energy_sum(out.job, st) : RBX_OK;
   ForceMixedArgs a;
   a.n = n;
   a.p = p;
@@ -1252,14 +1299,11 @@ int launch_rbe_force_mixed(int n, int p, const KTab* tab, const uint4* atoms,
   a.atoms = atoms;
   a.ep = make_ep(out);
   if (block != 128 && block != 512) block = 256;
-  if (batch_recorder())
-    return record_phase(PH_FORCE, block, (n + block - 1) / block, block, 0, &a, sizeof a);
-  if (block == 128)
-    k_rbe_force_mixed<128><<<(n + 127) / 128, 128, 0, st>>>(a);
-  else if (block == 512)
-    k_rbe_force_mixed<512><<<(n + 511) / 512, 512, 0, st>>>(a);
-  else
-    k_rbe_force_mixed<256><<<(n + 255) / 256, 256, 0, st>>>(a);
+  const int grid = (n + block - 1) / block + extra;
+  if (batch_recorder()) return record_phase(PH_FORCE, block, grid, block, 0, &a, sizeof a);
+  const auto kern = block == 128 ? k_rbe_force_mixed<128>
+                                 : (block == 512 ? k_rbe_force_mixed<512> : k_rbe_force_mixed<256>);
+  kern<<<grid, block, 0, st>>>(a);
   count_launch();
   return check_launch("rbe_force_mixed");
 }

@@ -227,28 +227,6 @@ k_rbsog_finalize(int p, int nparts, const double* __restrict__ part_re,
   }
 }
 
-// Energy: one warp adds the per-k terms in increasing k, then the self term;
-// the virial terms likewise when vterm is given.
-__global__ void __launch_bounds__(32)
-k_rbsog_energy_sum(int p, const double* __restrict__ kterm, double self_energy,
-                   double* __restrict__ energy, const double* __restrict__ vterm,
-                   double* __restrict__ virial) {
-  if (energy) {
-    double t = 0.0;
-    for (int k = threadIdx.x; k < p; k += 32) t += kterm[k];
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-    if (threadIdx.x == 0) *energy = t + self_energy;
-  }
-  if (vterm) {
-    for (int c = 0; c < 6; ++c) {
-      double t = 0.0;
-      for (int k = threadIdx.x; k < p; k += 32) t += vterm[6 * (size_t)k + c];
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-      if (threadIdx.x == 0) virial[c] = t;
-    }
-  }
-}
-
 // VERLET-SOG pair force (ComputeLJCutCoulForceUserKernel with lj126 and
 // CoulCutForceUser, lj_cut_coul_kspace_op.hip.cu:196-254, 357-470): for
 // r^2 < cut_off^2, the LJ 12-6 force plus the short-range SOG Coulomb force
@@ -416,7 +394,7 @@ int launch_rbsog_finalize(const DBox& b, int p, int nparts, const double* part_r
                           const double* mz, const double4* w, double* rho_re, double* rho_im,
                           KTab* tab, double* kterm, double self_energy, double* energy,
                           int mean_parts, const double* fpart, int n_atoms, double* mean_out,
-                          cudaStream_t st, const SogVirial* vir) {
+                          cudaStream_t st, const SogVirial* vir, EnergyJob* job) {
   const int grid = p + (mean_out ? 3 : 0);
   const SogVirial v = vir ? *vir : SogVirial{0, nullptr, nullptr, nullptr, nullptr};
   if (grid > 0) {
@@ -427,12 +405,18 @@ int launch_rbsog_finalize(const DBox& b, int p, int nparts, const double* part_r
     const int rc = check_launch("rbsog_finalize");
     if (rc) return rc;
   }
+  EnergyJob sum;
   if (energy || v.vterm) {
-    k_rbsog_energy_sum<<<1, 32, 0, st>>>(p, kterm, self_energy, energy, v.vterm, v.out);
-    count_launch();
-    return check_launch("rbsog_energy_sum");
+    sum.kind = EnergyJob::RBSOG;
+    sum.p = p;
+    sum.kterm = kterm;
+    sum.vterm = v.vterm;
+    sum.self_energy = self_energy;
+    sum.energy = energy;
+    sum.virial = v.out;
   }
-  return RBX_OK;
+  if (job) *job = sum;
+  return sum.kind != EnergyJob::NONE && !job ? launch_energy_sum(sum, st) : RBX_OK;
 }
 
 int launch_rbsog_npt_chain(const DBox& b, int p, const double* mx, const double* my,
