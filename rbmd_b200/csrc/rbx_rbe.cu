@@ -662,9 +662,11 @@ __device__ void rbe_finalize_one(int k, int p, int nparts, const double* __restr
 }
 
 // ---------------------------------------------------------------------------
-// Force scatter over the charged atoms of a block: one thread an atom where
-// most are charged, otherwise the idle threads share the atoms' k-vectors
-// (partial sums meet in shuffles).  The k table is staged in shared memory.
+// Force scatter over the charged atoms of a block, compacted onto its first
+// threads.  FP64: where few are charged, the idle threads share the atoms'
+// k-vectors (partial sums meet in shuffles).  Mixed: one thread an atom, k in
+// increasing order, since FP32 sums in another order move a force by 1e-7.  The
+// k table is staged in shared memory.
 // Epilogue variants: plain store of F_k, or the fused combine
 // F = F_pair - mean + F_k with the second velocity-Verlet half kick.
 // ---------------------------------------------------------------------------
@@ -860,10 +862,8 @@ __device__ __forceinline__ void force_mixed_body(const ForceMixedArgs& A, int bx
   const bool take = __uint_as_float(ai.w) != 0.f;
   if (take) s_atom[threadIdx.x] = ai;
   const int count = block_compact<FB>(take, s_list, s_cnt);
-  const int share = threads_per_atom<FB>(count);
-  const int slot = (int)threadIdx.x / share, part = (int)threadIdx.x % share;
-  const bool mine = slot < count;
-  const int own = mine ? s_list[slot] : 0;
+  const bool mine = (int)threadIdx.x < count;
+  const int own = mine ? s_list[threadIdx.x] : 0;
   const uint4 a = mine ? s_atom[own] : make_uint4(0, 0, 0, 0);
   const float ang = (float)(2.0 * RBX_PI / 4294967296.0);
   float fx = 0.f, fy = 0.f, fz = 0.f;
@@ -885,7 +885,8 @@ __device__ __forceinline__ void force_mixed_body(const ForceMixedArgs& A, int bx
     }
     __syncthreads();
     if (mine) {
-      auto add = [&](int s) {
+#pragma unroll 4
+      for (int s = 0; s < kn; ++s) {
         const KTabF t = s_tab[s];
         const unsigned ph = (unsigned)t.m0 * a.x + (unsigned)t.m1 * a.y + (unsigned)t.m2 * a.z;
         float sn, cs;
@@ -894,19 +895,10 @@ __device__ __forceinline__ void force_mixed_body(const ForceMixedArgs& A, int bx
         fx = fmaf(f, t.kx, fx);
         fy = fmaf(f, t.ky, fy);
         fz = fmaf(f, t.kz, fz);
-      };
-      if (share == 1)
-        for (int s = 0; s < kn; ++s) add(s);
-      else
-        for (int s = part; s < kn; s += share) add(s);
+      }
     }
   }
-  for (int o = share >> 1; o > 0; o >>= 1) {  // a share never crosses a warp
-    fx += __shfl_xor_sync(0xffffffffu, fx, o);
-    fy += __shfl_xor_sync(0xffffffffu, fy, o);
-    fz += __shfl_xor_sync(0xffffffffu, fz, o);
-  }
-  if (mine && part == 0) {
+  if (mine) {
     s_f[0][own] = fx;
     s_f[1][own] = fy;
     s_f[2][own] = fz;
