@@ -500,13 +500,10 @@ int rbx_fix_rbl_force(int num_atoms, double* fx, double* fy, double* fz, double*
   }
   RBX_TRY(require_device());
   cudaStream_t st = (cudaStream_t)stream;
-  double* mean = mean_out;
-  if (!mean) RBX_TRY(async_alloc(&mean, 3, st));
-  int rc = launch_reduce_cols(num_atoms, 1, fx, mean, 1.0 / num_atoms, st);
-  if (!rc) rc = launch_reduce_cols(num_atoms, 1, fy, mean + 1, 1.0 / num_atoms, st);
-  if (!rc) rc = launch_reduce_cols(num_atoms, 1, fz, mean + 2, 1.0 / num_atoms, st);
-  if (!rc) rc = launch_sub_mean(num_atoms, fx, fy, fz, mean, st);
-  if (!mean_out) cudaFreeAsync(mean, st);
+  double* part = nullptr;
+  RBX_TRY(async_alloc(&part, (size_t)3 * fix_rbl_parts(num_atoms), st));
+  const int rc = launch_fix_rbl(num_atoms, fx, fy, fz, mean_out, part, st);
+  cudaFreeAsync(part, st);
   return rc;
 }
 

@@ -22,26 +22,49 @@
 
 namespace rbx {
 
-__global__ void k_widen(int n, const float* __restrict__ src, double* __restrict__ dst) {
+// Up to eight float arrays of one length widened into consecutive runs of
+// dst, in one launch (blockIdx.y: the array).
+struct FloatSet {
+  const float* src[8];
+};
+__global__ void k_widen(int n, FloatSet s, double* __restrict__ dst) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = (double)src[i];
+  if (i < n) dst[(size_t)n * blockIdx.y + i] = (double)s.src[blockIdx.y][i];
 }
-__global__ void k_narrow(int n, const double* __restrict__ src, float* __restrict__ dst) {
+// Consecutive runs of src narrowed into up to eight float arrays.
+struct FloatOut {
+  float* dst[8];
+};
+__global__ void k_narrow(int n, const double* __restrict__ src, FloatOut o) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = (float)src[i];
+  if (i < n) o.dst[blockIdx.y][i] = (float)src[(size_t)n * blockIdx.y + i];
 }
 
-int launch_widen(int n, const float* src, double* dst, cudaStream_t st) {
-  if (n <= 0) return RBX_OK;
-  k_widen<<<(n + 255) / 256, 256, 0, st>>>(n, src, dst);
-  count_launch();
-  return check_launch("widen");
-}
-int launch_narrow(int n, const double* src, float* dst, cudaStream_t st) {
-  if (n <= 0) return RBX_OK;
-  k_narrow<<<(n + 255) / 256, 256, 0, st>>>(n, src, dst);
-  count_launch();
-  return check_launch("narrow");
+// Fixed-point records {u_x, u_y, u_z, q} of float positions and charges, and
+// (in the blocks after the atoms') the k-vectors and any further p-element
+// arrays widened, the integer k-vectors: one launch prepares a whole call.
+constexpr int PREP_BLOCK = 256;
+__global__ void __launch_bounds__(PREP_BLOCK)
+k_prepare_f32(DBox b, int n, const float* __restrict__ q, const float* __restrict__ x,
+              const float* __restrict__ y, const float* __restrict__ z, uint4* __restrict__ atoms,
+              int p, int narr, FloatSet s, double* __restrict__ wide, int* __restrict__ mi) {
+  const int blocks_n = (n + PREP_BLOCK - 1) / PREP_BLOCK;
+  if ((int)blockIdx.x < blocks_n) {
+    const int i = blockIdx.x * PREP_BLOCK + threadIdx.x;
+    if (i >= n) return;
+    uint4 a;
+    a.x = to_fixed((double)x[i], b.lo[0], 4294967296.0 / b.len[0]);
+    a.y = to_fixed((double)y[i], b.lo[1], 4294967296.0 / b.len[1]);
+    a.z = to_fixed((double)z[i], b.lo[2], 4294967296.0 / b.len[2]);
+    a.w = __float_as_uint(q[i]);
+    atoms[i] = a;
+    return;
+  }
+  const int k = ((int)blockIdx.x - blocks_n) * PREP_BLOCK + threadIdx.x;
+  if (k >= p) return;
+  for (int a = 0; a < narr; ++a) wide[(size_t)p * a + k] = (double)s.src[a][k];
+  if (mi)
+    for (int d = 0; d < 3; ++d) mi[3 * k + d] = (int)s.src[d][k];
 }
 
 namespace {
@@ -64,21 +87,41 @@ struct Scratch {
 
 // Widened copies of n-element float arrays (contiguous, in argument order).
 int widen_all(Scratch& s, int n, std::initializer_list<const float*> src, double** dst) {
-  double* w = nullptr;
-  RBX_TRY(s.get(&w, (size_t)n * src.size()));
-  *dst = w;
+  RBX_TRY(s.get(dst, (size_t)n * src.size()));
+  FloatSet fs{};
   int k = 0;
-  for (const float* a : src) RBX_TRY(launch_widen(n, a, w + (size_t)n * k++, s.st));
-  return RBX_OK;
+  for (const float* a : src) fs.src[k++] = a;
+  k_widen<<<dim3((n + 255) / 256, k), 256, 0, s.st>>>(n, fs, *dst);
+  count_launch();
+  return check_launch("widen");
 }
 
-// Fixed-point records {u_x, u_y, u_z, q} of float positions and charges.
-int fixed_records(Scratch& s, const DBox& b, int n, const float* q, const float* x,
-                  const float* y, const float* z, uint4** atoms) {
-  double* w = nullptr;
-  RBX_TRY(widen_all(s, n, {x, y, z, q}, &w));
+int launch_narrow(int n, const double* src, std::initializer_list<float*> dst, cudaStream_t st) {
+  if (n <= 0) return RBX_OK;
+  FloatOut o{};
+  int k = 0;
+  for (float* a : dst) o.dst[k++] = a;
+  k_narrow<<<dim3((n + 255) / 256, k), 256, 0, st>>>(n, src, o);
+  count_launch();
+  return check_launch("narrow");
+}
+
+// Records of n atoms, p-element arrays widened (the first three are the
+// k-vectors) and, with want_mi, the integer k-vectors.
+int prepare(Scratch& s, const DBox& b, int n, const float* q, const float* x, const float* y,
+            const float* z, uint4** atoms, int p, std::initializer_list<const float*> src,
+            double** wide, int** mi) {
   RBX_TRY(s.get(atoms, (size_t)n));
-  return launch_to_fixed(b, n, w, w + n, w + 2 * (size_t)n, w + 3 * (size_t)n, *atoms, s.st);
+  RBX_TRY(s.get(wide, (size_t)p * src.size()));
+  if (mi) RBX_TRY(s.get(mi, (size_t)3 * p));
+  FloatSet fs{};
+  int k = 0;
+  for (const float* a : src) fs.src[k++] = a;
+  const int grid = (n + PREP_BLOCK - 1) / PREP_BLOCK + (p + PREP_BLOCK - 1) / PREP_BLOCK;
+  k_prepare_f32<<<grid, PREP_BLOCK, 0, s.st>>>(b, n, q, x, y, z, *atoms, p, k, fs, *wide,
+                                               mi ? *mi : nullptr);
+  count_launch();
+  return check_launch("prepare_f32");
 }
 }  // namespace
 }  // namespace rbx
@@ -103,7 +146,6 @@ int rbx_rbe_structure_factor_f32(const rbx_box* box, int num_atoms, int p_number
   Scratch s(st);
   const DBox b = make_dbox(*box);
   double* m = nullptr;  // samples widened: mx, my, mz
-  RBX_TRY(widen_all(s, p_number, {p_sample_x, p_sample_y, p_sample_z}, &m));
   const int nb = rbe_partial_blocks(num_atoms);
   double *part = nullptr, *rho = nullptr;
   RBX_TRY(s.get(&part, (size_t)2 * nb * p_number));
@@ -112,18 +154,17 @@ int rbx_rbe_structure_factor_f32(const rbx_box* box, int num_atoms, int p_number
   if (num_atoms > 0) {
     uint4* atoms = nullptr;
     int* mi = nullptr;
-    RBX_TRY(fixed_records(s, b, num_atoms, charge, px, py, pz, &atoms));
-    RBX_TRY(s.get(&mi, (size_t)3 * p_number));
-    RBX_TRY(launch_m_to_int(p_number, m, m + p_number, m + 2 * p_number, mi, st));
+    RBX_TRY(prepare(s, b, num_atoms, charge, px, py, pz, &atoms, p_number,
+                    {p_sample_x, p_sample_y, p_sample_z}, &m, &mi));
     RBX_TRY(launch_rbe_rho_partial_mixed(num_atoms, p_number, mi, atoms, pr, pi, nb, st));
   } else {
+    RBX_TRY(widen_all(s, p_number, {p_sample_x, p_sample_y, p_sample_z}, &m));
     cudaMemsetAsync(part, 0, sizeof(double) * 2 * nb * p_number, st);
   }
   RBX_TRY(launch_rbe_finalize(b, p_number, nb, pr, pi, m, m + p_number, m + 2 * p_number, 1.0,
                               0.0, 1.0, 0.0, 0.0, rho, rho + p_number, nullptr, nullptr, nullptr,
                               0, nullptr, 0, nullptr, nullptr, st));
-  RBX_TRY(launch_narrow(p_number, rho, density_real, st));
-  return launch_narrow(p_number, rho + p_number, density_imag, st);
+  return launch_narrow(p_number, rho, {density_real, density_imag}, st);
 }
 
 int rbx_rbe_force_f32(const rbx_box* box, int num_atoms, int p_number, float alpha,
@@ -142,26 +183,24 @@ int rbx_rbe_force_f32(const rbx_box* box, int num_atoms, int p_number, float alp
   cudaStream_t st = (cudaStream_t)stream;
   Scratch s(st);
   const DBox b = make_dbox(*box);
-  double *m = nullptr, *rho = nullptr, *f = nullptr;
-  RBX_TRY(widen_all(s, p_number, {p_sample_x, p_sample_y, p_sample_z}, &m));
-  RBX_TRY(widen_all(s, p_number, {real_array, imag_array}, &rho));
+  double *m = nullptr, *f = nullptr;
+  uint4* atoms = nullptr;
+  RBX_TRY(prepare(s, b, num_atoms, charge, px, py, pz, &atoms, p_number,
+                  {p_sample_x, p_sample_y, p_sample_z, real_array, imag_array}, &m, nullptr));
+  const double* rho = m + 3 * (size_t)p_number;
   KTab* tab = nullptr;
   RBX_TRY(s.get(&tab, (size_t)p_number));
   RBX_TRY(launch_rbe_finalize(b, p_number, 1, rho, rho + p_number, m, m + p_number,
                               m + 2 * p_number, alpha, rbe_sum_gauss, qqr2e, 0.0, 0.0, nullptr,
                               nullptr, nullptr, nullptr, tab, 0, nullptr, 0, nullptr, nullptr,
                               st));
-  uint4* atoms = nullptr;
-  RBX_TRY(fixed_records(s, b, num_atoms, charge, px, py, pz, &atoms));
   RBX_TRY(s.get(&f, (size_t)3 * num_atoms));
   RbeForceOut o;
   o.f_out_x = f;
   o.f_out_y = f + num_atoms;
   o.f_out_z = f + 2 * (size_t)num_atoms;
   RBX_TRY(launch_rbe_force_mixed(num_atoms, p_number, tab, atoms, o, st));
-  RBX_TRY(launch_narrow(num_atoms, o.f_out_x, fx, st));
-  RBX_TRY(launch_narrow(num_atoms, o.f_out_y, fy, st));
-  return launch_narrow(num_atoms, o.f_out_z, fz, st);
+  return launch_narrow(num_atoms, f, {fx, fy, fz}, st);
 }
 
 int rbx_rbe_energy_virial_f32(const rbx_box* box, int p, float alpha, float rbe_sum_gauss,
@@ -178,15 +217,15 @@ int rbx_rbe_energy_virial_f32(const rbx_box* box, int p, float alpha, float rbe_
   cudaStream_t st = (cudaStream_t)stream;
   Scratch s(st);
   const DBox b = make_dbox(*box);
-  double *m = nullptr, *rho = nullptr, *out = nullptr;
-  RBX_TRY(widen_all(s, p, {p_sample_x, p_sample_y, p_sample_z}, &m));
-  RBX_TRY(widen_all(s, p, {real_array, imag_array}, &rho));
+  double *m = nullptr, *out = nullptr;
+  RBX_TRY(widen_all(s, p, {p_sample_x, p_sample_y, p_sample_z, real_array, imag_array}, &m));
+  const double* rho = m + 3 * (size_t)p;
   RBX_TRY(s.get(&out, 7));  // virial[6], energy
   RBX_TRY(launch_rbe_finalize(b, p, 1, rho, rho + p, m, m + p, m + 2 * p, alpha, rbe_sum_gauss,
                               qqrd2e, qsqsum, qsum, nullptr, nullptr, out + 6, out, nullptr, 0,
                               nullptr, 0, nullptr, nullptr, st));
-  RBX_TRY(launch_narrow(6, out, virial_tensor, st));
-  return launch_narrow(1, out + 6, energy, st);
+  RBX_TRY(launch_narrow(6, out, {virial_tensor}, st));
+  return launch_narrow(1, out + 6, {energy}, st);
 }
 
 int rbx_rbl_filter_f32(float core_cutoff_2, float force_cutoff_2, int total_atom_num,
@@ -242,14 +281,9 @@ int rbx_fix_rbl_force_f32(int num_atoms, float* fx, float* fy, float* fz, float*
   RBX_TRY(require_device());
   cudaStream_t st = (cudaStream_t)stream;
   Scratch s(st);
-  double* mean = nullptr;
-  RBX_TRY(s.get(&mean, 3));
-  RBX_TRY(launch_reduce_cols(num_atoms, 1, fx, mean, 1.0 / num_atoms, st));
-  RBX_TRY(launch_reduce_cols(num_atoms, 1, fy, mean + 1, 1.0 / num_atoms, st));
-  RBX_TRY(launch_reduce_cols(num_atoms, 1, fz, mean + 2, 1.0 / num_atoms, st));
-  RBX_TRY(launch_sub_mean(num_atoms, fx, fy, fz, mean, st));
-  if (mean_out) RBX_TRY(launch_narrow(3, mean, mean_out, st));
-  return RBX_OK;
+  double* part = nullptr;
+  RBX_TRY(s.get(&part, (size_t)3 * fix_rbl_parts(num_atoms)));
+  return launch_fix_rbl(num_atoms, fx, fy, fz, mean_out, part, st);
 }
 
 int rbx_pair_force_verlet_f32(const rbx_box* box, float cut_off, int num_atoms, float alpha,
@@ -275,8 +309,8 @@ int rbx_pair_force_verlet_f32(const rbx_box* box, float cut_off, int num_atoms, 
                                  sigma, eps, start_id, end_id, id_verletlist, charge, px, py, pz,
                                  fx, fy, fz, flat_virial, epart, st));
   RBX_TRY(launch_reduce_cols(num_atoms, 2, epart, tot, 1.0, st));
-  if (total_evdwl) RBX_TRY(launch_narrow(1, tot, total_evdwl, st));
-  if (total_ecoul) RBX_TRY(launch_narrow(1, tot + 1, total_ecoul, st));
+  if (total_evdwl) RBX_TRY(launch_narrow(1, tot, {total_evdwl}, st));
+  if (total_ecoul) RBX_TRY(launch_narrow(1, tot + 1, {total_ecoul}, st));
   return RBX_OK;
 }
 

@@ -85,8 +85,9 @@ int launch_rbe_finalize(const DBox& b, int p, int nparts, const double* part_re,
                         double* virial, KTab* tab, int mean_parts, const double* fpart,
                         int n_atoms, double* mean_out, double* kterm, cudaStream_t st,
                         EnergyJob* job = nullptr);
-// kterm: scratch of 8 p doubles for the per-k energy/virial terms (parallel
-// finalize); when null and energy is requested, one block does the finalize.
+// kterm: scratch of 8 p doubles for the per-k energy/virial terms; when null and
+// energy is requested, the structure factors are given (nparts = 1) and one block
+// sums their terms.
 // job: the sum over k is not launched here but described for the force pass.
 int launch_energy_sum(const EnergyJob& job, cudaStream_t st);
 int launch_rbe_force_f64(const DBox& b, int n, int p, const KTab* tab, const double* q,
@@ -232,16 +233,14 @@ int launch_ref_pair_verlet(const DBox& b, float cut_off, int n, double alpha, do
                            cudaStream_t st);
 int launch_reduce_cols(int n, int ncols, const float* cols, double* out, double scale,
                        cudaStream_t st);
-int launch_sub_mean(int n, float* fx, float* fy, float* fz, const double* mean,
-                    cudaStream_t st);
-// Element-wise conversions between float and double device arrays.
-int launch_widen(int n, const float* src, double* dst, cudaStream_t st);
-int launch_narrow(int n, const double* src, float* dst, cudaStream_t st);
+int launch_fix_rbl(int n, float* fx, float* fy, float* fz, float* mean_out, double* part,
+                   cudaStream_t st);
 int launch_sum_i32(int n, const int* src, long long* out, cudaStream_t st);
 int launch_reduce_cols(int n, int ncols, const double* cols, double* out, double scale,
                        cudaStream_t st);
-int launch_sub_mean(int n, double* fx, double* fy, double* fz, const double* mean,
-                    cudaStream_t st);
+int fix_rbl_parts(int n);
+int launch_fix_rbl(int n, double* fx, double* fy, double* fz, double* mean_out, double* part,
+                   cudaStream_t st);
 
 // ---- cells, lists, integration (rbx_cells.cu) ----
 // Bookkeeping of an engine rebuild folded into its kernels (each member may be

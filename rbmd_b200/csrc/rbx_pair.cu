@@ -742,6 +742,14 @@ __device__ __forceinline__ double ref_list_d2(double dx, double dy, double dz) {
 __device__ __forceinline__ float ref_list_d2(float dx, float dy, float dz) {
   return __fadd_rn(__fadd_rn(powf(dx, 2.f), powf(dy, 2.f)), powf(dz, 2.f));
 }
+// The same with plain products, to screen: powf is within 4 ulp and the
+// products within half of one, so the two differ by less than 1e-6 relative.
+__device__ __forceinline__ double ref_list_d2_fast(double dx, double dy, double dz) {
+  return ref_list_d2(dx, dy, dz);
+}
+__device__ __forceinline__ float ref_list_d2_fast(float dx, float dy, float dz) {
+  return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+}
 template <typename T>
 struct RefLen {
   T len[3];
@@ -754,42 +762,86 @@ RefLen<T> ref_len(const DBox& b) {
 }
 
 // FilterRBLNeighborCandidates semantics (rbl_full_neighbor_list_op.hip.cu:237-304).
-template <typename T>
-__global__ void k_ref_rbl_filter(T core2, T force2, int n, const int* __restrict__ gid,
-                                 const T* __restrict__ x, const T* __restrict__ y,
-                                 const T* __restrict__ z, const int* __restrict__ cstart,
-                                 const int* __restrict__ cend, const int* __restrict__ cand,
-                                 const int* __restrict__ core_cap,
-                                 const int* __restrict__ core_start, int* __restrict__ core_end,
-                                 int* __restrict__ core, int shell_cap, int* __restrict__ shell,
-                                 int* __restrict__ shell_num, int* __restrict__ required,
-                                 RefLen<T> b, int* __restrict__ realloc, DivTest div, int epoch) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// A warp an atom: lanes take consecutive candidates and append their hits
+// through ballot prefixes, so both lists keep the candidates' order.  (One
+// thread an atom walked 485 candidates in series with uncoalesced reads.)
+// Bound by the gathers and the integer work of the hash: 598 -> 177 us for the
+// float build's 50,000 atoms x 485 candidates.
+// FREQ_LOW2: freq is 1, 2 or 4 and the batch test needs two bits of the hash.
+template <typename T, bool FREQ_LOW2>
+__global__ void __launch_bounds__(PAIR_BLOCK)
+k_ref_rbl_filter(T core2, T force2, int n, const int* __restrict__ gid,
+                 const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ z,
+                 const int* __restrict__ cstart, const int* __restrict__ cend,
+                 const int* __restrict__ cand, const int* __restrict__ core_cap,
+                 const int* __restrict__ core_start, int* __restrict__ core_end,
+                 int* __restrict__ core, int shell_cap, int* __restrict__ shell,
+                 int* __restrict__ shell_num, int* __restrict__ required, RefLen<T> b,
+                 int* __restrict__ realloc, DivTest div, int epoch) {
+  constexpr int U = 2;  // candidates a lane takes per iteration
+  const int lane = threadIdx.x & 31;
+  const int i = blockIdx.x * PAIR_WARPS + (int)(threadIdx.x >> 5);
   if (i >= n) return;
+  const unsigned lt = lanemask_lt();
+  const unsigned mask = (1u << div.shift) - 1u;
+  const T band_core = (T)4e-6 * (T)fabs(core2), band_force = (T)4e-6 * (T)fabs(force2);
   const unsigned long long ea = rbl_key_a(gid[i]) ^ (unsigned long long)(long long)epoch;
   int nc = 0, ns = 0;
   const int out0 = core_start[i], ccap = core_cap[i];
   const T xi = x[i], yi = y[i], zi = z[i];
-  for (int pos = cstart[i]; pos < cend[i]; ++pos) {
-    const int j = cand[pos];
-    if (j == i) continue;
-    const T d2 = ref_list_d2(ref_min_image<T>(xi - x[j], b.len[0]),
-                             ref_min_image<T>(yi - y[j], b.len[1]),
-                             ref_min_image<T>(zi - z[j], b.len[2]));
-    if (d2 < core2) {
-      if (nc < ccap)
-        core[out0 + nc] = j;
-      else
-        atomicOr(realloc, 1);
-      ++nc;
-    } else if (d2 < force2 && rbl_selected(ea, rbl_key_b(gid[j]), div)) {
-      if (ns < shell_cap) shell[(size_t)ns * n + i] = j;
-      ++ns;
+  const int c0 = cstart[i], c1 = cend[i];
+  for (int pos = c0; pos < c1; pos += 32 * U) {
+    int j[U];
+    T d2[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = pos + 32 * u + lane;
+      j[u] = k < c1 ? cand[k] : i;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const T dx = ref_min_image<T>(xi - x[j[u]], b.len[0]),
+              dy = ref_min_image<T>(yi - y[j[u]], b.len[1]),
+              dz = ref_min_image<T>(zi - z[j[u]], b.len[2]);
+      d2[u] = ref_list_d2_fast(dx, dy, dz);
+      // float: near a threshold the reference's own powf expression decides
+      if (sizeof(T) == 4 && (fabs(d2[u] - core2) <= band_core || fabs(d2[u] - force2) <= band_force))
+        d2[u] = ref_list_d2(dx, dy, dz);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool other = j[u] != i;
+      const bool in_core = other && d2[u] < core2;
+      bool in_shell = other && !in_core && d2[u] < force2;
+      if (in_shell) {
+        const unsigned long long kb = rbl_key_b(gid[j[u]]);
+        in_shell = FREQ_LOW2 ? rbl_selected_low2(ea ^ kb, mask) : rbl_selected(ea, kb, div);
+      }
+      const unsigned mc = __ballot_sync(0xffffffffu, in_core);
+      const unsigned ms = __ballot_sync(0xffffffffu, in_shell);
+      if (in_core) {
+        const int o = nc + __popc(mc & lt);
+        if (o < ccap) core[out0 + o] = j[u];
+      }
+      if (in_shell) {
+        const int o = ns + __popc(ms & lt);
+        if (o < shell_cap) shell[(size_t)o * n + i] = j[u];
+      }
+      nc += __popc(mc);
+      ns += __popc(ms);
     }
   }
-  core_end[i] = out0 + (nc < ccap ? nc : ccap);
-  shell_num[i] = ns < shell_cap ? ns : shell_cap;
-  atomicMax(required, ns);
+  if (lane == 0) {
+    if (nc > ccap) atomicOr(realloc, 1);
+    core_end[i] = out0 + (nc < ccap ? nc : ccap);
+    shell_num[i] = ns < shell_cap ? ns : shell_cap;
+    atomicMax(required, ns);
+  }
+}
+
+__device__ __forceinline__ double pow6(double v) {
+  const double v2 = v * v;
+  return v2 * v2 * v2;
 }
 
 // Pair vector r_j - r_i in T with the minimum image, and its r^2 as the
@@ -835,7 +887,7 @@ k_ref_pair_rbl(RefLen<T> b, T rs, T rc, int n, int pice, double alpha, double sq
     if (p.d2 < rs2 && p.d2 > eps_t) {
       const double dx = p.dx, dy = p.dy, dz = p.dz, d2 = dx * dx + dy * dy + dz * dz;
       const double sij = (si + (double)sigma[type[j]]) / 2, eij = sqrt(ei * (double)eps[type[j]]);
-      double f = lj_f64(eij, pow(sij, 6.0), d2);
+      double f = lj_f64(eij, pow6(sij), d2);
       const double qq = qi * (double)q[j];
       if (qq != 0.0) f += coul_f64(alpha, sqa, qqr2e, qq, d2);
       s[0] += f * dx;
@@ -849,7 +901,7 @@ k_ref_pair_rbl(RefLen<T> b, T rs, T rc, int n, int pice, double alpha, double sq
     if (p.d2 < rc2 && p.d2 > rs2) {
       const double dx = p.dx, dy = p.dy, dz = p.dz, d2 = dx * dx + dy * dy + dz * dz;
       const double sij = (si + (double)sigma[type[j]]) / 2, eij = sqrt(ei * (double)eps[type[j]]);
-      double f = lj_f64(eij, pow(sij, 6.0), d2);
+      double f = lj_f64(eij, pow6(sij), d2);
       const double qq = qi * (double)q[j];
       if (qq != 0.0) f += coul_f64(alpha, sqa, qqr2e, qq, d2);
       f *= (double)pice;
@@ -895,7 +947,7 @@ k_ref_pair_verlet(RefLen<T> b, T cut_off, int n, double alpha, double sqa, doubl
     const double dx = p.dx, dy = p.dy, dz = p.dz, d2 = dx * dx + dy * dy + dz * dz;
     const double sij = ((double)sigma[ti] + (double)sigma[type[j]]) / 2,
                  eij = sqrt((double)eps[ti] * (double)eps[type[j]]);
-    const double s6 = pow(sij, 6.0), d6 = d2 * d2 * d2, sd6 = s6 / d6;
+    const double s6 = pow6(sij), d6 = d2 * d2 * d2, sd6 = s6 / d6;
     double f = -24 * eij * ((2 * sd6 - 1) * sd6) / d2;
     a[3] += 0.5 * (4 * eij * (s6 / d6 - 1) * sd6);
     const double qq = qi * (double)q[j];
@@ -949,14 +1001,47 @@ __global__ void k_sum_i32(int n, const int* __restrict__ src, long long* __restr
   if ((threadIdx.x & 31) == 0) atomicAdd((unsigned long long*)out, (unsigned long long)s);
 }
 
+// Mean removal, two launches: per-block sums of the three force columns over
+// a fixed grid, then every block adds those sums in the same order and
+// subtracts the mean; block 0 writes it out.
+constexpr int FIX_BLOCK = 256;
+
 template <typename T>
-__global__ void k_sub_mean(int n, T* __restrict__ fx, T* __restrict__ fy, T* __restrict__ fz,
-                           const double* __restrict__ mean) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(FIX_BLOCK)
+k_col_sums3(int n, const T* __restrict__ fx, const T* __restrict__ fy, const T* __restrict__ fz,
+            double* __restrict__ part) {
+  __shared__ double sh[FIX_BLOCK / 32];
+  double s[3] = {0, 0, 0};
+  for (int i = blockIdx.x * FIX_BLOCK + threadIdx.x; i < n; i += gridDim.x * FIX_BLOCK) {
+    s[0] += (double)fx[i];
+    s[1] += (double)fy[i];
+    s[2] += (double)fz[i];
+  }
+  for (int d = 0; d < 3; ++d) {
+    const double v = block_sum_det<FIX_BLOCK>(s[d], sh);
+    if (threadIdx.x == 0) part[d * gridDim.x + blockIdx.x] = v;
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(FIX_BLOCK)
+k_sub_mean(int n, int nparts, const double* __restrict__ part, T* __restrict__ fx,
+           T* __restrict__ fy, T* __restrict__ fz, T* __restrict__ mean_out) {
+  __shared__ double s_mean[3];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp < 3) {
+    double s = 0.0;
+    for (int b = lane; b < nparts; b += 32) s += part[warp * nparts + b];
+    s = warp_sum(s);
+    if (lane == 0) s_mean[warp] = s * (1.0 / n);
+  }
+  __syncthreads();
+  if (mean_out && blockIdx.x == 0 && threadIdx.x < 3) mean_out[threadIdx.x] = (T)s_mean[threadIdx.x];
+  const int i = blockIdx.x * FIX_BLOCK + threadIdx.x;
   if (i >= n) return;
-  fx[i] = (T)((double)fx[i] - mean[0]);
-  fy[i] = (T)((double)fy[i] - mean[1]);
-  fz[i] = (T)((double)fz[i] - mean[2]);
+  fx[i] = (T)((double)fx[i] - s_mean[0]);
+  fy[i] = (T)((double)fy[i] - s_mean[1]);
+  fz[i] = (T)((double)fz[i] - s_mean[2]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1143,7 +1228,10 @@ int launch_ref_rbl_filter_t(T core2, T force2, int n, const int* gid, const T* x
                             const DBox& b, int* realloc, const DivTest& div, int epoch,
                             cudaStream_t st) {
   if (n <= 0) return RBX_OK;
-  k_ref_rbl_filter<T><<<(n + 127) / 128, 128, 0, st>>>(
+  // freq = 1, 2 or 4 (DivTest of a power of two: inverse 1, shift log2)
+  const bool low2 = div.trivial || (div.inv == 1ULL && div.shift <= 2);
+  auto kern = low2 ? k_ref_rbl_filter<T, true> : k_ref_rbl_filter<T, false>;
+  kern<<<(n + PAIR_WARPS - 1) / PAIR_WARPS, PAIR_BLOCK, 0, st>>>(
       core2, force2, n, gid, x, y, z, cstart, cend, cand, core_cap, core_start, core_end, core,
       shell_cap, shell, shell_num, required, ref_len<T>(b), realloc, div, epoch);
   count_launch();
@@ -1259,20 +1347,29 @@ int launch_sum_i32(int n, const int* src, long long* out, cudaStream_t st) {
   return check_launch("sum_i32");
 }
 
+// part: 3 * fix_rbl_parts(n) doubles of scratch.
+int fix_rbl_parts(int n) {
+  const int b = (n + FIX_BLOCK - 1) / FIX_BLOCK;
+  return b < sm_count() ? b : sm_count();
+}
 template <typename T>
-int launch_sub_mean_t(int n, T* fx, T* fy, T* fz, const double* mean, cudaStream_t st) {
+int launch_fix_rbl_t(int n, T* fx, T* fy, T* fz, T* mean_out, double* part, cudaStream_t st) {
   if (n <= 0) return RBX_OK;
-  k_sub_mean<T><<<(n + 255) / 256, 256, 0, st>>>(n, fx, fy, fz, mean);
+  const int nparts = fix_rbl_parts(n);
+  k_col_sums3<T><<<nparts, FIX_BLOCK, 0, st>>>(n, fx, fy, fz, part);
   count_launch();
-  return check_launch("sub_mean");
+  k_sub_mean<T><<<(n + FIX_BLOCK - 1) / FIX_BLOCK, FIX_BLOCK, 0, st>>>(n, nparts, part, fx, fy, fz,
+                                                                       mean_out);
+  count_launch();
+  return check_launch("fix_rbl");
 }
-int launch_sub_mean(int n, double* fx, double* fy, double* fz, const double* mean,
-                    cudaStream_t st) {
-  return launch_sub_mean_t<double>(n, fx, fy, fz, mean, st);
+int launch_fix_rbl(int n, double* fx, double* fy, double* fz, double* mean_out, double* part,
+                   cudaStream_t st) {
+  return launch_fix_rbl_t<double>(n, fx, fy, fz, mean_out, part, st);
 }
-int launch_sub_mean(int n, float* fx, float* fy, float* fz, const double* mean,
-                    cudaStream_t st) {
-  return launch_sub_mean_t<float>(n, fx, fy, fz, mean, st);
+int launch_fix_rbl(int n, float* fx, float* fy, float* fz, float* mean_out, double* part,
+                   cudaStream_t st) {
+  return launch_fix_rbl_t<float>(n, fx, fy, fz, mean_out, part, st);
 }
 
 }  // namespace rbx

@@ -358,104 +358,61 @@ k_rbe_rho_partial_mixed_batch(const RhoMixedArgs* __restrict__ a, const int* __r
 }
 
 // ---------------------------------------------------------------------------
-// Finalize (one block of 1024 threads): rho_p = sum over the k-major partials
-// (one warp per k, fixed tree); optional energy/virial (ComputeRBEVirial0,
-// kspace_calculator_op.hip.cu:573-674) summed over k in fixed order; force
-// table tab[p] = {kx, ky, kz, coef*Re, coef*Im} with coef = -4 pi qqr2e S /
-// (P V k^2); optional mean of a force-partial array (RBL mean removal).
+// Finalize: rho_p = sum over the k-major partials; energy/virial terms
+// (ComputeRBEVirial0, kspace_calculator_op.hip.cu:573-674) summed over k in
+// fixed order; force table tab[p] = {kx, ky, kz, coef*Re, coef*Im} with coef =
+// -4 pi qqr2e S / (P V k^2); optional mean of a force-partial array (RBL mean
+// removal).
 // ---------------------------------------------------------------------------
 constexpr int FIN_BLOCK = 256;
-constexpr int FIN_WIDE = 1024;
 
-__global__ void __launch_bounds__(FIN_WIDE)
-k_rbe_finalize(int p, int nparts, const double* __restrict__ part_re,
-               const double* __restrict__ part_im, const double* __restrict__ mx,
-               const double* __restrict__ my, const double* __restrict__ mz, double Lx,
-               double Ly, double Lz, double alpha, double S, double qqr2e, double qsq,
-               double qsum, double* __restrict__ rho_re, double* __restrict__ rho_im,
-               double* __restrict__ energy, double* __restrict__ virial,
-               KTab* __restrict__ tab, int mean_parts, const double* __restrict__ fpart,
-               double n_atoms, double* __restrict__ mean_out) {
-  __shared__ double s_e[7][FIN_WIDE / 32];
-  __shared__ double sh[FIN_WIDE / 32];
+// Energy and virial of structure factors that are already sums: a thread a k,
+// then a fixed tree.  (A warp a k with one lane at work, and one thread adding
+// the warps' sums, took 9.1 us at 100 vectors.)
+__global__ void __launch_bounds__(FIN_BLOCK)
+k_rbe_energy_virial(int p, const double* __restrict__ re, const double* __restrict__ im,
+                    const double* __restrict__ mx, const double* __restrict__ my,
+                    const double* __restrict__ mz, double Lx, double Ly, double Lz, double alpha,
+                    double S, double qqr2e, double qsq, double qsum, double* __restrict__ energy,
+                    double* __restrict__ virial) {
+  __shared__ double s_w[7][FIN_BLOCK / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double V = Lx * Ly * Lz;
   const double coef = (2 * RBX_PI * S) / (p * V);
-  const double fcoef = -4 * RBX_PI * qqr2e * S / p;
-  // per-warp running sums of the per-k energy/virial terms, k in increasing order
-  double we[7] = {0, 0, 0, 0, 0, 0, 0};
-  for (int k = warp; k < p; k += FIN_WIDE / 32) {
-    double r = 0.0, im = 0.0;
-    const double* pr = part_re + (size_t)k * nparts;
-    const double* pi = part_im + (size_t)k * nparts;
-    for (int b = lane; b < nparts; b += 32) {
-      r += pr[b];
-      im += pi[b];
-    }
+  double t[7] = {0, 0, 0, 0, 0, 0, 0};
+  for (int k = threadIdx.x; k < p; k += FIN_BLOCK) {
+    const double r = re[k], i = im[k];
+    const double kx = 2 * RBX_PI * mx[k] / Lx;
+    const double ky = 2 * RBX_PI * my[k] / Ly;
+    const double kz = 2 * RBX_PI * mz[k] / Lz;
+    const double k2 = kx * kx + ky * ky + kz * kz;
+    const double base = coef * (r * r + i * i) / k2;
+    const double inner = (1.0 / (4 * alpha)) + (1.0 / k2);
+    t[0] += base;
+    t[1] += base * (1.0 - 2 * kx * kx * inner);
+    t[2] += base * (1.0 - 2 * ky * ky * inner);
+    t[3] += base * (1.0 - 2 * kz * kz * inner);
+    t[4] += base * (-2 * kx * ky * inner);
+    t[5] += base * (-2 * kx * kz * inner);
+    t[6] += base * (-2 * ky * kz * inner);
+  }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      r += __shfl_xor_sync(0xffffffffu, r, o);
-      im += __shfl_xor_sync(0xffffffffu, im, o);
-    }
-    if (lane == 0) {
-      if (rho_re) {
-        rho_re[k] = r;
-        rho_im[k] = im;
-      }
-      const double kx = 2 * RBX_PI * mx[k] / Lx;
-      const double ky = 2 * RBX_PI * my[k] / Ly;
-      const double kz = 2 * RBX_PI * mz[k] / Lz;
-      const double k2 = kx * kx + ky * ky + kz * kz;
-      const double rho2 = r * r + im * im;
-      const double base = coef * rho2 / k2;
-      const double inner = (1.0 / (4 * alpha)) + (1.0 / k2);
-      we[0] += base;
-      we[1] += base * (1.0 - 2 * kx * kx * inner);
-      we[2] += base * (1.0 - 2 * ky * ky * inner);
-      we[3] += base * (1.0 - 2 * kz * kz * inner);
-      we[4] += base * (-2 * kx * ky * inner);
-      we[5] += base * (-2 * kx * kz * inner);
-      we[6] += base * (-2 * ky * kz * inner);
-      if (tab) {
-        const double c = fcoef / (V * k2);
-        KTab t;
-        t.kx = kx;
-        t.ky = ky;
-        t.kz = kz;
-        t.a = c * r;
-        t.b = c * im;
-        t.m[0] = (int)mx[k];
-        t.m[1] = (int)my[k];
-        t.m[2] = (int)mz[k];
-        t.m[3] = 0;
-        t.md[0] = mx[k];
-        t.md[1] = my[k];
-        t.md[2] = mz[k];
-        tab[k] = t;
-      }
-    }
+  for (int c = 0; c < 7; ++c) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t[c] += __shfl_down_sync(0xffffffffu, t[c], o);
+    if (lane == 0) s_w[c][warp] = t[c];
   }
-  if (energy) {
-    if (lane == 0)
-      for (int c = 0; c < 7; ++c) s_e[c][warp] = we[c];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t[7] = {0, 0, 0, 0, 0, 0, 0};
-      for (int w = 0; w < FIN_WIDE / 32; ++w)
-        for (int c = 0; c < 7; ++c) t[c] += s_e[c][w];
-      const double MY_PIS = 1.77245385090551602729, MY_PI2 = 1.57079632679489661923;
-      const double etot = t[0] - (sqrt(alpha) * qsq / MY_PIS + MY_PI2 * qsum * qsum / (alpha * V));
-      *energy = etot * qqr2e;
-      for (int c = 0; c < 6; ++c) virial[c] = t[1 + c] * qqr2e;
-    }
-  }
-  if (mean_out) {
-    for (int d = 0; d < 3; ++d) {
-      double s = 0.0;
-      for (int b = threadIdx.x; b < mean_parts; b += FIN_WIDE) s += fpart[(size_t)b * 3 + d];
-      s = block_sum_det<FIN_WIDE>(s, sh);
-      if (threadIdx.x == 0) mean_out[d] = s / n_atoms;
-    }
+  __syncthreads();
+  if (threadIdx.x >= 7) return;
+  double s = 0.0;
+#pragma unroll
+  for (int w = 0; w < FIN_BLOCK / 32; ++w) s += s_w[threadIdx.x][w];
+  if (threadIdx.x == 0) {
+    const double MY_PIS = 1.77245385090551602729, MY_PI2 = 1.57079632679489661923;
+    s -= sqrt(alpha) * qsq / MY_PIS + MY_PI2 * qsum * qsum / (alpha * V);
+    *energy = s * qqr2e;
+  } else {
+    virial[threadIdx.x - 1] = s * qqr2e;
   }
 }
 
@@ -1181,13 +1138,16 @@ int launch_rbe_finalize(const DBox& b, int p, int nparts, const double* part_re,
                         double* virial, KTab* tab, int mean_parts, const double* fpart,
                         int n_atoms, double* mean_out, double* kterm, cudaStream_t st,
                         EnergyJob* job) {
-  if (energy && !kterm) {  // no per-k scratch: one block does it all
-    k_rbe_finalize<<<1, FIN_WIDE, 0, st>>>(p, nparts, part_re, part_im, mx, my, mz, b.len[0],
-                                            b.len[1], b.len[2], alpha, S, qqr2e, qsq, qsum,
-                                            rho_re, rho_im, energy, virial, tab, mean_parts, fpart,
-                                            (double)n_atoms, mean_out);
+  if (energy && !kterm) {  // no per-k scratch: rho is given (one partial a k)
+    if (nparts != 1 || tab || mean_out || rho_re) {
+      set_error("rbe_finalize: energies without per-k scratch need finished structure factors");
+      return RBX_ERR_INVALID;
+    }
+    k_rbe_energy_virial<<<1, FIN_BLOCK, 0, st>>>(p, part_re, part_im, mx, my, mz, b.len[0],
+                                                 b.len[1], b.len[2], alpha, S, qqr2e, qsq, qsum,
+                                                 energy, virial);
     count_launch();
-    return check_launch("rbe_finalize");
+    return check_launch("rbe_energy_virial");
   }
   const int grid = p + (mean_out ? 3 : 0);
   EnergyJob sum;

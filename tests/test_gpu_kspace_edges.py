@@ -104,3 +104,27 @@ def test_ewald_blocks(cuda, rbx, oracle, n, kmax, share):
     cuda.cuda.synchronize()
     _close(np.stack([a.cpu().numpy() for a in F], 1), f, 1e-12)
     assert abs(en.item() - e) <= 1e-11 * abs(e)
+
+
+@pytest.mark.parametrize("p", [1, 31, 256, 257, 1000])
+def test_energy_virial_sums(cuda, rbx, p):
+    """Energy and virial of given structure factors, FP64: sums of p terms."""
+    lo, hi, _, _, m = _system(2, p, 1.0, p)
+    L, V, alpha, S = hi - lo, float(np.prod(hi - lo)), 0.16, 40.0
+    rng = np.random.default_rng(p)
+    re, im = rng.normal(size=p), rng.normal(size=p)
+    k = 2 * np.pi * m / L[:, None]
+    k2 = (k * k).sum(0)
+    base = 2 * np.pi * S / (p * V) * (re * re + im * im) / k2
+    inner = 2 * (1 / (4 * alpha) + 1 / k2)
+    vir = [(base * ((a == b) - inner * k[a] * k[b])).sum()
+           for a, b in ((0, 0), (1, 1), (2, 2), (0, 1), (0, 2), (1, 2))]
+    e_self = np.sqrt(alpha / np.pi) * 3.0 + 0.5 * np.pi * 0.25 / (alpha * V)
+    dev = lambda a: cuda.as_tensor(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    dv, de = dev(np.zeros(6)), dev(np.zeros(1))
+    rbx.rbe_energy_virial(rbx.Box.make(lo, hi), alpha, S, 2.0, 3.0, 0.5, dev(re), dev(im),
+                          *(dev(v) for v in m), dv, de)
+    cuda.cuda.synchronize()
+    scale = np.abs(base).sum()
+    assert abs(de.item() - 2.0 * (base.sum() - e_self)) < 1e-13 * (scale + e_self)
+    assert np.abs(dv.cpu().numpy() - 2.0 * np.array(vir)).max() < 1e-12 * np.abs(vir).max()
