@@ -24,6 +24,7 @@
 #include "rbx_common.cuh"
 #include "rbx_kernels.h"
 #include "rbx_pair_device.cuh"
+#include "rbx_phase.cuh"
 
 namespace rbx {
 
@@ -91,54 +92,71 @@ __device__ __forceinline__ PairTerms pair_terms_f32(float e, float sg, float qq,
 
 // Block partials: [block][2 * ntypes + 1] = d_eps[0..nt), d_sigma[0..nt), d_alpha.
 // F32: pair terms in FP32 (mixed form), sums in FP64 either way.
+//
+// A warp per atom.  Candidates are screened in batches (fixed-point |d|^2, the
+// FP64 predicate inside its guard bands) and hashed from both sides; the 44 %
+// that carry a gradient wait in a per-warp queue, so that the pair terms run on
+// full warps.  The parameter sums of the partner's type live in shared memory,
+// one column a lane (an array indexed by a run-time type is local memory: the
+// kernel was bound by it and by idle lanes).  Four blocks an SM, some words
+// spilled, beat two without: 20,000 atoms, 417 us before, 247 at two blocks, 185
+// at four (FP64: 275).
+constexpr int ADJ_U = 2;           // 32-candidate groups per batch
+constexpr int AQ_M = (int)0x80000000;  // j is in m's list
+constexpr int AQ_J = 0x40000000;       // m is in j's list
+constexpr int AQ_CORE = 0x20000000;    // core pair: scale 1, not freq
+constexpr int AQ_INDEX = 0x1fffffff;   // atom index (n < 2^29)
+
 template <bool F32>
-__global__ void __launch_bounds__(ADJ_BLOCK)
-k_adj_pair(PairParams pp, int n, const double* __restrict__ x, const double* __restrict__ y,
-           const double* __restrict__ z, const double* __restrict__ q,
-           const int* __restrict__ type, const double* __restrict__ sigma_t,
-           const double* __restrict__ eps_t, const unsigned long long* __restrict__ key_a,
+__global__ void __launch_bounds__(ADJ_BLOCK, 4)
+k_adj_pair(PairParams pp, int n, const uint4* __restrict__ atoms, const double* __restrict__ x,
+           const double* __restrict__ y, const double* __restrict__ z,
+           const double* __restrict__ q, const int* __restrict__ type,
+           const double* __restrict__ sigma_t, const double* __restrict__ eps_t,
+           const unsigned long long* __restrict__ key_a,
            const unsigned long long* __restrict__ key_b, int epoch, Rows rows,
            const double* __restrict__ gx, const double* __restrict__ gy,
            const double* __restrict__ gz, double mgx, double mgy, double mgz,
            double* __restrict__ d_rx, double* __restrict__ d_ry, double* __restrict__ d_rz,
            double* __restrict__ d_q, double* __restrict__ part) {
+  extern __shared__ double s_lane[];  // [2 * nt][ADJ_BLOCK]: d_eps, d_sigma sums of a lane
   __shared__ double s_part[ADJ_WARPS][2 * ADJ_MAX_TYPES + 1];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ int s_q[ADJ_WARPS][32 + 32 * ADJ_U];
+  const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int nt = pp.ntypes, npar = 2 * nt + 1;
-  for (int t = threadIdx.x; t < ADJ_WARPS * (2 * ADJ_MAX_TYPES + 1); t += ADJ_BLOCK)
-    (&s_part[0][0])[t] = 0.0;
-  __syncthreads();
-  double acc[2 * ADJ_MAX_TYPES + 1];
-  for (int t = 0; t < npar; ++t) acc[t] = 0.0;
+  const unsigned lt = (1u << lane) - 1u;
+  int* const wq = s_q[warp];
+  double* const mine = s_lane + threadIdx.x;
+  for (int t = 0; t < 2 * nt; ++t) mine[t * ADJ_BLOCK] = 0.0;
+  double d_alpha = 0.0;
   const double freq = (double)pp.freq;
   for (int m = blockIdx.x * ADJ_WARPS + warp; m < n; m += gridDim.x * ADJ_WARPS) {
+    const uint4 am = atoms[m];
     const double xm = x[m], ym = y[m], zm = z[m], qm = q[m];
     const int tm = type[m];
+    const double eps_m = eps_t[tm], sig_m = sigma_t[tm];
     const double gpx = gx[m] - mgx, gpy = gy[m] - mgy, gpz = gz[m] - mgz;
     const unsigned long long ea_m = key_a[m] ^ (unsigned long long)(long long)epoch;
     const unsigned long long kb_m = key_b[m];
-    double rx = 0.0, ry = 0.0, rz = 0.0, dq = 0.0;
+    double rx = 0.0, ry = 0.0, rz = 0.0, dq = 0.0, de_m = 0.0, ds_m = 0.0;
     int nf, nb;
     row_extent(rows, m, nf, nb);
+    const int cnt = nf + nb;
     const int* row = rows.idx + (size_t)m * rows.cap;
-    for (int k = lane; k < nf + nb; k += 32) {
-      const int j = row_at(row, rows.cap, nf, nb, k);
-      if (j == m) continue;
-      const Classified c = classify_exact(exact_d2(pp, x, y, z, m, j), pp);
-      if (!c.core_active && !c.shell_window) continue;
-      const bool in_m = c.core_active || rbl_selected(ea_m, key_b[j], pp.div);
-      const unsigned long long ea_j = key_a[j] ^ (unsigned long long)(long long)epoch;
-      const bool in_j = c.core_active || rbl_selected(ea_j, kb_m, pp.div);
-      if (!in_m && !in_j) continue;
-      const double s = c.core_active ? 1.0 : freq;
+    int qn = 0;
+    auto pair = [&](int slot) {
+      const int c = wq[slot];
+      const int j = c & AQ_INDEX;
+      const bool in_m = c < 0, in_j = c & AQ_J;
+      const double s = (c & AQ_CORE) ? 1.0 : freq;
       // r_j - r_m, MinImageDistance (box.h:51-73), as in the force kernel
       const double dx = min_image1(x[j] - xm, pp.box.len[0], pp.box.half[0]);
       const double dy = min_image1(y[j] - ym, pp.box.len[1], pp.box.half[1]);
       const double dz = min_image1(z[j] - zm, pp.box.len[2], pp.box.half[2]);
       const double r2 = dx * dx + dy * dy + dz * dz;
       const int tj = type[j];
-      const double e = sqrt(eps_t[tm] * eps_t[tj]);
-      const double sg = 0.5 * (sigma_t[tm] + sigma_t[tj]);
+      const double e = sqrt(eps_m * eps_t[tj]);
+      const double sg = 0.5 * (sig_m + sigma_t[tj]);
       const double qj = q[j];
       const PairTerms pt =
           F32 ? pair_terms_f32((float)e, (float)sg, (float)(qm * qj), (float)r2, (float)pp.alpha,
@@ -152,11 +170,12 @@ k_adj_pair(PairParams pp, int n, const double* __restrict__ x, const double* __r
         ry -= cf * gpy + cd * dy;
         rz -= cf * gpz + cd * dz;
         dq += w * pt.h * qj;
-        acc[tm] += w * pt.df_de * e / (2.0 * eps_t[tm]);
-        acc[tj] += w * pt.df_de * e / (2.0 * eps_t[tj]);
-        acc[nt + tm] += 0.5 * w * pt.df_ds;
-        acc[nt + tj] += 0.5 * w * pt.df_ds;
-        acc[2 * nt] += w * qm * qj * pt.dh_da;
+        const double we = w * pt.df_de * e, ws = 0.5 * w * pt.df_ds;
+        de_m += we;
+        ds_m += ws;
+        mine[tj * ADJ_BLOCK] += we;
+        mine[(nt + tj) * ADJ_BLOCK] += ws;
+        d_alpha += w * qm * qj * pt.dh_da;
       }
       if (in_j) {  // pair (j, m) of j's force: +c on r_m, and its q_m factor
         const double gjx = gx[j] - mgx, gjy = gy[j] - mgy, gjz = gz[j] - mgz;
@@ -167,7 +186,47 @@ k_adj_pair(PairParams pp, int n, const double* __restrict__ x, const double* __r
         rz += cf * gjz + cd * dz;
         dq -= s * gd * pt.h * qj;  // w_j = s g'_j . (r_m - r_j) = -s gd
       }
+    };
+    for (int k0 = 0; k0 < cnt; k0 += 32 * ADJ_U) {
+      int j[ADJ_U];
+      uint4 aj[ADJ_U];
+#pragma unroll
+      for (int u = 0; u < ADJ_U; ++u) {
+        const int k = k0 + 32 * u + lane;
+        j[u] = k < cnt ? row_at(row, rows.cap, nf, nb, k) : m;
+      }
+#pragma unroll
+      for (int u = 0; u < ADJ_U; ++u) aj[u] = __ldg(atoms + j[u]);
+#pragma unroll
+      for (int u = 0; u < ADJ_U; ++u) {
+        bool unsure;
+        Classified c = classify_screen(pp, pp.cubic ? fixed_d2(am, aj[u])
+                                                    : fixed_d2_weighted(pp, am, aj[u]), &unsure);
+        if (unsure && j[u] != m) c = classify_exact(exact_d2(pp, x, y, z, m, j[u]), pp);
+        int f = c.core_active ? AQ_M | AQ_J | AQ_CORE : 0;
+        if (c.shell_window) {
+          if (rbl_selected(ea_m, __ldg(key_b + j[u]), pp.div)) f |= AQ_M;
+          if (rbl_selected(__ldg(key_a + j[u]) ^ (unsigned long long)(long long)epoch, kb_m,
+                           pp.div))
+            f |= AQ_J;
+        }
+        const bool push = f != 0 && j[u] != m;
+        const unsigned mk = __ballot_sync(0xffffffffu, push);
+        if (push) wq[qn + __popc(mk & lt)] = j[u] | f;
+        qn += __popc(mk);
+      }
+      __syncwarp();
+      while (qn >= 32) {  // full batches from the tail of the queue
+        qn -= 32;
+        pair(qn + lane);
+      }
+      __syncwarp();
     }
+    if (lane < qn) pair(lane);
+    __syncwarp();
+    // d(eps_ij)/d(eps_m) = e / (2 eps_m); the partner's side below
+    mine[tm * ADJ_BLOCK] += de_m;
+    mine[(nt + tm) * ADJ_BLOCK] += ds_m;
     rx = warp_sum(rx);
     ry = warp_sum(ry);
     rz = warp_sum(rz);
@@ -180,7 +239,8 @@ k_adj_pair(PairParams pp, int n, const double* __restrict__ x, const double* __r
     }
   }
   for (int t = 0; t < npar; ++t) {
-    const double v = warp_sum(acc[t]);
+    double v = warp_sum(t < 2 * nt ? mine[t * ADJ_BLOCK] : d_alpha);
+    if (t < nt) v /= 2.0 * eps_t[t];
     if (lane == 0) s_part[warp][t] = v;
   }
   __syncthreads();
@@ -194,7 +254,8 @@ k_adj_pair(PairParams pp, int n, const double* __restrict__ x, const double* __r
 // k-space, pass 1: per-block partial sums of a_k and b_k, part[k][block].
 constexpr int ADJK_BLOCK = 128;
 __global__ void __launch_bounds__(ADJK_BLOCK)
-k_adj_k_ab(int n, int p, int chunk, const KTab* __restrict__ tab, const double* __restrict__ q,
+k_adj_k_ab(int n, int p, int chunk, double sx, double sy, double sz,
+           const KTab* __restrict__ tab, const double* __restrict__ q,
            const double* __restrict__ x, const double* __restrict__ y,
            const double* __restrict__ z, const double* __restrict__ gx,
            const double* __restrict__ gy, const double* __restrict__ gz,
@@ -202,11 +263,15 @@ k_adj_k_ab(int n, int p, int chunk, const KTab* __restrict__ tab, const double* 
   const int k = blockIdx.y * ADJK_BLOCK + threadIdx.x;
   if (k >= p) return;
   const double kx = tab[k].kx, ky = tab[k].ky, kz = tab[k].kz;
+  // phase in quarter turns: 4 m / L per length (sx, sy, sz = 4 / L)
+  const double mx = tab[k].md[0] * sx, my = tab[k].md[1] * sy, mz = tab[k].md[2] * sz;
   const int a0 = blockIdx.x * chunk, a1 = min(n, a0 + chunk);
   double sa = 0.0, sb = 0.0;
   for (int i = a0; i < a1; ++i) {
     double s, c;
-    sincos(kx * x[i] + ky * y[i] + kz * z[i], &s, &c);
+    if (q[i] + 0.0 * (x[i] + y[i] + z[i] + gx[i] + gy[i] + gz[i]) == 0.0)
+      continue;  // a neutral atom's weight q_i (g_i . k) is zero
+    sincos_quarter(mx * x[i] + my * y[i] + mz * z[i], &s, &c);
     const double w = q[i] * (gx[i] * kx + gy[i] * ky + gz[i] * kz);
     sa += w * c;
     sb += w * s;
@@ -218,43 +283,58 @@ k_adj_k_ab(int n, int p, int chunk, const KTab* __restrict__ tab, const double* 
 // k-space, pass 2: per-atom dL/dq and dL/dr, and per-block sums of g . K
 // (for dL/dalpha).  ab[k] = {a_k, b_k} reduced in fixed order beforehand.
 __global__ void __launch_bounds__(ADJK_BLOCK)
-k_adj_k_scatter(int n, int p, double cscale, const KTab* __restrict__ tab,
-                const double* __restrict__ ab, const double* __restrict__ q,
-                const double* __restrict__ x, const double* __restrict__ y,
-                const double* __restrict__ z, const double* __restrict__ gx,
-                const double* __restrict__ gy, const double* __restrict__ gz,
-                double* __restrict__ d_rx, double* __restrict__ d_ry, double* __restrict__ d_rz,
-                double* __restrict__ d_q, double* __restrict__ part_gk) {
+k_adj_k_scatter(int n, int p, double cscale, double sx, double sy, double sz,
+                const KTab* __restrict__ tab, const double* __restrict__ ab,
+                const double* __restrict__ q, const double* __restrict__ x,
+                const double* __restrict__ y, const double* __restrict__ z,
+                const double* __restrict__ gx, const double* __restrict__ gy,
+                const double* __restrict__ gz, double* __restrict__ d_rx,
+                double* __restrict__ d_ry, double* __restrict__ d_rz, double* __restrict__ d_q,
+                double* __restrict__ part_gk) {
+  struct K64 {  // per-k constants, formed once a block
+    double mx, my, mz, kx, ky, kz, ta, tb, ca, cb;
+  };
+  constexpr int kTile = 128;
+  __shared__ K64 s_k[kTile];
   __shared__ double s_sum[ADJK_BLOCK / 32];
   const int i = blockIdx.x * ADJK_BLOCK + threadIdx.x;
-  double gk_sum = 0.0;
-  if (i < n) {
-    const double xi = x[i], yi = y[i], zi = z[i], qi = q[i];
-    const double gix = gx[i], giy = gy[i], giz = gz[i];
-    double rx = 0.0, ry = 0.0, rz = 0.0, dq = 0.0;
-    for (int k = 0; k < p; ++k) {
-      const KTab t = tab[k];
-      const double k2 = t.kx * t.kx + t.ky * t.ky + t.kz * t.kz;
-      const double ck = cscale / k2;  // -4 pi qqr2e S / (P V k^2)
+  const bool live = i < n;
+  const double ux = live ? x[i] * sx : 0.0, uy = live ? y[i] * sy : 0.0,
+               uz = live ? z[i] * sz : 0.0, qi = live ? q[i] : 0.0;
+  const double gix = live ? gx[i] : 0.0, giy = live ? gy[i] : 0.0, giz = live ? gz[i] : 0.0;
+  double rx = 0.0, ry = 0.0, rz = 0.0, dq = 0.0, gk_sum = 0.0;
+  for (int k0 = 0; k0 < p; k0 += kTile) {
+    const int kn = min(kTile, p - k0);
+    __syncthreads();
+    for (int k = threadIdx.x; k < kn; k += ADJK_BLOCK) {
+      const KTab& t = tab[k0 + k];
+      const double ck = cscale / (t.kx * t.kx + t.ky * t.ky + t.kz * t.kz);
+      // t.a = c_k Re rho_k, t.b = c_k Im rho_k, c_k = -4 pi qqr2e S / (P V k^2)
+      s_k[k] = K64{t.md[0], t.md[1], t.md[2], t.kx, t.ky, t.kz, t.a, t.b,
+                   ck * ab[2 * (k0 + k)], ck * ab[2 * (k0 + k) + 1]};
+    }
+    __syncthreads();
+    for (int k = 0; k < kn; ++k) {
+      const K64 t = s_k[k];
       double s, c;
-      sincos(t.kx * xi + t.ky * yi + t.kz * zi, &s, &c);
+      sincos_quarter(t.mx * ux + t.my * uy + t.mz * uz, &s, &c);
       const double gk = gix * t.kx + giy * t.ky + giz * t.kz;
-      // t.a = c_k Re rho_k, t.b = c_k Im rho_k
-      const double ak = ab[2 * k], bk = ab[2 * k + 1];
-      dq += gk * (c * t.b - s * t.a) + ck * (ak * s - bk * c);
-      const double coef = -gk * (s * t.b + c * t.a) + ck * (ak * c + bk * s);
+      const double g1 = gk * (c * t.tb - s * t.ta);
+      dq += g1 + (t.ca * s - t.cb * c);
+      const double coef = -gk * (s * t.tb + c * t.ta) + (t.ca * c + t.cb * s);
       rx += coef * t.kx;
       ry += coef * t.ky;
       rz += coef * t.kz;
-      gk_sum += gk * (c * t.b - s * t.a);
+      gk_sum += g1;
     }
+  }
+  if (live) {
     d_rx[i] += qi * rx;
     d_ry[i] += qi * ry;
     d_rz[i] += qi * rz;
     d_q[i] += dq;
-    gk_sum *= qi;
   }
-  gk_sum = block_sum_det<ADJK_BLOCK>(gk_sum, s_sum);
+  gk_sum = block_sum_det<ADJK_BLOCK>(live ? gk_sum * qi : 0.0, s_sum);
   if (threadIdx.x == 0) part_gk[blockIdx.x] = gk_sum;
 }
 
@@ -295,40 +375,66 @@ k_adj_k_scatter_mixed(int n, int p, double cscale, const KTab* __restrict__ tab,
                       const double* __restrict__ gz, double* __restrict__ d_rx,
                       double* __restrict__ d_ry, double* __restrict__ d_rz,
                       double* __restrict__ d_q, double* __restrict__ part_gk) {
+  // the per-k constants in FP32, formed once a block (c_k took an FP64 divide
+  // per atom and k)
+  struct K32 {
+    unsigned m0, m1, m2;
+    float kx, ky, kz, ck, ta, tb, ak, bk;
+  };
+  constexpr int kTile = 256;
+  __shared__ K32 s_k[kTile];
   __shared__ double s_sum[ADJK_BLOCK / 32];
   const int i = blockIdx.x * ADJK_BLOCK + threadIdx.x;
   double gk_sum = 0.0;
-  if (i < n) {
-    const uint4 a = atoms[i];
-    const float qi = __uint_as_float(a.w);
-    const float gix = (float)gx[i], giy = (float)gy[i], giz = (float)gz[i];
-    const float ang = (float)(2.0 * RBX_PI / 4294967296.0);
-    double rx = 0.0, ry = 0.0, rz = 0.0, dq = 0.0;
-    for (int k = 0; k < p; ++k) {
-      const KTab t = tab[k];
-      const float kx = (float)t.kx, ky = (float)t.ky, kz = (float)t.kz;
-      const float ck = (float)(cscale / (t.kx * t.kx + t.ky * t.ky + t.kz * t.kz));
-      const unsigned ph =
-          (unsigned)t.m[0] * a.x + (unsigned)t.m[1] * a.y + (unsigned)t.m[2] * a.z;
+  const bool live = i < n;
+  const uint4 a = live ? atoms[i] : make_uint4(0, 0, 0, 0);
+  const float qi = __uint_as_float(a.w);
+  const float gix = live ? (float)gx[i] : 0.f, giy = live ? (float)gy[i] : 0.f,
+              giz = live ? (float)gz[i] : 0.f;
+  const float ang = (float)(2.0 * RBX_PI / 4294967296.0);
+  double rx = 0.0, ry = 0.0, rz = 0.0, dq = 0.0;
+  for (int k0 = 0; k0 < p; k0 += kTile) {
+    const int kn = min(kTile, p - k0);
+    __syncthreads();
+    for (int k = threadIdx.x; k < kn; k += ADJK_BLOCK) {
+      const KTab& t = tab[k0 + k];
+      K32 c;
+      c.m0 = (unsigned)t.m[0];
+      c.m1 = (unsigned)t.m[1];
+      c.m2 = (unsigned)t.m[2];
+      c.kx = (float)t.kx;
+      c.ky = (float)t.ky;
+      c.kz = (float)t.kz;
+      c.ck = (float)(cscale / (t.kx * t.kx + t.ky * t.ky + t.kz * t.kz));
+      c.ta = (float)t.a;
+      c.tb = (float)t.b;
+      c.ak = (float)ab[2 * (k0 + k)];
+      c.bk = (float)ab[2 * (k0 + k) + 1];
+      s_k[k] = c;
+    }
+    __syncthreads();
+    for (int k = 0; k < kn; ++k) {
+      const K32 c = s_k[k];
+      const unsigned ph = c.m0 * a.x + c.m1 * a.y + c.m2 * a.z;
       float sn, cs;
       __sincosf((float)(int)ph * ang, &sn, &cs);
-      const float gk = gix * kx + giy * ky + giz * kz;
-      const float ta = (float)t.a, tb = (float)t.b;
-      const float ak = (float)ab[2 * k], bk = (float)ab[2 * k + 1];
-      const float g1 = gk * (cs * tb - sn * ta);
-      dq += (double)(g1 + ck * (ak * sn - bk * cs));
-      const float coef = -gk * (sn * tb + cs * ta) + ck * (ak * cs + bk * sn);
-      rx += (double)(coef * kx);
-      ry += (double)(coef * ky);
-      rz += (double)(coef * kz);
+      const float gk = gix * c.kx + giy * c.ky + giz * c.kz;
+      const float g1 = gk * (cs * c.tb - sn * c.ta);
+      dq += (double)(g1 + c.ck * (c.ak * sn - c.bk * cs));
+      const float coef = -gk * (sn * c.tb + cs * c.ta) + c.ck * (c.ak * cs + c.bk * sn);
+      rx += (double)(coef * c.kx);
+      ry += (double)(coef * c.ky);
+      rz += (double)(coef * c.kz);
       gk_sum += (double)g1;
     }
+  }
+  if (live) {
     d_rx[i] += (double)qi * rx;
     d_ry[i] += (double)qi * ry;
     d_rz[i] += (double)qi * rz;
     d_q[i] += dq;
-    gk_sum *= (double)qi;
   }
+  gk_sum = live ? gk_sum * (double)qi : 0.0;
   gk_sum = block_sum_det<ADJK_BLOCK>(gk_sum, s_sum);
   if (threadIdx.x == 0) part_gk[blockIdx.x] = gk_sum;
 }
@@ -371,12 +477,14 @@ int launch_gather_vec3(int n, const int* orig, const double* src, double* x, dou
 }
 
 int adj_pair_blocks(int n) {
+  // up to four waves of the four resident blocks: the scheduler evens out the
+  // atoms' work
   const int b = (n + ADJ_WARPS - 1) / ADJ_WARPS;
-  return b < 4 * sm_count() ? (b < 1 ? 1 : b) : 4 * sm_count();
+  return b < 16 * sm_count() ? (b < 1 ? 1 : b) : 16 * sm_count();
 }
 
-int launch_adj_pair(const PairParams& pp, int n, const double* x, const double* y,
-                    const double* z, const double* q, const int* type, const double* sigma_t,
+int launch_adj_pair(const PairParams& pp, int n, const uint4* atoms, const double* x,
+                    const double* y, const double* z, const double* q, const int* type, const double* sigma_t,
                     const double* eps_t, const unsigned long long* key_a,
                     const unsigned long long* key_b, int epoch, const Rows& rows,
                     const double* gx, const double* gy,
@@ -387,17 +495,26 @@ int launch_adj_pair(const PairParams& pp, int n, const double* x, const double* 
     set_error("adjoint: at most %d atom types", ADJ_MAX_TYPES);
     return RBX_ERR_INVALID;
   }
+  if (n > AQ_INDEX) {
+    set_error("adjoint: at most %d atoms", AQ_INDEX);
+    return RBX_ERR_INVALID;
+  }
   auto kern = f32 ? k_adj_pair<true> : k_adj_pair<false>;
-  kern<<<nblocks, ADJ_BLOCK, 0, st>>>(pp, n, x, y, z, q, type, sigma_t, eps_t, key_a, key_b,
-                                            epoch, rows, gx, gy, gz, mean_g[0],
-                                            mean_g[1], mean_g[2], d_rx, d_ry, d_rz, d_q, part);
+  const size_t smem = sizeof(double) * 2 * pp.ntypes * ADJ_BLOCK;  // at most 64 KB
+  if (smem > 32 * 1024 &&
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+          cudaSuccess)
+    return check_launch("adj_pair (shared memory)");
+  kern<<<nblocks, ADJ_BLOCK, smem, st>>>(pp, n, atoms, x, y, z, q, type, sigma_t, eps_t, key_a,
+                                         key_b, epoch, rows, gx, gy, gz, mean_g[0], mean_g[1],
+                                         mean_g[2], d_rx, d_ry, d_rz, d_q, part);
   count_launch();
   return check_launch("adj_pair");
 }
 
 int adj_k_blocks(int n) { return (n + ADJK_BLOCK - 1) / ADJK_BLOCK; }
 
-int launch_adj_kspace(int n, int p, double cscale, const KTab* tab, const double* q,
+int launch_adj_kspace(const DBox& b, int n, int p, double cscale, const KTab* tab, const double* q,
                       const double* x, const double* y, const double* z, const double* gx,
                       const double* gy, const double* gz, double* part_a, double* part_b,
                       int nparts, double* ab, double* d_rx, double* d_ry, double* d_rz,
@@ -406,7 +523,8 @@ int launch_adj_kspace(int n, int p, double cscale, const KTab* tab, const double
   const int chunk = (n + nparts - 1) / nparts;
   const int nb = (n + chunk - 1) / chunk;
   k_adj_k_ab<<<dim3(nb, (p + ADJK_BLOCK - 1) / ADJK_BLOCK), ADJK_BLOCK, 0, st>>>(
-      n, p, chunk, tab, q, x, y, z, gx, gy, gz, part_a, part_b);
+      n, p, chunk, 4.0 / b.len[0], 4.0 / b.len[1], 4.0 / b.len[2], tab, q, x, y, z, gx, gy, gz,
+      part_a, part_b);
   count_launch();
   int rc = check_launch("adj_k_ab");
   if (rc) return rc;
@@ -414,8 +532,9 @@ int launch_adj_kspace(int n, int p, double cscale, const KTab* tab, const double
   count_launch();
   rc = check_launch("adj_reduce_k");
   if (rc) return rc;
-  k_adj_k_scatter<<<adj_k_blocks(n), ADJK_BLOCK, 0, st>>>(n, p, cscale, tab, ab, q, x, y, z, gx,
-                                                          gy, gz, d_rx, d_ry, d_rz, d_q, part_gk);
+  k_adj_k_scatter<<<adj_k_blocks(n), ADJK_BLOCK, 0, st>>>(
+      n, p, cscale, 4.0 / b.len[0], 4.0 / b.len[1], 4.0 / b.len[2], tab, ab, q, x, y, z, gx, gy,
+      gz, d_rx, d_ry, d_rz, d_q, part_gk);
   count_launch();
   return check_launch("adj_k_scatter");
 }

@@ -1498,7 +1498,7 @@ int rbx_engine::force_vjp(const double* g, double* d_eps, double* d_sigma, doubl
   // mixed form: FP32 pair and k-space terms (exact fixed-point phases, the k
   // table of the last force evaluation), FP64 sums; plain FP64 otherwise
   const bool mixed = prm.precision == RBX_MIXED;
-  ETRY(launch_adj_pair(pp, n, x, y, z, q, type, sig_t, eps_t, key_a, key_b, epoch, rows(), gx,
+  ETRY(launch_adj_pair(pp, n, atoms, x, y, z, q, type, sig_t, eps_t, key_a, key_b, epoch, rows(), gx,
                        gy, gz, mean_g, rx, ry, rz, dq, ppart, nb_pair, st, mixed));
   if (P > 0) {
     const double V = dbox.len[0] * dbox.len[1] * dbox.len[2];
@@ -1507,7 +1507,7 @@ int rbx_engine::force_vjp(const double* g, double* d_eps, double* d_sigma, doubl
       ETRY(launch_adj_kspace_mixed(n, P, cscale, tab, atoms, gx, gy, gz, part_re, part_im,
                                    nparts, kterm, rx, ry, rz, dq, kpart, st));
     else
-      ETRY(launch_adj_kspace(n, P, cscale, tab, q, x, y, z, gx, gy, gz, part_re, part_im, nparts,
+      ETRY(launch_adj_kspace(dbox, n, P, cscale, tab, q, x, y, z, gx, gy, gz, part_re, part_im, nparts,
                              kterm, rx, ry, rz, dq, kpart, st));
   }
   std::vector<double> hp((size_t)nb_pair * npar), hk(P > 0 ? nb_k : 0);

@@ -274,8 +274,8 @@ int launch_full_list(const DBox& b, const int dims[3], double cutoff, int n, con
 // Force adjoint (rbx_adjoint.cu).  Pair part: per-atom dL/dr, dL/dq and
 // per-block partials [nblocks][2 ntypes + 1] (d_eps, d_sigma, d_alpha).
 int adj_pair_blocks(int n);
-int launch_adj_pair(const PairParams& pp, int n, const double* x, const double* y,
-                    const double* z, const double* q, const int* type, const double* sigma_t,
+int launch_adj_pair(const PairParams& pp, int n, const uint4* atoms, const double* x,
+                    const double* y, const double* z, const double* q, const int* type, const double* sigma_t,
                     const double* eps_t, const unsigned long long* key_a,
                     const unsigned long long* key_b, int epoch, const Rows& rows,
                     const double* gx, const double* gy,
@@ -285,7 +285,7 @@ int launch_adj_pair(const PairParams& pp, int n, const double* x, const double* 
 // k-space part, added to d_r and d_q; part_gk[adj_k_blocks(n)] = block sums of g . K.
 // cscale = -4 pi qqr2e S / (P V); ab: 2p scratch; part_a/b: p * nparts scratch.
 int adj_k_blocks(int n);
-int launch_adj_kspace(int n, int p, double cscale, const KTab* tab, const double* q,
+int launch_adj_kspace(const DBox& b, int n, int p, double cscale, const KTab* tab, const double* q,
                       const double* x, const double* y, const double* z, const double* gx,
                       const double* gy, const double* gz, double* part_a, double* part_b,
                       int nparts, double* ab, double* d_rx, double* d_ry, double* d_rz,

@@ -130,53 +130,6 @@ __device__ __forceinline__ void write_block_partial(double (*s_acc)[3], double* 
 }
 
 // ---------------------------------------------------------------------------
-// Candidate classification shared by both forms.
-//
-// The pair vector in fixed point, d = u_j - u_i (wrapped int32), is the exact
-// minimum image of the FP64 pair vector to within 3 units of s_d = L_d/2^32
-// per coordinate.  |d|^2 is formed in FP32 in units of s^2, s = L_max/2^32
-// (on a box with unequal edges each coordinate is first weighted by
-// L_d/L_max, which keeps its error below 3 units of s), and each predicate
-// "r^2 < C" is decided when |d|^2 lies outside a guard band [lo, hi] around
-// C/s^2 that exceeds every rounding and quantisation error; inside the band
-// the reference's FP64 expression (CaculateDistance: i minus j, min image, no
-// FMA) decides.  The outcome is therefore identical to the FP64 predicate on
-// every pair, in both precision forms.
-// ---------------------------------------------------------------------------
-// Screened classification; *unsure is set when a threshold band is hit.  The
-// band around core2_list and the one around rs2 (which lies just above it)
-// are merged into one undecided interval, as are d2 values at or below the
-// EPS band: each undecided pair is settled by the FP64 predicate, so five
-// comparisons classify a pair.
-__device__ __forceinline__ Classified classify_screen(const PairParams& pp, float d2s,
-                                                      bool* unsure) {
-  const bool A = d2s < pp.sc_core.lo;    // certainly d2 < core2_list
-  const bool B = d2s <= pp.sc_rs.hi;     // not certainly d2 > rs2
-  const bool C = d2s < pp.sc_force.lo;   // certainly d2 < force2_list
-  const bool D = d2s < pp.sc_force.hi;   // not certainly d2 >= force2_list
-  const bool E = d2s <= pp.sc_eps.hi;    // not certainly d2 > EPS
-  *unsure = (!A && B) || (!C && D) || E;
-  Classified c;
-  c.core_active = A;
-  c.shell_window = !B && C;
-  return c;
-}
-
-__device__ __forceinline__ float fixed_d2(const uint4& ai, const uint4& aj) {
-  const float dx = (float)(int)(aj.x - ai.x), dy = (float)(int)(aj.y - ai.y),
-              dz = (float)(int)(aj.z - ai.z);
-  return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-}
-// The same in units of the longest edge's fixed-point step on a box with
-// unequal edges (each difference weighted by L_d / L_max).
-__device__ __forceinline__ float fixed_d2_weighted(const PairParams& pp, const uint4& ai,
-                                                   const uint4& aj) {
-  const float dx = (float)(int)(aj.x - ai.x) * pp.sw[0], dy = (float)(int)(aj.y - ai.y) * pp.sw[1],
-              dz = (float)(int)(aj.z - ai.z) * pp.sw[2];
-  return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-}
-
-// ---------------------------------------------------------------------------
 // Fused RBL filter + pair force over split candidate rows.
 //
 // The list builder writes each candidate row in two segments (see Rows): the
