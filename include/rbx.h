@@ -542,6 +542,9 @@ int rbx_engine_step_host(rbx_engine* e, const double* x_in, const double* v_in,
 int rbx_engine_get_state(rbx_engine* e, double* px, double* py, double* pz,
                          double* vx, double* vy, double* vz, double* fx,
                          double* fy, double* fz);
+/* The same as [n][3] rows per quantity (x y z of an atom together); pos, vel
+ * or force may be NULL. */
+int rbx_engine_get_state_rows(rbx_engine* e, double* pos, double* vel, double* force);
 /* Autotuner (no counterpart in the reference): times the engine's kernels on
  * its current state for each candidate launch shape -- rho(k): k-vectors per
  * thread 1/2/4/8 (32 per warp each) x atom blocks (1, 2, 4, 8 per SM); force

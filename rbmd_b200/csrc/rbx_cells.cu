@@ -1038,6 +1038,26 @@ __global__ void k_scatter_set(int n, const int* __restrict__ idx, ArraySet s) {
     if (a < s.nu64) s.dst_u64[a][p] = s.src_u64[a][i];
 }
 
+// dst[3 idx[i] + d] = column d at i.
+__global__ void k_scatter_rows(int n, const int* __restrict__ idx, const double* __restrict__ a,
+                               const double* __restrict__ b, const double* __restrict__ c,
+                               double* __restrict__ dst) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double* const p = dst + 3 * (size_t)idx[i];
+  p[0] = a[i];
+  p[1] = b[i];
+  p[2] = c[i];
+}
+
+int launch_scatter_rows(int n, const int* idx, const double* a, const double* b, const double* c,
+                        double* dst, cudaStream_t st) {
+  if (n <= 0) return RBX_OK;
+  k_scatter_rows<<<(n + 255) / 256, 256, 0, st>>>(n, idx, a, b, c, dst);
+  count_launch();
+  return check_launch("scatter_rows");
+}
+
 int launch_scatter_set(int n, const int* idx, const ArraySet& set, cudaStream_t st) {
   if (n <= 0) return RBX_OK;
   k_scatter_set<<<(n + 255) / 256, 256, 0, st>>>(n, idx, set);

@@ -147,6 +147,7 @@ struct rbx_engine {
   double* kterm = nullptr;  // per-k energy/virial terms [P][8]
   double *ek = nullptr, *virk = nullptr;
   double* sample_tables = nullptr;
+  int sample_cap = 0;  // entries sample_tables has room for
   int tcnt[3] = {0, 0, 0};
   double ttot[3] = {0, 0, 0};
 
@@ -248,6 +249,7 @@ struct rbx_engine {
   int check_sampler();
   int step(int nsteps);
   int step_host(const double* xin, const double* vin, double* xout, double* vout, double* fout);
+  int get_state_rows(double* pos, double* vel, double* force);
   int get_state(double* px, double* py, double* pz, double* vx, double* vy, double* vz,
                 double* fx, double* fy, double* fz);
   int get_force_parts(double* f_pair, double* f_kspace);

@@ -95,8 +95,8 @@ EXPORTS = [
     "rbx_pair_force_verlet", "rbx_engine_create", "rbx_engine_create_json",
     "rbx_engine_destroy", "rbx_engine_set_state", "rbx_engine_set_k_samples",
     "rbx_engine_compute_forces", "rbx_engine_step", "rbx_engine_step_host",
-    "rbx_engine_get_state", "rbx_engine_get_force_parts", "rbx_engine_get_rbl_pairs",
-    "rbx_engine_pair_energy",
+    "rbx_engine_get_state", "rbx_engine_get_state_rows", "rbx_engine_get_force_parts",
+    "rbx_engine_get_rbl_pairs", "rbx_engine_pair_energy",
     "rbx_engine_get_stats", "rbx_engine_stream", "rbx_engine_phase_ms",
     "rbx_engine_set_profiling", "rbx_rbe_structure_factor_noalloc", "rbx_engine_set_step_graph",
     "rbx_nlist_should_reuse", "rbx_batch_create", "rbx_batch_destroy", "rbx_batch_step",
@@ -183,6 +183,7 @@ def lib():
     L.rbx_engine_step.argtypes = [vp, ip]
     L.rbx_engine_step_host.argtypes = [vp] * 6
     L.rbx_engine_get_state.argtypes = [vp] * 10
+    L.rbx_engine_get_state_rows.argtypes = [vp] * 4
     L.rbx_engine_get_force_parts.argtypes = [vp, vp, vp]
     L.rbx_engine_pair_energy.argtypes = [vp, vp, vp, vp]
     L.rbx_engine_get_rbl_pairs.argtypes = [vp, vp, C.POINTER(C.c_int64), vp,
@@ -574,7 +575,10 @@ class Engine:
     def set_positions(self, pos, vel=None):
         """New positions (host order, [n, 3]); velocities kept unless given."""
         pos = np.ascontiguousarray(pos, dtype=np.float64).reshape(self.n, 3)
-        vel = self.get_state()["vel"] if vel is None else np.asarray(vel, dtype=np.float64)
+        if vel is None:
+            vel = np.empty((self.n, 3))
+            check(lib().rbx_engine_get_state_rows(self._h, None, _np_ptr(vel), None), "get_state")
+        vel = np.asarray(vel, dtype=np.float64)
         cols = [np.ascontiguousarray(pos[:, d]) for d in range(3)] + \
                [np.ascontiguousarray(vel[:, d]) for d in range(3)]
         check(lib().rbx_engine_set_state(self._h, _np_ptr(self._gid), _np_ptr(self._typ),
@@ -602,10 +606,10 @@ class Engine:
                                          _np_ptr(v_out), _np_ptr(f_out)), "rbx_engine_step_host")
 
     def get_state(self):
-        a = [np.zeros(self.n) for _ in range(9)]
-        check(lib().rbx_engine_get_state(self._h, *[_np_ptr(v) for v in a]), "get_state")
-        return {"pos": np.stack(a[0:3], 1), "vel": np.stack(a[3:6], 1),
-                "force": np.stack(a[6:9], 1)}
+        out = {k: np.empty((self.n, 3)) for k in ("pos", "vel", "force")}
+        check(lib().rbx_engine_get_state_rows(self._h, *[_np_ptr(v) for v in out.values()]),
+              "get_state")
+        return out
 
     def force_parts(self):
         fp = np.zeros((self.n, 3))
