@@ -612,59 +612,124 @@ k_full_list(DBox b, int dimx, int dimy, int dimz, double cut2, float cut2_up, fl
 // list and ceil((cut_off + skin) / r_core) for RBL (linked_cell_locator.cpp:
 // 26-40), and its (2c + 1)^3 stencil wraps onto the same cell more than once
 // along an axis with fewer than 2c + 1 cells, WrapFullNeighborStencilIndex in
-// full_neighbor_list_op.hip.cu:9-80, listing those pairs repeatedly.)  A warp
-// per atom; hits are appended in index order through a ballot prefix, far
-// pairs (see FarSplit) to the back.
+// full_neighbor_list_op.hip.cu:9-80, listing those pairs repeatedly.)
+//
+// Bound by latency and issue: n / 32 tests a lane of a warp, a few blocks an SM.
+// A warp takes SL_C centre atoms; a block stages the fixed-point records of all
+// atoms tile by tile.  Their wrapped differences are the minimum image, and
+// |d|^2 in FP32 decides every pair outside a guard band (the RBL kernels'
+// bound); the FP64 predicate settles the rest.  Hits are appended in index order
+// through a ballot prefix, far pairs (certainly at least r_near, see FarSplit)
+// to the back.  Measured, B200, 1,000 / 1,500 / 3,000 atoms: 10.8 / 14.9 / 36.0 us;
+// 16.5 / 23.6 / 43.0 us with a warp an atom and FP64 distances.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128)
-k_full_list_small(DBox b, double cut2, double near2, int n, const double* __restrict__ x,
-                  const double* __restrict__ y, const double* __restrict__ z, int cap,
-                  int* __restrict__ count, int* __restrict__ nbrs, int* __restrict__ overflow,
-                  int* __restrict__ far, long long* __restrict__ total) {
-  const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (i >= n) return;
+constexpr int SL_WARPS = 8;
+constexpr int SL_C = 2;       // centre atoms of a warp
+constexpr int SL_TILE = 1024; // atoms staged at a time
+
+struct SmallScreen {
+  float lo, hi, far;  // thresholds of the fixed-point |d|^2: cutoff band, certainly far
+  float w[3];         // L_d / L_max
+};
+
+template <bool SPLIT>
+__global__ void __launch_bounds__(32 * SL_WARPS)
+k_full_list_small(DBox b, double cut2, SmallScreen sc, int n, const uint4* __restrict__ atoms,
+                  const double* __restrict__ x, const double* __restrict__ y,
+                  const double* __restrict__ z, int cap, int* __restrict__ count,
+                  int* __restrict__ nbrs, int* __restrict__ overflow, int* __restrict__ far,
+                  long long* __restrict__ total) {
+  __shared__ uint4 s_u[SL_TILE];
+  const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const unsigned lt = (1u << lane) - 1u;
-  const double xi = x[i], yi = y[i], zi = z[i];
-  int nf = 0, nb = 0;  // near (front) and far (back) entries found
-  int* row = nbrs + (size_t)i * cap;
-  for (int j0 = 0; j0 < n; j0 += 32) {
-    const int j = j0 + lane;
-    double d2 = INFINITY;
-    if (j < n && j != i) d2 = dist2_list(b, xi, yi, zi, x[j], y[j], z[j]);
-    const bool hit = d2 < cut2;
-    const bool is_far = hit && !(d2 < near2);
-    const unsigned mh = __ballot_sync(0xffffffffu, hit && !is_far);
-    const unsigned mf = __ballot_sync(0xffffffffu, is_far);
-    if (hit && !is_far) {
-      const int pos = nf + __popc(mh & lt);
-      if (pos < cap) row[pos] = j;
-    } else if (is_far) {
-      const int k = nb + __popc(mf & lt);
-      if (k < cap) row[cap - 1 - k] = j;
+  const int i0 = (blockIdx.x * SL_WARPS + warp) * SL_C;
+  uint4 u[SL_C];
+  int nf[SL_C], nb[SL_C];
+#pragma unroll
+  for (int q = 0; q < SL_C; ++q) {
+    u[q] = atoms[min(i0 + q, n - 1)];
+    nf[q] = nb[q] = 0;
+  }
+  int* const row = nbrs + (size_t)i0 * cap;
+  for (int t0 = 0; t0 < n; t0 += SL_TILE) {
+    const int tn = min(SL_TILE, n - t0);
+    __syncthreads();  // the previous tile has been read
+    for (int t = threadIdx.x; t < tn; t += 32 * SL_WARPS) s_u[t] = atoms[t0 + t];
+    __syncthreads();
+    if (i0 >= n) continue;
+    for (int k0 = 0; k0 < tn; k0 += 32) {
+      const int j = t0 + k0 + lane;
+      const bool there = k0 + lane < tn;
+      const uint4 v = s_u[min(k0 + lane, tn - 1)];
+      float d2[SL_C];
+      bool odd = false;
+#pragma unroll
+      for (int q = 0; q < SL_C; ++q) {
+        const float dx = (float)(int)(v.x - u[q].x) * sc.w[0],
+                    dy = (float)(int)(v.y - u[q].y) * sc.w[1],
+                    dz = (float)(int)(v.z - u[q].z) * sc.w[2];
+        d2[q] = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        odd |= (d2[q] >= sc.lo) & (d2[q] < sc.hi);
+      }
+      const bool settle = __any_sync(0xffffffffu, odd & there);
+#pragma unroll
+      for (int q = 0; q < SL_C; ++q) {
+        const int i = i0 + q;
+        bool in = d2[q] < sc.lo;
+        if (settle && d2[q] >= sc.lo && d2[q] < sc.hi && there && i < n)
+          in = dist2_list(b, x[i], y[i], z[i], x[j], y[j], z[j]) < cut2;
+        in = in & there & (j != i) & (i < n);
+        const bool bk = SPLIT & in & (d2[q] >= sc.far);
+        const unsigned mb = SPLIT ? __ballot_sync(0xffffffffu, bk) : 0u;
+        const unsigned mf = __ballot_sync(0xffffffffu, in) ^ mb;
+        const int pos = (bk ? nb[q] : nf[q]) + __popc((bk ? mb : mf) & lt);
+        store_if(in & (pos < cap), row + (q * cap + (bk ? cap - 1 - pos : pos)), j);
+        nb[q] += __popc(mb);
+        nf[q] += __popc(mf);
+      }
     }
-    nf += __popc(mh);
-    nb += __popc(mf);
   }
-  if (lane == 0) {
-    count[i] = nf + nb;
-    if (far) far[i] = nb;
-    if (nf + nb > cap) atomicOr(overflow, 1);
-    if (total) atomicAdd((unsigned long long*)total, (unsigned long long)(nf + nb));
+  int sum = 0;
+#pragma unroll
+  for (int q = 0; q < SL_C; ++q) {
+    if (i0 + q >= n) continue;
+    sum += nf[q] + nb[q];
+    if (lane == q) {
+      count[i0 + q] = nf[q] + nb[q];
+      if (SPLIT) far[i0 + q] = nb[q];
+      if (nf[q] + nb[q] > cap) atomicOr(overflow, 1);
+    }
   }
+  if (total && lane == 0 && sum) atomicAdd((unsigned long long*)total, (unsigned long long)sum);
 }
 
-int launch_full_list_small(const DBox& b, double cutoff, int n, const double* x, const double* y,
-                           const double* z, int cap, int* count, int* nbrs, int* overflow,
-                           cudaStream_t st, const FarSplit* split, long long* total) {
+int launch_full_list_small(const DBox& b, double cutoff, int n, const uint4* atoms,
+                           const double* x, const double* y, const double* z, int cap,
+                           int* count, int* nbrs, int* overflow, cudaStream_t st,
+                           const FarSplit* split, long long* total) {
   if (n <= 0) return RBX_OK;
-  // near threshold raised by 1e-9 relative: FP64 rounding never moves a pair
-  // that could come within r_core before the next rebuild to the far segment
-  const double near2 =
-      split ? split->r_near * split->r_near * (1.0 + 1e-9) : (double)INFINITY;
-  k_full_list_small<<<(n + 3) / 4, 128, 0, st>>>(b, cutoff * cutoff, near2, n, x, y, z, cap,
-                                                 count, nbrs, overflow,
-                                                 split ? split->far : nullptr, total);
+  // the fixed-point screen's guard band in r^2 (see PairParams' screens):
+  // quantisation below 6 s |d| and FP32 rounding below 2e-6 relative, several
+  // times both
+  double L = 0.0;
+  for (int d = 0; d < 3; ++d) L = fmax(L, b.len[d]);
+  const double qerr = 64.0 * (L / 4294967296.0) * (cutoff + 1.0);
+  const double cut2 = cutoff * cutoff;
+  const IntScreen c = make_screen(cut2, L, 1e-4 + 8e-6 * cut2 + qerr);
+  SmallScreen sc;
+  sc.lo = c.lo;
+  sc.hi = c.hi;
+  sc.far = INFINITY;
+  if (split) {
+    const double near2 = split->r_near * split->r_near;
+    sc.far = make_screen(near2, L, 1e-4 + 8e-6 * near2 + qerr).hi;
+  }
+  for (int d = 0; d < 3; ++d) sc.w[d] = (float)(b.len[d] / L);
+  const int per_block = SL_WARPS * SL_C;
+  const auto kern = split ? k_full_list_small<true> : k_full_list_small<false>;
+  kern<<<(n + per_block - 1) / per_block, 32 * SL_WARPS, 0, st>>>(
+      b, cut2, sc, n, atoms, x, y, z, cap, count, nbrs, overflow, split ? split->far : nullptr,
+      total);
   count_launch();
   return check_launch("full_list_small");
 }
@@ -976,12 +1041,17 @@ size_t full_list_scratch_bytes(int n, int ncell) {
 int launch_full_list(const DBox& b, const int dims[3], double cutoff, int n, const double* x,
                      const double* y, const double* z, const int* cell_start, int cap,
                      int* count, int* nbrs, int* overflow, void* scratch, cudaStream_t st,
-                     const FarSplit* split, long long* total) {
+                     const FarSplit* split, long long* total, const uint4* atoms) {
   const int ncell = dims[0] * dims[1] * dims[2];
   if (n <= 0) return RBX_OK;
-  if (dims[0] < 3 || dims[1] < 3 || dims[2] < 3)
-    return launch_full_list_small(b, cutoff, n, x, y, z, cap, count, nbrs, overflow, st, split,
-                                  total);
+  if (dims[0] < 3 || dims[1] < 3 || dims[2] < 3) {
+    if (!atoms) {
+      set_error("full_list: fewer than three cells along an axis need fixed-point records");
+      return RBX_ERR_INVALID;
+    }
+    return launch_full_list_small(b, cutoff, n, atoms, x, y, z, cap, count, nbrs, overflow, st,
+                                  split, total);
+  }
   const double cut2 = cutoff * cutoff;
   double emax = 0.0;
   for (int d = 0; d < 3; ++d) emax = fmax(emax, b.len[d] / dims[d]);

@@ -410,7 +410,7 @@ int rbx_engine::rebuild_launches(cudaStream_t s, bool in_graph) {
   ETRY(launch_to_fixed(dbox, n, x, y, z, q, atoms, s));
   ETRY(launch_full_list(dbox, dims, prm.cut_off + prm.skin, n, x, y, z, cell_start, cap,
                         cand_count, cand, dflags + 1, list_scratch, s, far_split(),
-                        (long long*)cand_total));
+                        (long long*)cand_total, atoms));
   return RBX_OK;
 }
 
@@ -450,7 +450,7 @@ int rbx_engine::rebuild() {
     ETRY(launch_zero_u64((unsigned long long*)cand_total, st));
     ETRY(launch_full_list(dbox, dims, prm.cut_off + prm.skin, n, x, y, z, cell_start, cap,
                           cand_count, cand, dflags + 1, list_scratch, st, far_split(),
-                          (long long*)cand_total));
+                          (long long*)cand_total, atoms));
   }
   set_error("candidate list capacity did not converge");
   return RBX_ERR_CAPACITY;

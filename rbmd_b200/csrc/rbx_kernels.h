@@ -267,10 +267,12 @@ struct FarSplit {
   double r_near;
   int* far;
 };
+// atoms: fixed-point records, needed with fewer than three cells along an axis.
 int launch_full_list(const DBox& b, const int dims[3], double cutoff, int n, const double* x,
                      const double* y, const double* z, const int* cell_start, int cap,
                      int* count, int* nbrs, int* overflow, void* scratch, cudaStream_t st,
-                     const FarSplit* split = nullptr, long long* total = nullptr);
+                     const FarSplit* split = nullptr, long long* total = nullptr,
+                     const uint4* atoms = nullptr);
 // Force adjoint (rbx_adjoint.cu).  Pair part: per-atom dL/dr, dL/dq and
 // per-block partials [nblocks][2 ntypes + 1] (d_eps, d_sigma, d_alpha).
 int adj_pair_blocks(int n);
