@@ -218,17 +218,22 @@ struct rbx_batch {
     return RBX_OK;
   }
 
-  // AUTO: the phased graph for replicas of fewer than kPhasedMeanAtoms atoms
-  // on average, else the branches.  One launch per phase pays off over many
-  // small replicas (910 x 2,000 atoms: 5.1x the branches, whose thousand-node
-  // graph is bound by node scheduling); at 256 x 7,100 atoms the designs are
-  // level, and with larger replicas the branches win (the phased force
-  // launches wait for every replica's rebuild).
+  // AUTO: the branches for replicas of kPhasedMeanAtoms atoms or more on
+  // average (the phased force launches wait for every replica's rebuild) and
+  // for nine to kBranchReplicas smaller ones; else the phased graph: one launch
+  // per phase pays off over many small replicas, whose graph of branches is
+  // bound by node scheduling, and a handful makes a small graph either way.
+  // Measured, us per step, phased and branches: 192 x 1,753 atoms 1864 / 3414,
+  // 96 x 2,095 1214 / 1314, 48 x 4,448 940 / 843, 24 x 1,990 367 / 337,
+  // 12 x 4,393 350 / 318, 8 x 1,364 136 / 122, 64 x 5,120 1523 / 1410;
+  // 910 x 2,000 atoms 5.1x in favour of phased.
   static constexpr int kPhasedMeanAtoms = 5000;
+  static constexpr size_t kBranchReplicas = 64;
   int capture() {
     long long atoms = 0;
     for (rbx_engine* e : eng) atoms += e->n;
-    const bool small = atoms < (long long)kPhasedMeanAtoms * (long long)eng.size();
+    const bool small = atoms < (long long)kPhasedMeanAtoms * (long long)eng.size() &&
+                       (eng.size() <= 8 || eng.size() > kBranchReplicas);
     if (mode == RBX_BATCH_PHASED || (mode == RBX_BATCH_AUTO && small)) {
       const int rc = capture_phased();
       if (rc == RBX_OK || mode == RBX_BATCH_PHASED) return rc;
