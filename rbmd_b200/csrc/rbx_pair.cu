@@ -718,11 +718,13 @@ RefLen<T> ref_len(const DBox& b) {
 // A warp an atom: lanes take consecutive candidates and append their hits
 // through ballot prefixes, so both lists keep the candidates' order.  (One
 // thread an atom walked 485 candidates in series with uncoalesced reads.)
-// Bound by the gathers and the integer work of the hash: 598 -> 177 us for the
-// float build's 50,000 atoms x 485 candidates.
+// Bound by the latency of the gathers, then the integer work of the hash; every
+// candidate is hashed (no branch) and eight blocks an SM are resident.  The float
+// build's 50,000 atoms x 485 candidates: 598 us serial; 177, 153, 146, 144 us at
+// the compiler's own choice of registers and at five, six and eight blocks.
 // FREQ_LOW2: freq is 1, 2 or 4 and the batch test needs two bits of the hash.
 template <typename T, bool FREQ_LOW2>
-__global__ void __launch_bounds__(PAIR_BLOCK)
+__global__ void __launch_bounds__(PAIR_BLOCK, 8)
 k_ref_rbl_filter(T core2, T force2, int n, const int* __restrict__ gid,
                  const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ z,
                  const int* __restrict__ cstart, const int* __restrict__ cend,
@@ -733,7 +735,7 @@ k_ref_rbl_filter(T core2, T force2, int n, const int* __restrict__ gid,
                  int* __restrict__ realloc, DivTest div, int epoch) {
   constexpr int U = 2;  // candidates a lane takes per iteration
   const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * PAIR_WARPS + (int)(threadIdx.x >> 5);
+  const int i = blockIdx.x * PAIR_WARPS + (int)__shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   if (i >= n) return;
   const unsigned lt = lanemask_lt();
   const unsigned mask = (1u << div.shift) - 1u;
@@ -744,13 +746,15 @@ k_ref_rbl_filter(T core2, T force2, int n, const int* __restrict__ gid,
   const T xi = x[i], yi = y[i], zi = z[i];
   const int c0 = cstart[i], c1 = cend[i];
   for (int pos = c0; pos < c1; pos += 32 * U) {
-    int j[U];
+    int j[U], g[U];
     T d2[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int k = pos + 32 * u + lane;
       j[u] = k < c1 ? cand[k] : i;
     }
+#pragma unroll
+    for (int u = 0; u < U; ++u) g[u] = gid[j[u]];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const T dx = ref_min_image<T>(xi - x[j[u]], b.len[0]),
@@ -765,11 +769,10 @@ k_ref_rbl_filter(T core2, T force2, int n, const int* __restrict__ gid,
     for (int u = 0; u < U; ++u) {
       const bool other = j[u] != i;
       const bool in_core = other && d2[u] < core2;
-      bool in_shell = other && !in_core && d2[u] < force2;
-      if (in_shell) {
-        const unsigned long long kb = rbl_key_b(gid[j[u]]);
-        in_shell = FREQ_LOW2 ? rbl_selected_low2(ea ^ kb, mask) : rbl_selected(ea, kb, div);
-      }
+      const unsigned long long kb = rbl_key_b(g[u]);
+      const bool in_shell =
+          other & !in_core & (d2[u] < force2) &
+          (FREQ_LOW2 ? rbl_selected_low2(ea ^ kb, mask) : rbl_selected(ea, kb, div));
       const unsigned mc = __ballot_sync(0xffffffffu, in_core);
       const unsigned ms = __ballot_sync(0xffffffffu, in_shell);
       if (in_core) {

@@ -327,8 +327,8 @@ k_verlet_sog(SogPairParams sp, int n, const double* __restrict__ x, const double
 // sums its pairs in FP32 and the warp reduces in FP64.  Four candidates a lane
 // are loaded before any is used, and the reciprocal is the fast one with a
 // Newton step (the division's slow path kept the loop from overlapping): 134 ->
-// 78 us at 50,021 atoms, 485 candidates an atom.
-__global__ void __launch_bounds__(SOG_PAIR_BLOCK)
+// 76 us at 50,021 atoms, 485 candidates an atom (twelve blocks an SM; 78 at ten).
+__global__ void __launch_bounds__(SOG_PAIR_BLOCK, 12)
 k_verlet_sog_mixed(SogPairParams sp, float sfx, float sfy, float sfz, int n,
                    const uint4* __restrict__ atoms, const int* __restrict__ type,
                    const int* __restrict__ cand_count, const int* __restrict__ cand, int cap,
@@ -342,7 +342,7 @@ k_verlet_sog_mixed(SogPairParams sp, float sfx, float sfy, float sfz, int n,
     s_s6[t] = (float)sp.lj_s6[t];
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, wib = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int i = blockIdx.x * (SOG_PAIR_BLOCK / 32) + wib;
   if (i >= n) return;
   const uint4 ai = atoms[i];
