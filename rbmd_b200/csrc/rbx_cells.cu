@@ -251,7 +251,7 @@ k_cell_segsort(int ncell, int n, const int* __restrict__ start, const unsigned* 
 // lane, as an earlier builder did; and a small box fills the chip (that
 // builder ran one warp per 32 atoms through all 27 cells).  Measured, B200,
 // rho* = 0.8, cutoff 5.3, that builder and this one: 200,000 atoms 660 and
-// 456 us (split rows 915 and 600), 20,000 atoms split 214 and 84, 4,000 atoms
+// 466 us (split rows 915 and 614), 20,000 atoms split 214 and 92, 4,000 atoms
 // split 171 and 42.
 // ---------------------------------------------------------------------------
 constexpr int NL_WARPS = 8;                // warps of a block
@@ -269,7 +269,7 @@ static size_t full_list_chunks(int n, int ncell) { return (size_t)(n / NL_CH) + 
 
 // Device scratch of one list build.
 struct ListTables {
-  float4* rel;      // per atom: FP32 position relative to its cell's centre
+  float4* rel;      // plain rows: an atom's FP32 position relative to its cell's centre
   float4 *lo, *hi;  // per chunk: its box relative to its cell's centre, rounded outwards
   int* group_cell;  // per group: its cell, -1 for an index between two cells
 };
@@ -302,7 +302,9 @@ k_chunk_boxes(DBox b, int dimx, int dimy, int dimz, const double* __restrict__ x
       }
     }
     if (!ok) continue;
-    T.rel[a] = make_float4((float)(p[0] - o[0]), (float)(p[1] - o[1]), (float)(p[2] - o[2]), 0.f);
+    if (T.rel)
+      T.rel[a] =
+          make_float4((float)(p[0] - o[0]), (float)(p[1] - o[1]), (float)(p[2] - o[2]), 0.f);
     if (threadIdx.x % NL_CH == 0) {
       const int k = base + (a - cs) / NL_CH;
       T.lo[k] = make_float4(lo[0], lo[1], lo[2], 0.f);
@@ -329,8 +331,9 @@ struct FullListSmem {
   int first[NL_BATCH + 1];              // its first atom
   unsigned short meta[NL_BATCH];        // stencil cell | atoms << 8
   unsigned short pick[NL_WARPS][NL_BATCH + 8];  // a warp's surviving chunks
-  float4 shift[27];                     // centre of a stencil cell's image, relative to the
+  float4 edge[27];                      // centre of a stencil cell's image, relative to the
   float shl[27][3], shh[27][3];         // centre cell's; and rounded down and up
+  double shift[27][3];                  // its periodic image minus the centre cell's centre
   int cs[27], ce[27], cb[27];           // atom range and first chunk index of a stencil cell
   int word0[28];                        // first cull word of a stencil cell
   unsigned mask[NL_WORDS];              // surviving chunks of a word
@@ -356,8 +359,11 @@ k_full_list(DBox b, int dimx, int dimy, int dimz, double cut2, float cut2_up, fl
   const int cs = cell_start[c], ce = cell_start[c + 1];
   const int g = (int)blockIdx.x - group_base(c, cs);
   const int i0 = cs + NL_GROUP * g + NL_CH * warp;  // this warp's first centre atom
+  const int cz = c / (dimx * dimy), cy = (c / dimx) % dimy, cx = c % dimx;
+  const double ox = b.lo[0] + (cx + 0.5) * (b.len[0] / dimx);  // the centre cell's centre
+  const double oy = b.lo[1] + (cy + 0.5) * (b.len[1] / dimy);
+  const double oz = b.lo[2] + (cz + 0.5) * (b.len[2] / dimz);
   if (warp == 0) {  // the stencil cells, and their cull words
-    const int cz = c / (dimx * dimy), cy = (c / dimx) % dimy, cx = c % dimx;
     int words = 0;
     if (lane < 27) {
       // stencil order of ComputeFullNeighborStencilCellOnTheFly:
@@ -365,20 +371,23 @@ k_full_list(DBox b, int dimx, int dimy, int dimz, double cut2, float cut2_up, fl
       // cell edges away
       const int o[3] = {lane % 3 - 1, (lane / 3) % 3 - 1, lane / 9 - 1};
       const int dim[3] = {dimx, dimy, dimz}, at[3] = {cx + o[0], cy + o[1], cz + o[2]};
+      const double cen[3] = {ox, oy, oz};
       int w[3];
-      float sh[3];
+      float ed[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
         w[d] = at[d] < 0 ? at[d] + dim[d] : (at[d] >= dim[d] ? at[d] - dim[d] : at[d]);
         const double e = o[d] * (b.len[d] / dim[d]);
-        sh[d] = (float)e;
+        ed[d] = (float)e;
+        S.shift[lane][d] =
+            (at[d] < 0 ? -b.len[d] : (at[d] >= dim[d] ? b.len[d] : 0.0)) - cen[d];
         // one FP64 rounding of the edge and of the two centres: 4 ulp of the
         // box's extent cover them
         const double slack = 1e-15 * (fabs(b.lo[d]) + b.len[d]);
         S.shl[lane][d] = __double2float_rd(__dsub_rd(e, slack));
         S.shh[lane][d] = __double2float_ru(__dadd_ru(e, slack));
       }
-      S.shift[lane] = make_float4(sh[0], sh[1], sh[2], 0.f);
+      S.edge[lane] = make_float4(ed[0], ed[1], ed[2], 0.f);
       const int nc = (w[2] * dimy + w[1]) * dimx + w[0];
       S.cs[lane] = cell_start[nc];
       S.ce[lane] = cell_start[nc + 1];
@@ -402,11 +411,12 @@ k_full_list(DBox b, int dimx, int dimy, int dimz, double cut2, float cut2_up, fl
 #pragma unroll
   for (int q = 0; q < NL_CH; ++q) {
     const bool live = i0 + q < ce;
-    const float4 u = T.rel[live ? i0 + q : cs];
-    const float uu = fmaf(u.x, u.x, fmaf(u.y, u.y, u.z * u.z));
-    ax[q] = live ? -2.f * u.x : 0.f;
-    ay[q] = live ? -2.f * u.y : 0.f;
-    az[q] = live ? -2.f * u.z : 0.f;
+    const int i = live ? i0 + q : cs;
+    const float ux = (float)(x[i] - ox), uy = (float)(y[i] - oy), uz = (float)(z[i] - oz);
+    const float uu = fmaf(ux, ux, fmaf(uy, uy, uz * uz));
+    ax[q] = live ? -2.f * ux : 0.f;
+    ay[q] = live ? -2.f * uy : 0.f;
+    az[q] = live ? -2.f * uz : 0.f;
     lo_i[q] = live ? lo_band - uu : -INFINITY;
     hi_i[q] = live ? hi_band - uu : -INFINITY;
     near_i[q] = near2 - uu;  // far pairs: d above this
@@ -519,13 +529,20 @@ k_full_list(DBox b, int dimx, int dimy, int dimz, double cut2, float cut2_up, fl
       for (int t = threadIdx.x; t < nb * NL_CH; t += NL_BLOCK) {  // its atoms
         const int slot = t / NL_CH, u = t % NL_CH;
         const int meta = S.meta[slot];
-        const float4 sh = S.shift[meta & 255];
+        const double* const sh = S.shift[meta & 255];
         float4 v = make_float4(0.f, 0.f, 0.f, INFINITY);
         if (u < meta >> 8) {
-          const float4 r = T.rel[S.first[slot] + u];
-          v.x = r.x + sh.x;
-          v.y = r.y + sh.y;
-          v.z = r.z + sh.z;
+          const int a = S.first[slot] + u;
+          if (SPLIT) {
+            v.x = (float)(x[a] + sh[0]);
+            v.y = (float)(y[a] + sh[1]);
+            v.z = (float)(z[a] + sh[2]);
+          } else {
+            const float4 r = T.rel[a], e = S.edge[meta & 255];
+            v.x = r.x + e.x;
+            v.y = r.y + e.y;
+            v.z = r.z + e.z;
+          }
           v.w = fmaf(v.x, v.x, fmaf(v.y, v.y, v.z * v.z));
         }
         S.atom[t] = v;
@@ -1060,15 +1077,18 @@ int launch_full_list(const DBox& b, const int dims[3], double cutoff, int n, con
   double emax = 0.0;
   for (int d = 0; d < 3; ++d) emax = fmax(emax, b.len[d] / dims[d]);
   // FP32 screening error of |v|^2 - 2 u.v against C - |u|^2.  u (|u_d| <= e/2)
-  // is rounded once relative to its cell's centre, v (|v_d| <= 3e/2) once
-  // relative to its own cell's centre (e/2), in the image's offset (e) and in
-  // their sum (3e/2), so a coordinate of v - u is off by at most 3.5 e 2^-24,
-  // which moves |d|^2 by at most 7 sqrt(3) r e 2^-24 (e = largest cell edge,
-  // r = cutoff); the roundings of |v|^2, the three FMAs, |u|^2 and C - |u|^2
-  // add at most (60 e^2 + 3 r^2) 2^-24.  Pairs within twice that of the cutoff
-  // take the FP64 path.
+  // is rounded once relative to its cell's centre.  v (|v_d| <= 3e/2) is rounded
+  // once relative to the same centre in split rows, where its value also places
+  // the pair in the near or the far segment; in plain rows it is the FP32 sum
+  // of the image's offset (e) and of the position relative to its own cell's
+  // centre (e/2), read as one word an atom (200,000 atoms: 466 us, 485 with the
+  // FP64 positions).  A coordinate of v - u is off by at most 2 or 3.5 e 2^-24,
+  // which moves |d|^2 by at most 4 or 7 sqrt(3) r e 2^-24 (e = largest cell
+  // edge, r = cutoff); the roundings of |v|^2, the three FMAs, |u|^2 and
+  // C - |u|^2 add at most (60 e^2 + 3 r^2) 2^-24.  Pairs within twice that of
+  // the cutoff take the FP64 path.
   const double err =
-      (7.0 * sqrt(3.0) * cutoff * emax + 60.0 * emax * emax + 3.0 * cut2) / 16777216.0;
+      ((split ? 4.0 : 7.0) * sqrt(3.0) * cutoff * emax + 60.0 * emax * emax + 3.0 * cut2) / 16777216.0;
   const double band = 2.0 * err;
   const float lo_band = (float)(cut2 - band), hi_band = (float)(cut2 + band);
   float cut2_up = (float)cut2;  // rounded up
@@ -1077,7 +1097,7 @@ int launch_full_list(const DBox& b, const int dims[3], double cutoff, int n, con
   list_pieces(n, ncell, piece);
   char* p = (char*)scratch;
   ListTables T;
-  T.rel = (float4*)p;
+  T.rel = split ? nullptr : (float4*)p;
   T.lo = (float4*)(p + piece[0]);
   T.hi = (float4*)(p + piece[0] + piece[1]);
   T.group_cell = (int*)(p + piece[0] + piece[1] + piece[2]);

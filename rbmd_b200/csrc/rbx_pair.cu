@@ -160,13 +160,18 @@ __device__ __forceinline__ void write_block_partial(double (*s_acc)[3], double* 
 // SM (32 registers, no spills), the FP64 form six (40, a few spilled words that
 // stay in L1).  What keeps the registers down is that the warp index comes
 // through a shuffle: atom, row and loop state are then uniform.  Queue pushes
-// are predicated stores at ballot prefixes; the far segment is read in full
-// 128-entry batches from the row's end, so only its front batch tests for
-// entries that are none.  Measured, B200, 200,000-atom LJ electrolyte: mixed
-// 464 -> 380 us (four blocks of 64 registers, per-thread state before; 415,
-// 397, 389, 381 at four to seven blocks), FP64 697 -> 554 us (three blocks
-// before; 608, 568 at four and five); water, 73,000 atoms: 271 -> 244 and
-// 523 -> 371 us.  A second queue that window-tests the selected far pairs
+// are predicated stores at ballot prefixes.  Measured, B200, 200,000-atom LJ
+// electrolyte: mixed 464 -> 390 us (four blocks of 64 registers, per-thread
+// state before; 415, 397, 389, 381, 378 at four to eight blocks with the far
+// segment queued in another order, below), FP64 697 -> 552 us (three blocks
+// before; 608, 568 at four and five); water, 73,000 atoms: 271 -> 247 and
+// 523 -> 370 us.
+//
+// The queue holds the pairs in row order: a lane's FP32 sums, and with them the
+// mixed form's forces, then depend on the row alone.  Batches from the row's end
+// queued entry by entry across the lanes need fewer instructions (378 us), but
+// change every force by an FP32 rounding, which 40 steps of water grow to a
+// pair at r_core that enters a step early.  A second queue that window-tests the selected far pairs
 // before they take a force slot was slower in the mixed form (+10 %), and split
 // rows with it slower than unsplit ones in FP64 (677 us then, 607 unsplit).
 // ---------------------------------------------------------------------------
@@ -386,40 +391,54 @@ __device__ __forceinline__ void rbl_fused_body(
       drain_full();
     }
 
-    // far segment: batch hash first; selected pairs are queued with the window
-    // test still to do
-    // 128 entries, four a lane (e); lanes' entries below `skip` are not in the
-    // segment
+    // far segment: batch hash first; selected pairs are queued, in row order,
+    // with the window test still to do.  128 entries a batch, four a lane, from
+    // the 16-byte boundary at or below the segment's start (rows start on
+    // 128-byte lines, cap % 32 == 0): only the first and the last batch hold
+    // entries that are not the segment's (skip: how many of the lane's first).
     auto far_batch = [&](int4 e, int skip) {
       const int jj[4] = {e.x, e.y, e.z, e.w};
       unsigned long long kb[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) kb[u] = __ldg(key_b + jj[u]);
+      bool sel[4];
+      unsigned at = qn;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const bool sel = batch_selected<SEL>(ea ^ kb[u], fmask, pp.div) & (u >= skip);
-        const unsigned m = __ballot_sync(0xffffffffu, sel);
-        push_if(sel, wq_at + 4 * (qn + __popc(m & lt)), jj[u] | (QF_SHELL | QF_CHECK));
+        sel[u] = batch_selected<SEL>(ea ^ kb[u], fmask, pp.div) & (u >= skip);
+        const unsigned m = __ballot_sync(0xffffffffu, sel[u]);
+        at += __popc(m & lt);
         qn += __popc(m);
+      }
+      at = wq_at + 4 * at;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        push_if(sel[u], at, jj[u] | (QF_SHELL | QF_CHECK));
+        at += sel[u] ? 4 : 0;
       }
       drain_full();
     };
-    {
-      // full batches from the row's end (rows start on 128-byte lines and
-      // cap % 32 == 0, so every lane's four entries are 16-byte aligned), then
-      // the ragged front one
-      int p0 = rows.cap - 128;
+    if (nb > 0) {
       const int fs = rows.cap - nb;  // first far entry
-      for (; p0 >= fs; p0 -= 128)
-        far_batch(__ldg(reinterpret_cast<const int4*>(row + p0) + lane), 0);
-      const int skip = fs - (p0 + 4 * lane);  // of this lane's entries
-      if (p0 + 128 > fs) {
+      int p0 = fs & ~3;
+      int skip = lane == 0 ? fs - p0 : 0;
+      for (; p0 + 128 <= rows.cap; p0 += 128) {
+        int4 e = __ldg(reinterpret_cast<const int4*>(row + p0) + lane);
+        if (skip > 0) e.x = i;  // what lies before the segment is no entry
+        if (skip > 1) e.y = i;
+        if (skip > 2) e.z = i;
+        far_batch(e, skip);
+        skip = 0;
+      }
+      if (p0 < rows.cap) {
         int4 e = make_int4(i, i, i, i);
-        if (skip < 4) {
-          e = __ldg(reinterpret_cast<const int4*>(row + p0 + 4 * lane));
-          if (skip > 0) e.x = i;  // what lies before the segment is no entry
+        if (p0 + 4 * lane < rows.cap) {
+          e = __ldg(reinterpret_cast<const int4*>(row + p0) + lane);
+          if (skip > 0) e.x = i;
           if (skip > 1) e.y = i;
           if (skip > 2) e.z = i;
+        } else {
+          skip = 4;
         }
         far_batch(e, skip);
       }
