@@ -231,8 +231,6 @@ int launch_ref_pair_verlet(const DBox& b, float cut_off, int n, double alpha, do
                            const float* x, const float* y, const float* z, float* fx,
                            float* fy, float* fz, float* flat_virial, double* epart,
                            cudaStream_t st);
-int launch_reduce_cols(int n, int ncols, const float* cols, double* out, double scale,
-                       cudaStream_t st);
 int launch_fix_rbl(int n, float* fx, float* fy, float* fz, float* mean_out, double* part,
                    cudaStream_t st);
 int launch_sum_i32(int n, const int* src, long long* out, cudaStream_t st);

@@ -956,12 +956,11 @@ k_ref_pair_verlet(RefLen<T> b, T cut_off, int n, double alpha, double sqa, doubl
 }
 
 // Deterministic column sums: out[c] = scale * sum_i cols[c*n + i] (one block per column).
-template <typename T>
-__global__ void k_reduce_cols(int n, const T* __restrict__ cols, double* __restrict__ out,
+__global__ void k_reduce_cols(int n, const double* __restrict__ cols, double* __restrict__ out,
                               double scale) {
   __shared__ double sh[8];
   double s = 0.0;
-  const T* col = cols + (size_t)blockIdx.x * n;
+  const double* col = cols + (size_t)blockIdx.x * n;
   for (int i = threadIdx.x; i < n; i += 256) s += col[i];
   s = block_sum_det<256>(s, sh);
   if (threadIdx.x == 0) out[blockIdx.x] = s * scale;
@@ -1299,21 +1298,12 @@ int launch_ref_pair_verlet(const DBox& b, float cut_off, int n, double alpha, do
                                          st);
 }
 
-template <typename T>
-int launch_reduce_cols_t(int n, int ncols, const T* cols, double* out, double scale,
-                         cudaStream_t st) {
-  if (ncols <= 0) return RBX_OK;
-  k_reduce_cols<T><<<ncols, 256, 0, st>>>(n, cols, out, scale);
-  count_launch();
-  return check_launch("reduce_cols");
-}
 int launch_reduce_cols(int n, int ncols, const double* cols, double* out, double scale,
                        cudaStream_t st) {
-  return launch_reduce_cols_t<double>(n, ncols, cols, out, scale, st);
-}
-int launch_reduce_cols(int n, int ncols, const float* cols, double* out, double scale,
-                       cudaStream_t st) {
-  return launch_reduce_cols_t<float>(n, ncols, cols, out, scale, st);
+  if (ncols <= 0) return RBX_OK;
+  k_reduce_cols<<<ncols, 256, 0, st>>>(n, cols, out, scale);
+  count_launch();
+  return check_launch("reduce_cols");
 }
 int launch_sum_i32(int n, const int* src, long long* out, cudaStream_t st) {
   if (n <= 0) return RBX_OK;
