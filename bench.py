@@ -54,10 +54,10 @@ UNIT = "atom-steps/s"
 # rows streamed once, plus neighbour-record and key gathers that miss L2).  Rows and
 # gathers grow with N, so the traffic is scaled by N.
 RBL_TRAFFIC_BYTES_PER_ATOM = 2151.0
-# Warp instructions per 32 candidates of the same launch (186.7 M for 47.9 M candidates in
-# the N = 100,000 capture), and the SM issue limit they are compared with: one warp
+# Warp instructions per 32 candidates of one launch (175.7 M for 47.8 M candidates in a
+# capture at N = 100,003), and the SM issue limit they are compared with: one warp
 # instruction per cycle per SM sub-partition, four per SM.
-RBL_WARP_INSTR_PER_32_CAND = 124.7
+RBL_WARP_INSTR_PER_32_CAND = 117.5
 ISSUE_SLOTS_PER_SM_CYCLE = 4
 
 

@@ -155,9 +155,10 @@ __device__ __forceinline__ void write_block_partial(double (*s_acc)[3], double* 
 // appended to a per-warp queue (index plus two flag bits) that is drained 32
 // pairs at a time from its tail.
 //
-// Bound by the latency of the gathers and, above that, by integer issue, so
-// resident warps count more than registers: the mixed form fits eight blocks an
-// SM (32 registers, no spills), the FP64 form six (40, a few spilled words that
+// Bound by the latency of the gathers until the warp slots are full, then by
+// integer issue (mixed, 100,000 atoms: 95 % of the slots, 76 % issue), so resident
+// warps count more than registers: the mixed form fits eight blocks an SM (32
+// registers, no spills), the FP64 form six (40, a few spilled words that
 // stay in L1).  What keeps the registers down is that the warp index comes
 // through a shuffle: atom, row and loop state are then uniform.  Queue pushes
 // are predicated stores at ballot prefixes.  Measured, B200, 200,000-atom LJ
