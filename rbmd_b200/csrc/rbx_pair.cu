@@ -764,14 +764,18 @@ k_ref_rbl_filter(T core2, T force2, int n, const int* __restrict__ gid,
   int nc = 0, ns = 0;
   const int out0 = core_start[i], ccap = core_cap[i];
   const T xi = x[i], yi = y[i], zi = z[i];
+  // positions count from the row's start, unsigned: stepping past the end of a
+  // row that ends near INT_MAX does not wrap
   const int c0 = cstart[i], c1 = cend[i];
-  for (int pos = c0; pos < c1; pos += 32 * U) {
+  const unsigned cnt = c1 > c0 ? (unsigned)c1 - (unsigned)c0 : 0u;
+  const int* const row = cand + c0;
+  for (unsigned pos = 0; pos < cnt; pos += 32 * U) {
     int j[U], g[U];
     T d2[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int k = pos + 32 * u + lane;
-      j[u] = k < c1 ? cand[k] : i;
+      const unsigned k = pos + 32 * u + lane;
+      j[u] = k < cnt ? row[k] : i;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) g[u] = gid[j[u]];
@@ -857,8 +861,9 @@ k_ref_pair_rbl(RefLen<T> b, T rs, T rc, int n, int pice, double alpha, double sq
   const double qi = q[i], si = sigma[ti], ei = eps[ti];
   double s[3] = {0, 0, 0}, c[3] = {0, 0, 0};
   const int a = start[i], e = end[i], ns = shell_num[i];
-  for (int t = a + lane; t < e; t += 32) {
-    const int j = core[t];
+  const unsigned nc = e > a ? (unsigned)e - (unsigned)a : 0u;  // does not wrap near INT_MAX
+  for (unsigned t = lane; t < nc; t += 32) {
+    const int j = core[(size_t)a + t];
     const RefPair<T> p = ref_pair<T>(b, xi, yi, zi, x[j], y[j], z[j]);
     if (p.d2 < rs2 && p.d2 > eps_t) {
       const double dx = p.dx, dy = p.dy, dz = p.dz, d2 = dx * dx + dy * dy + dz * dz;
@@ -916,8 +921,10 @@ k_ref_pair_verlet(RefLen<T> b, T cut_off, int n, double alpha, double sqa, doubl
   const T xi = x[i], yi = y[i], zi = z[i];
   const double qi = q[i];
   double a[11] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int t = start[i] + lane; t < end[i]; t += 32) {
-    const int j = nbrs[t];
+  const int r0 = start[i], r1 = end[i];
+  const unsigned nc = r1 > r0 ? (unsigned)r1 - (unsigned)r0 : 0u;  // does not wrap near INT_MAX
+  for (unsigned t = lane; t < nc; t += 32) {
+    const int j = nbrs[(size_t)r0 + t];
     const RefPair<T> p = ref_pair<T>(b, xi, yi, zi, x[j], y[j], z[j]);
     if (!(p.d2 < cut2)) continue;
     const double dx = p.dx, dy = p.dy, dz = p.dz, d2 = dx * dx + dy * dy + dz * dz;

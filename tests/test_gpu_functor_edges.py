@@ -1,6 +1,7 @@
 """The RBL filter, mean removal and row-wise state read-back at their edges:
 rows that overflow either capacity, candidate counts around a warp's 64-entry
-batch, one atom, more atoms than one block's partial sums.
+batch, rows that end at the largest 32-bit position, one atom, more atoms than
+one block's partial sums.
 
 Lists against a numpy restatement of the filter over the same candidates
 (whole numbers, exactly); the mean removal against numpy in FP64 (1e-12; float
@@ -68,6 +69,46 @@ def test_filter_capacities(cuda, rbx, freq, caps):
                 assert hshell[:int(snum[i]), i].tolist() == want[:scap].tolist()
     assert need.item() == most
     assert realloc.item() == (1 if most_core > ccap else 0)
+
+
+@pytest.mark.parametrize("real", ["f64", "f32"])
+def test_rows_at_the_last_positions(cuda, rbx, real):
+    """A row that ends at INT_MAX gives what it gives elsewhere (filter, RBL and
+    Verlet pair functors); its buffer holds 2^31 - 1 entries and no more."""
+    t = cuda.float64 if real == "f64" else cuda.float32
+    sfx = "" if real == "f64" else "_f32"
+    rng = np.random.default_rng(2)
+    n, L, k, end = 96, 6.0, 70, 2 ** 31 - 1
+    dev = lambda a: cuda.as_tensor(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    ints = lambda *s: cuda.zeros(s, dtype=cuda.int32, device="cuda")  # noqa: E731
+    g = np.stack(np.meshgrid(*[np.arange(5)] * 3), -1).reshape(-1, 3)[:n] * 1.2
+    x = [dev((g[:, d] + rng.uniform(0, 0.1, n))).to(t) for d in range(3)]
+    q, typ, gid = dev(rng.normal(size=n)).to(t), ints(n), dev(np.arange(n, dtype=np.int32))
+    one, box = cuda.ones(1, dtype=t, device="cuda"), rbx.Box.make([0] * 3, [L] * 3)
+    cand = rng.permutation(np.arange(1, n))[:k].astype(np.int32)
+    buf = cuda.empty(end, dtype=cuda.int32, device="cuda")
+    got = []
+    for at in (0, end - k):  # atom 0's row; the other rows are empty
+        buf[at:at + k] = dev(cand)
+        start = ints(n) + at
+        stop = start.clone()
+        stop[0] = at + k
+        core_start, core_end, core = ints(n), ints(n), ints(128)
+        shell, snum, need, realloc = ints(64 * n), ints(n), ints(1), ints(1)
+        getattr(rbx, "rbl_filter" + sfx)(2.0, 9.0, gid, *x, start, stop, buf, ints(n) + 128,
+                                         core_start, core_end, core, 64, shell, snum, need, box,
+                                         realloc, 2, 3)
+        F, V = [cuda.zeros_like(q) for _ in range(3)], [cuda.zeros_like(q) for _ in range(3)]
+        getattr(rbx, "pair_force_rbl" + sfx)(box, 2.0, 3.0, 10, 2, 0.16, 1.0, typ, one, one, start,
+                                             stop, buf, shell, snum, q, *x, *F)
+        vir, e = cuda.zeros(6 * n, dtype=t, device="cuda"), cuda.zeros(2, dtype=t, device="cuda")
+        getattr(rbx, "pair_force_verlet" + sfx)(box, 3.0, 0.16, 1.0, typ, one, one, start, stop,
+                                                buf, q, *x, *V, vir, e[:1], e[1:])
+        cuda.cuda.synchronize()
+        got.append([a.cpu().numpy() for a in (core_end, core, snum, shell, need, *F, *V, vir, e)])
+    assert got[0][0][0] > 0 and got[0][2][0] > 0 and np.abs(got[0][8]).max() > 0
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
 
 
 @pytest.mark.parametrize("n", [1, 255, 257, 148 * 256 + 3])
