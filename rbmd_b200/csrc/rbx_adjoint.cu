@@ -240,7 +240,8 @@ k_adj_pair(PairParams pp, int n, const uint4* __restrict__ atoms, const double* 
   }
   for (int t = 0; t < npar; ++t) {
     double v = warp_sum(t < 2 * nt ? mine[t * ADJ_BLOCK] : d_alpha);
-    if (t < nt) v /= 2.0 * eps_t[t];
+    // a type without force-carrying pairs sums to 0, also with eps = 0
+    if (t < nt && v != 0.0) v /= 2.0 * eps_t[t];
     if (lane == 0) s_part[warp][t] = v;
   }
   __syncthreads();
