@@ -690,8 +690,10 @@ int rbx_engine_set_alpha(rbx_engine* e, double alpha);
  * eps_ij = sqrt(eps_i eps_j), sigma_ij = (sigma_i + sigma_j)/2), dL/dq_i
  * ([n], host order), dL/dalpha ([1]) and dL/dr_i ([n][3], host order, the
  * Hessian-vector product), with the same RBL lists, batch selection and
- * k-samples held fixed.  Computed in FP64 in both forms (the mixed form's
- * rho(k) is recomputed in FP64); any output may be null.  RBL engines only.
+ * k-samples held fixed.  FP64 in the plain form; the mixed form takes FP32
+ * pair and k-space terms, summed in FP64.  sqrt(eps_i eps_j) has no derivative
+ * in an eps that is 0: dL/d(eps_t) of such a type is NaN when one of its atoms
+ * has a pair, 0 when none has.  Any output may be null.  RBL engines only.
  * No counterpart in the reference (RBMD has no adjoint). */
 int rbx_engine_force_vjp(rbx_engine* e, const double* g, double* d_eps, double* d_sigma,
                          double* d_charge, double* d_alpha, double* d_pos);

@@ -74,10 +74,10 @@ def pair_terms(pos, L, typ, sigma, eps, q, alpha, qqr2e, i, j, is_core, r_core, 
     ui = 1.0 / r2
     s6 = sg ** 6
     u = s6 * ui ** 3                      # sigma^6 / r^6
-    f_lj = -24 * e * (2 * u * u - u) * ui
+    df_de = -24 * (2 * u * u - u) * ui
+    f_lj = e * df_de
     # df/d(r^2) of the LJ term: 24 eps (14 s12 u^8 - 4 s6 u^5) in u = 1/r^2
     fp_lj = 24 * e * (14 * s6 * s6 * ui ** 8 - 4 * s6 * ui ** 5)
-    df_de = f_lj / e
     df_ds = -144 * e * (4 * u * u - u) * ui / sg
     r = np.sqrt(r2)
     b = math.sqrt(alpha)

@@ -45,7 +45,8 @@ __device__ __forceinline__ PairTerms pair_terms(double e, double sg, double qq, 
   const double ui = 1.0 / r2;
   const double s6 = sg * sg * sg * sg * sg * sg;
   const double u = s6 * ui * ui * ui;  // sigma^6 / r^6
-  const double f_lj = -24.0 * e * (2.0 * u * u - u) * ui;
+  t.df_de = -24.0 * (2.0 * u * u - u) * ui;  // f_lj / e, also where e = 0
+  const double f_lj = e * t.df_de;
   const double ui2 = ui * ui, ui4 = ui2 * ui2;
   const double fp_lj = 24.0 * e * (14.0 * s6 * s6 * ui4 * ui4 - 4.0 * s6 * ui4 * ui);
   const double r = sqrt(r2);
@@ -58,7 +59,6 @@ __device__ __forceinline__ PairTerms pair_terms(double e, double sg, double qq, 
   t.dh_da = qqr2e * two_b_pi * ex;
   t.f = f_lj + qq * t.h;
   t.fp = fp_lj + qq * dh_dr / (2.0 * r);
-  t.df_de = f_lj / e;
   t.df_ds = -144.0 * e * (4.0 * u * u - u) * ui / sg;
   return t;
 }
@@ -70,7 +70,8 @@ __device__ __forceinline__ PairTerms pair_terms_f32(float e, float sg, float qq,
   const float ui = 1.0f / r2;
   const float s2 = sg * sg, s6 = s2 * s2 * s2;
   const float u = s6 * ui * ui * ui;
-  const float f_lj = -24.0f * e * (2.0f * u * u - u) * ui;
+  const float df_de = -24.0f * (2.0f * u * u - u) * ui;
+  const float f_lj = e * df_de;
   const float ui2 = ui * ui, ui4 = ui2 * ui2;
   const float fp_lj = 24.0f * e * (14.0f * s6 * s6 * ui4 * ui4 - 4.0f * s6 * ui4 * ui);
   const float r = sqrtf(r2);
@@ -85,7 +86,7 @@ __device__ __forceinline__ PairTerms pair_terms_f32(float e, float sg, float qq,
   t.dh_da = qqr2e * two_b_pi * ex;
   t.f = f_lj + qq * h;
   t.fp = fp_lj + qq * dh_dr / (2.0f * r);
-  t.df_de = f_lj / e;
+  t.df_de = df_de;
   t.df_ds = -144.0f * e * (4.0f * u * u - u) * ui / sg;
   return t;
 }
@@ -155,7 +156,8 @@ k_adj_pair(PairParams pp, int n, const uint4* __restrict__ atoms, const double* 
       const double dz = min_image1(z[j] - zm, pp.box.len[2], pp.box.half[2]);
       const double r2 = dx * dx + dy * dy + dz * dz;
       const int tj = type[j];
-      const double e = sqrt(eps_m * eps_t[tj]);
+      const double eps_j = eps_t[tj];
+      const double e = sqrt(eps_m * eps_j);
       const double sg = 0.5 * (sig_m + sigma_t[tj]);
       const double qj = q[j];
       const PairTerms pt =
@@ -171,9 +173,10 @@ k_adj_pair(PairParams pp, int n, const uint4* __restrict__ atoms, const double* 
         rz -= cf * gpz + cd * dz;
         dq += w * pt.h * qj;
         const double we = w * pt.df_de * e, ws = 0.5 * w * pt.df_ds;
-        de_m += we;
+        // sqrt(eps_m eps_j) has no derivative in an eps that is 0
+        de_m += eps_m > 0.0 ? we : NAN;
         ds_m += ws;
-        mine[tj * ADJ_BLOCK] += we;
+        mine[tj * ADJ_BLOCK] += eps_j > 0.0 ? we : NAN;
         mine[(nt + tj) * ADJ_BLOCK] += ws;
         d_alpha += w * qm * qj * pt.dh_da;
       }
@@ -240,7 +243,8 @@ k_adj_pair(PairParams pp, int n, const uint4* __restrict__ atoms, const double* 
   }
   for (int t = 0; t < npar; ++t) {
     double v = warp_sum(t < 2 * nt ? mine[t * ADJ_BLOCK] : d_alpha);
-    // a type without force-carrying pairs sums to 0, also with eps = 0
+    // a type without force-carrying pairs sums to 0, also with eps = 0; with
+    // eps = 0 and pairs the sum is NaN
     if (t < nt && v != 0.0) v /= 2.0 * eps_t[t];
     if (lane == 0) s_part[warp][t] = v;
   }
