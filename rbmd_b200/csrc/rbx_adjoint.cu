@@ -259,8 +259,7 @@ k_adj_pair(PairParams pp, int n, const uint4* __restrict__ atoms, const double* 
 // k-space, pass 1: per-block partial sums of a_k and b_k, part[k][block].
 constexpr int ADJK_BLOCK = 128;
 __global__ void __launch_bounds__(ADJK_BLOCK)
-k_adj_k_ab(int n, int p, int chunk, double sx, double sy, double sz,
-           const KTab* __restrict__ tab, const double* __restrict__ q,
+k_adj_k_ab(int n, int p, int chunk, const KTab* __restrict__ tab, const double* __restrict__ q,
            const double* __restrict__ x, const double* __restrict__ y,
            const double* __restrict__ z, const double* __restrict__ gx,
            const double* __restrict__ gy, const double* __restrict__ gz,
@@ -268,15 +267,13 @@ k_adj_k_ab(int n, int p, int chunk, double sx, double sy, double sz,
   const int k = blockIdx.y * ADJK_BLOCK + threadIdx.x;
   if (k >= p) return;
   const double kx = tab[k].kx, ky = tab[k].ky, kz = tab[k].kz;
-  // phase in quarter turns: 4 m / L per length (sx, sy, sz = 4 / L)
-  const double mx = tab[k].md[0] * sx, my = tab[k].md[1] * sy, mz = tab[k].md[2] * sz;
   const int a0 = blockIdx.x * chunk, a1 = min(n, a0 + chunk);
   double sa = 0.0, sb = 0.0;
   for (int i = a0; i < a1; ++i) {
     double s, c;
     if (q[i] + 0.0 * (x[i] + y[i] + z[i] + gx[i] + gy[i] + gz[i]) == 0.0)
       continue;  // a neutral atom's weight q_i (g_i . k) is zero
-    sincos_quarter(mx * x[i] + my * y[i] + mz * z[i], &s, &c);
+    sincos_phase_any(kx * x[i] + ky * y[i] + kz * z[i], &s, &c);
     const double w = q[i] * (gx[i] * kx + gy[i] * ky + gz[i] * kz);
     sa += w * c;
     sb += w * s;
@@ -288,24 +285,23 @@ k_adj_k_ab(int n, int p, int chunk, double sx, double sy, double sz,
 // k-space, pass 2: per-atom dL/dq and dL/dr, and per-block sums of g . K
 // (for dL/dalpha).  ab[k] = {a_k, b_k} reduced in fixed order beforehand.
 __global__ void __launch_bounds__(ADJK_BLOCK)
-k_adj_k_scatter(int n, int p, double cscale, double sx, double sy, double sz,
-                const KTab* __restrict__ tab, const double* __restrict__ ab,
-                const double* __restrict__ q, const double* __restrict__ x,
-                const double* __restrict__ y, const double* __restrict__ z,
-                const double* __restrict__ gx, const double* __restrict__ gy,
-                const double* __restrict__ gz, double* __restrict__ d_rx,
-                double* __restrict__ d_ry, double* __restrict__ d_rz, double* __restrict__ d_q,
-                double* __restrict__ part_gk) {
+k_adj_k_scatter(int n, int p, double cscale, const KTab* __restrict__ tab,
+                const double* __restrict__ ab, const double* __restrict__ q,
+                const double* __restrict__ x, const double* __restrict__ y,
+                const double* __restrict__ z, const double* __restrict__ gx,
+                const double* __restrict__ gy, const double* __restrict__ gz,
+                double* __restrict__ d_rx, double* __restrict__ d_ry, double* __restrict__ d_rz,
+                double* __restrict__ d_q, double* __restrict__ part_gk) {
   struct K64 {  // per-k constants, formed once a block
-    double mx, my, mz, kx, ky, kz, ta, tb, ca, cb;
+    double kx, ky, kz, ta, tb, ca, cb;
   };
   constexpr int kTile = 128;
   __shared__ K64 s_k[kTile];
   __shared__ double s_sum[ADJK_BLOCK / 32];
   const int i = blockIdx.x * ADJK_BLOCK + threadIdx.x;
   const bool live = i < n;
-  const double ux = live ? x[i] * sx : 0.0, uy = live ? y[i] * sy : 0.0,
-               uz = live ? z[i] * sz : 0.0, qi = live ? q[i] : 0.0;
+  const double xi = live ? x[i] : 0.0, yi = live ? y[i] : 0.0, zi = live ? z[i] : 0.0,
+               qi = live ? q[i] : 0.0;
   const double gix = live ? gx[i] : 0.0, giy = live ? gy[i] : 0.0, giz = live ? gz[i] : 0.0;
   double rx = 0.0, ry = 0.0, rz = 0.0, dq = 0.0, gk_sum = 0.0;
   for (int k0 = 0; k0 < p; k0 += kTile) {
@@ -315,14 +311,14 @@ k_adj_k_scatter(int n, int p, double cscale, double sx, double sy, double sz,
       const KTab& t = tab[k0 + k];
       const double ck = cscale / (t.kx * t.kx + t.ky * t.ky + t.kz * t.kz);
       // t.a = c_k Re rho_k, t.b = c_k Im rho_k, c_k = -4 pi qqr2e S / (P V k^2)
-      s_k[k] = K64{t.md[0], t.md[1], t.md[2], t.kx, t.ky, t.kz, t.a, t.b,
+      s_k[k] = K64{t.kx, t.ky, t.kz, t.a, t.b,
                    ck * ab[2 * (k0 + k)], ck * ab[2 * (k0 + k) + 1]};
     }
     __syncthreads();
     for (int k = 0; k < kn; ++k) {
       const K64 t = s_k[k];
       double s, c;
-      sincos_quarter(t.mx * ux + t.my * uy + t.mz * uz, &s, &c);
+      sincos_phase_any(t.kx * xi + t.ky * yi + t.kz * zi, &s, &c);
       const double gk = gix * t.kx + giy * t.ky + giz * t.kz;
       const double g1 = gk * (c * t.tb - s * t.ta);
       dq += g1 + (t.ca * s - t.cb * c);
@@ -519,7 +515,7 @@ int launch_adj_pair(const PairParams& pp, int n, const uint4* atoms, const doubl
 
 int adj_k_blocks(int n) { return (n + ADJK_BLOCK - 1) / ADJK_BLOCK; }
 
-int launch_adj_kspace(const DBox& b, int n, int p, double cscale, const KTab* tab, const double* q,
+int launch_adj_kspace(int n, int p, double cscale, const KTab* tab, const double* q,
                       const double* x, const double* y, const double* z, const double* gx,
                       const double* gy, const double* gz, double* part_a, double* part_b,
                       int nparts, double* ab, double* d_rx, double* d_ry, double* d_rz,
@@ -528,8 +524,7 @@ int launch_adj_kspace(const DBox& b, int n, int p, double cscale, const KTab* ta
   const int chunk = (n + nparts - 1) / nparts;
   const int nb = (n + chunk - 1) / chunk;
   k_adj_k_ab<<<dim3(nb, (p + ADJK_BLOCK - 1) / ADJK_BLOCK), ADJK_BLOCK, 0, st>>>(
-      n, p, chunk, 4.0 / b.len[0], 4.0 / b.len[1], 4.0 / b.len[2], tab, q, x, y, z, gx, gy, gz,
-      part_a, part_b);
+      n, p, chunk, tab, q, x, y, z, gx, gy, gz, part_a, part_b);
   count_launch();
   int rc = check_launch("adj_k_ab");
   if (rc) return rc;
@@ -537,9 +532,8 @@ int launch_adj_kspace(const DBox& b, int n, int p, double cscale, const KTab* ta
   count_launch();
   rc = check_launch("adj_reduce_k");
   if (rc) return rc;
-  k_adj_k_scatter<<<adj_k_blocks(n), ADJK_BLOCK, 0, st>>>(
-      n, p, cscale, 4.0 / b.len[0], 4.0 / b.len[1], 4.0 / b.len[2], tab, ab, q, x, y, z, gx, gy,
-      gz, d_rx, d_ry, d_rz, d_q, part_gk);
+  k_adj_k_scatter<<<adj_k_blocks(n), ADJK_BLOCK, 0, st>>>(n, p, cscale, tab, ab, q, x, y, z, gx,
+                                                          gy, gz, d_rx, d_ry, d_rz, d_q, part_gk);
   count_launch();
   return check_launch("adj_k_scatter");
 }

@@ -288,7 +288,7 @@ int rbx_rbe_force(const rbx_box* box, int num_atoms, int p_number, double alpha,
     o.f_out_x = fx;
     o.f_out_y = fy;
     o.f_out_z = fz;
-    rc = launch_rbe_force_f64(b, num_atoms, p_number, tab, charge, px, py, pz, o, st);
+    rc = launch_rbe_force_f64(num_atoms, p_number, tab, charge, px, py, pz, o, st);
   }
   cudaFreeAsync(tab, st);
   return rc;
@@ -801,7 +801,7 @@ int rbx_rbsog_force(const rbx_box* box, int level, double cut_off, double qqr2e,
       o.f_out_x = fx;
       o.f_out_y = fy;
       o.f_out_z = fz;
-      rc = launch_rbe_force_f64(b, num_atoms, pt, tab, charge, px, py, pz, o, st);
+      rc = launch_rbe_force_f64(num_atoms, pt, tab, charge, px, py, pz, o, st);
     }
     if (!rc && energy) {
       cudaMemcpyAsync(energy, en, sizeof(double), cudaMemcpyDeviceToHost, st);

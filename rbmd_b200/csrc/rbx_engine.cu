@@ -567,7 +567,7 @@ int rbx_engine::kspace_finish(bool kick, const int* epoch_dev) {
   if (mixed)
     ETRY(launch_rbe_force_mixed(n, Pk, tab, atoms, o, st, tun.frc_block));
   else
-    ETRY(launch_rbe_force_f64(dbox, n, Pk, tab, q, x, y, z, o, st, tun.frc_block));
+    ETRY(launch_rbe_force_f64(n, Pk, tab, q, x, y, z, o, st, tun.frc_block));
   return RBX_OK;
 }
 
@@ -692,7 +692,7 @@ int rbx_engine::autotune(bool force, rbx_tuning* out) {
         rc = time_it(
             [&]() {
               return mixed ? launch_rbe_force_mixed(n, Pk, tab, atoms, o, st, blk)
-                           : launch_rbe_force_f64(dbox, n, Pk, tab, q, x, y, z, o, st, blk);
+                           : launch_rbe_force_f64(n, Pk, tab, q, x, y, z, o, st, blk);
             },
             &ms);
         c.push_back({blk, 0, ms});
@@ -1525,7 +1525,7 @@ int rbx_engine::force_vjp(const double* g, double* d_eps, double* d_sigma, doubl
       ETRY(launch_adj_kspace_mixed(n, P, cscale, tab, atoms, gx, gy, gz, part_re, part_im,
                                    nparts, kterm, rx, ry, rz, dq, kpart, st));
     else
-      ETRY(launch_adj_kspace(dbox, n, P, cscale, tab, q, x, y, z, gx, gy, gz, part_re, part_im, nparts,
+      ETRY(launch_adj_kspace(n, P, cscale, tab, q, x, y, z, gx, gy, gz, part_re, part_im, nparts,
                              kterm, rx, ry, rz, dq, kpart, st));
   }
   std::vector<double> hp((size_t)nb_pair * npar), hk(P > 0 ? nb_k : 0);

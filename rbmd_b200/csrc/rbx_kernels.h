@@ -14,7 +14,6 @@ struct KTab {
   double kx, ky, kz;
   double a, b;  // coef * Re rho, coef * Im rho, coef = -4 pi qqr2e S / (P V k^2)
   int m[4];     // integer m (mixed form)
-  double md[3]; // m as given (FP64 form)
 };
 
 // Energy and virial from the per-k terms of a finalize: one warp adds them in
@@ -90,9 +89,9 @@ int launch_rbe_finalize(const DBox& b, int p, int nparts, const double* part_re,
 // sums their terms.
 // job: the sum over k is not launched here but described for the force pass.
 int launch_energy_sum(const EnergyJob& job, cudaStream_t st);
-int launch_rbe_force_f64(const DBox& b, int n, int p, const KTab* tab, const double* q,
-                         const double* x, const double* y, const double* z,
-                         const RbeForceOut& out, cudaStream_t st, int block = 256);
+int launch_rbe_force_f64(int n, int p, const KTab* tab, const double* q, const double* x,
+                         const double* y, const double* z, const RbeForceOut& out,
+                         cudaStream_t st, int block = 256);
 int launch_rbe_force_mixed(int n, int p, const KTab* tab, const uint4* atoms,
                            const RbeForceOut& out, cudaStream_t st, int block = 256);
 // step_dev (may be null): read the step from device memory (step graphs).
@@ -285,7 +284,7 @@ int launch_adj_pair(const PairParams& pp, int n, const uint4* atoms, const doubl
 // k-space part, added to d_r and d_q; part_gk[adj_k_blocks(n)] = block sums of g . K.
 // cscale = -4 pi qqr2e S / (P V); ab: 2p scratch; part_a/b: p * nparts scratch.
 int adj_k_blocks(int n);
-int launch_adj_kspace(const DBox& b, int n, int p, double cscale, const KTab* tab, const double* q,
+int launch_adj_kspace(int n, int p, double cscale, const KTab* tab, const double* q,
                       const double* x, const double* y, const double* z, const double* gx,
                       const double* gy, const double* gz, double* part_a, double* part_b,
                       int nparts, double* ab, double* d_rx, double* d_ry, double* d_rz,

@@ -4,41 +4,59 @@
 
 namespace rbx {
 
-// sin and cos of t quarter turns (angle t pi / 2): t minus its nearest integer
-// is exact for |t| < 2^51, and two polynomials in r^2 on |r| <= 1/2 follow, the
-// interpolants of sin(pi r / 2) / r and (cos(pi r / 2) - 1) / r^2 at the seven
-// Chebyshev nodes of r^2 in [0, 1/4], computed in 60-digit arithmetic
-// (truncation 3.5e-18 and 1.2e-19; evaluated in FP64 2.2e-16 at most, relative).
-// About 21 FP64 instructions; sincos of the phase in radians takes about 85
-// (its reduction by pi covers any argument), and FP64 issue bounds both passes:
-// with the neutral atoms left out, 46 -> 11 us for the structure factor and
-// 38 -> 10 us for the force of 100,003 atoms (10 % charged) x 100 vectors.
-__device__ __forceinline__ void sincos_quarter(double t, double* s, double* c) {
-  const double kShift = 6755399441055744.0;  // 1.5 * 2^52
-  const double b = __dadd_rn(t, kShift);
+// Largest phase that sincos_phase takes.  A pass checks its atoms and k-vectors
+// against it before its loops (a check a phase costs the structure factor a third)
+// and leaves what lies beyond, NaN and infinities to the library's sincos.
+constexpr double PHASE_MAX = 35184372088832.0;  // 2^45
+
+// |k.r| is at most norm1(k) times norm1(r).
+__device__ __forceinline__ double norm1(double x, double y, double z) {
+  return fabs(x) + fabs(y) + fabs(z);
+}
+
+// sin and cos of t radians, |t| <= PHASE_MAX.  t less its nearest multiple n of pi/2, pi/2 in two
+// FP64 parts (Cody and Waite): n times the first part is exact in the fused
+// multiply-add and cancels against t without rounding, so the remainder r is
+// rounded once.  Then polynomials in r^2 on |r| <= pi/4: the interpolants of
+// (sin(r) / r - 1) / r^2 and (cos(r) - 1) / r^2 at the six and seven Chebyshev
+// nodes of r^2 in [0, pi^2/16], computed in 60-digit arithmetic (truncation
+// 1.3e-17 and 1.2e-19 relative).  Some 20 FP64 instructions, where the library's sincos takes about 85, and FP64
+// issue bounds the passes that call it.
+__device__ __forceinline__ void sincos_phase(double t, double* s, double* c) {
+  const double kShift = 6755399441055744.0;                 // 1.5 * 2^52
+  const double b = fma(t, 0.6366197723675814, kShift);      // 2 / pi
   const int n = __double2loint(b);  // nearest integer, modulo 2^32
-  const double r = __dsub_rn(t, __dsub_rn(b, kShift));
+  const double m = __dsub_rn(b, kShift);
+  double r = fma(m, -1.5707963267948966, t);
+  r = fma(m, -6.123233995736766e-17, r);
   const double z = r * r;
-  double p = 5.633933781537854e-08;
-  p = fma(p, z, -3.59864335298231e-06);
-  p = fma(p, z, 0.0001604411507421909);
-  p = fma(p, z, -0.004681754132340976);
-  p = fma(p, z, 0.07969262624604301);
-  p = fma(p, z, -0.6459640975062443);
-  p = fma(p, z, 1.5707963267948966);
-  p *= r;
-  double q = -6.329396344967424e-09;
-  q = fma(q, z, 4.710678405505227e-07);
-  q = fma(q, z, -2.5202039028029178e-05);
-  q = fma(q, z, 0.0009192602745468447);
-  q = fma(q, z, -0.020863480763340773);
-  q = fma(q, z, 0.2536695079010478);
-  q = fma(q, z, -1.2337005501361697);
+  double p = 1.5918129294866608e-10;
+  p = fma(p, z, -2.5051131845003624e-08);
+  p = fma(p, z, 2.755731610255244e-06);
+  p = fma(p, z, -0.00019841269836758574);
+  p = fma(p, z, 0.008333333333330948);
+  p = fma(p, z, -0.16666666666666666);
+  p = fma(r * z, p, r);
+  double q = -1.1367998654022494e-11;
+  q = fma(q, z, 2.0875886738047052e-09);
+  q = fma(q, z, -2.7557315566341895e-07);
+  q = fma(q, z, 2.480158729369346e-05);
+  q = fma(q, z, -0.0013888888888880775);
+  q = fma(q, z, 0.04166666666666664);
+  q = fma(q, z, -0.5);
   q = fma(q, z, 1.0);
   const bool odd = n & 1;
   const double ss = odd ? q : p, cc = odd ? p : q;
   *s = __hiloint2double(__double2hiint(ss) ^ ((n << 30) & 0x80000000), __double2loint(ss));
   *c = __hiloint2double(__double2hiint(cc) ^ (((n + 1) << 30) & 0x80000000), __double2loint(cc));
+}
+
+// The same for any phase, checked here.
+__device__ __forceinline__ void sincos_phase_any(double t, double* s, double* c) {
+  if (fabs(t) <= PHASE_MAX)
+    sincos_phase(t, s, c);
+  else
+    sincos(t, s, c);
 }
 
 }  // namespace rbx

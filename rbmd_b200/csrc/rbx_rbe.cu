@@ -11,8 +11,7 @@
 // both passes evaluate phases for the charged atoms only (10 % of an LJ
 // electrolyte's atoms, all of a water's).
 //
-// Plain form: FP64 positions; the phase m.r/L is formed in quarter turns and
-// reduced to [-1/2, 1/2] exactly before FP64 polynomials.
+// Plain form: FP64 positions and phases k.r, FP64 sine and cosine.
 // Mixed form: 32-bit fixed-point fractional coordinates u = frac((x-lo)/L)*2^32
 // so the phase m.u mod 2^32 is exact integer arithmetic; the angle goes to the
 // SFU (__sincosf) in FP32; per-thread FP32 partial sums are folded with a
@@ -29,6 +28,12 @@ namespace rbx {
 // that is not finite (which then shows in the sums).
 __device__ __forceinline__ bool kspace_atom(double q, double x, double y, double z) {
   return q + 0.0 * (x + y + z) != 0.0;
+}
+
+// The largest double with this high word: a bound of nonnegative doubles by the
+// integer maximum of their high words (NaN and infinity come out as NaN).
+__device__ __forceinline__ double bound_of_hi(unsigned hi) {
+  return __hiloint2double((int)hi, -1);
 }
 
 // ---------------------------------------------------------------------------
@@ -120,7 +125,7 @@ __device__ __forceinline__ void rbe_group_samples(const SampleArgs& sa, int p, i
 
 template <int KPT>
 __global__ void __launch_bounds__(RBE_BLOCK)
-k_rbe_rho_partial_f64(int n, int p, int chunk, double kxs, double kys, double kzs,
+k_rbe_rho_partial_f64(int n, int p, int chunk, double Lx, double Ly, double Lz,
                       const double* __restrict__ mx, const double* __restrict__ my,
                       const double* __restrict__ mz, const double* __restrict__ q,
                       const double* __restrict__ x, const double* __restrict__ y,
@@ -129,53 +134,69 @@ k_rbe_rho_partial_f64(int n, int p, int chunk, double kxs, double kys, double kz
   __shared__ double s_re[RBE_WARPS][(32 * KPT)];
   __shared__ double s_im[RBE_WARPS][(32 * KPT)];
   __shared__ int s_m[3][32 * KPT];
+  __shared__ double s_k[3][32 * KPT];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kbase = blockIdx.y * (32 * KPT);
   if (sa.tables) rbe_group_samples<KPT>(sa, p, kbase, s_m, blockIdx.x == 0);
-  double kx[KPT], ky[KPT], kz[KPT], sr[KPT], si[KPT];  // integer m as doubles
+  // the block's k-vectors, k = 2 pi m / L evaluated as (2 pi * m) / L like the
+  // reference: a division a thread or two, where each warp's own took a fifth of
+  // the kernel at 400 vectors
+  for (int t = threadIdx.x; t < 96 * KPT; t += RBE_BLOCK) {
+    const int d = t / (32 * KPT), s = t % (32 * KPT);
+    const double* const m = d == 0 ? mx : (d == 1 ? my : mz);
+    const double md = sa.tables ? (double)s_m[d][s] : (kbase + s < p ? m[kbase + s] : 0.0);
+    s_k[d][s] = (2 * RBX_PI * md) / (d == 0 ? Lx : (d == 1 ? Ly : Lz));
+  }
+  __syncthreads();
+  double kx[KPT], ky[KPT], kz[KPT], sr[KPT], si[KPT];
+  unsigned kmax_hi = 0;
 #pragma unroll
   for (int t = 0; t < KPT; ++t) {
-    const int k = kbase + lane + 32 * t;
-    const bool ok = k < p;
-    kx[t] = sa.tables ? (double)s_m[0][lane + 32 * t] : (ok ? mx[k] : 0.0);
-    ky[t] = sa.tables ? (double)s_m[1][lane + 32 * t] : (ok ? my[k] : 0.0);
-    kz[t] = sa.tables ? (double)s_m[2][lane + 32 * t] : (ok ? mz[k] : 0.0);
+    kx[t] = s_k[0][lane + 32 * t];
+    ky[t] = s_k[1][lane + 32 * t];
+    kz[t] = s_k[2][lane + 32 * t];
+    kmax_hi = max(kmax_hi, (unsigned)__double2hiint(norm1(kx[t], ky[t], kz[t])));
     sr[t] = 0.0;
     si[t] = 0.0;
   }
+  const double kmax = bound_of_hi(__reduce_max_sync(0xffffffffu, kmax_hi));
   const int a0 = blockIdx.x * chunk;
   const int a1 = min(n, a0 + chunk);
   const int sub = (chunk + RBE_WARPS - 1) / RBE_WARPS;
   const int w0 = a0 + warp * sub, w1 = min(a1, w0 + sub);
   // 32 atoms at a time, one a lane; the charged ones are then broadcast in
-  // atom order, positions in quarter turns of the box (4 x / L)
+  // atom order
   for (int jt = w0; jt < w1; jt += 32) {
     const int j = jt + lane;
-    double ux = 0.0, uy = 0.0, uz = 0.0, qj = 0.0;
+    double xl = 0.0, yl = 0.0, zl = 0.0, ql = 0.0;
     if (j < w1) {
-      ux = x[j];
-      uy = y[j];
-      uz = z[j];
-      qj = q[j];
+      xl = x[j];
+      yl = y[j];
+      zl = z[j];
+      ql = q[j];
     }
-    unsigned m = __ballot_sync(0xffffffffu, kspace_atom(qj, ux, uy, uz));
+    unsigned m = __ballot_sync(0xffffffffu, kspace_atom(ql, xl, yl, zl));
     if (m == 0) continue;
-    ux = 4.0 * (ux / kxs);
-    uy = 4.0 * (uy / kys);
-    uz = 4.0 * (uz / kzs);
-    do {
-      const int src = __ffs(m) - 1;
-      m &= m - 1;
-      const double xj = __shfl_sync(0xffffffffu, ux, src), yj = __shfl_sync(0xffffffffu, uy, src),
-                   zj = __shfl_sync(0xffffffffu, uz, src), cj = __shfl_sync(0xffffffffu, qj, src);
+    const bool small =
+        __all_sync(0xffffffffu, norm1(xl, yl, zl) * kmax <= PHASE_MAX);
+    auto add = [&](auto phase) {
+      for (unsigned left = m; left; left &= left - 1) {
+        const int src = __ffs(left) - 1;
+        const double xj = __shfl_sync(0xffffffffu, xl, src), yj = __shfl_sync(0xffffffffu, yl, src),
+                     zj = __shfl_sync(0xffffffffu, zl, src), qj = __shfl_sync(0xffffffffu, ql, src);
 #pragma unroll
-      for (int t = 0; t < KPT; ++t) {
-        double s, c;
-        sincos_quarter(kx[t] * xj + ky[t] * yj + kz[t] * zj, &s, &c);
-        sr[t] += cj * c;
-        si[t] += cj * s;
+        for (int t = 0; t < KPT; ++t) {
+          double s, c;
+          phase(kx[t] * xj + ky[t] * yj + kz[t] * zj, &s, &c);
+          sr[t] += qj * c;
+          si[t] += qj * s;
+        }
       }
-    } while (m);
+    };
+    if (small)
+      add([](double t, double* s, double* c) { sincos_phase(t, s, c); });
+    else
+      add([](double t, double* s, double* c) { sincos(t, s, c); });
   }
 #pragma unroll
   for (int t = 0; t < KPT; ++t) {
@@ -575,9 +596,6 @@ __device__ void rbe_finalize_one(int k, int p, int nparts, const double* __restr
     t.m[1] = (int)my[k];
     t.m[2] = (int)mz[k];
     t.m[3] = 0;
-    t.md[0] = mx[k];
-    t.md[1] = my[k];
-    t.md[2] = mz[k];
     tab[k] = t;
   }
 }
@@ -672,63 +690,76 @@ __device__ __forceinline__ int threads_per_atom(int count) {
   return s;
 }
 
-// FP64 table entry in shared memory: integer m as doubles, coef Re / Im rho.
+// FP64 table entry in shared memory: k, coef Re / Im rho.
 struct KTabD {
-  double mx, my, mz, a, b;
+  double kx, ky, kz, a, b;
 };
 
 template <int FB>
 __global__ void __launch_bounds__(FB)
-k_rbe_force_f64(int n, int p, double Lx, double Ly, double Lz, const KTab* __restrict__ tab,
-                const double* __restrict__ q, const double* __restrict__ x,
-                const double* __restrict__ y, const double* __restrict__ z, ForceEpilogue ep) {
+k_rbe_force_f64(int n, int p, const KTab* __restrict__ tab, const double* __restrict__ q,
+                const double* __restrict__ x, const double* __restrict__ y,
+                const double* __restrict__ z, ForceEpilogue ep) {
   if (ep.job.kind != EnergyJob::NONE && blockIdx.x == gridDim.x - 1) {
     if (threadIdx.x < 32) energy_job(ep.job);
     return;
   }
   __shared__ KTabD s_tab[FRC_TABLE];
-  __shared__ double s_x[FB], s_y[FB], s_z[FB];  // positions in quarter turns, then forces
+  __shared__ double s_x[FB], s_y[FB], s_z[FB];  // positions, then forces
   __shared__ unsigned short s_list[FB];
   __shared__ int s_cnt[FB / 32];
+  __shared__ unsigned s_far[FB / 32];  // the warps' farthest charged atoms
   const int i = blockIdx.x * FB + threadIdx.x;
   const bool live = i < n;
   const double xi = live ? x[i] : 0.0, yi = live ? y[i] : 0.0, zi = live ? z[i] : 0.0;
   const double qi = live ? q[i] : 0.0;
   const bool take = live && kspace_atom(qi, xi, yi, zi);
   if (take) {
-    s_x[threadIdx.x] = 4.0 * (xi / Lx);
-    s_y[threadIdx.x] = 4.0 * (yi / Ly);
-    s_z[threadIdx.x] = 4.0 * (zi / Lz);
+    s_x[threadIdx.x] = xi;
+    s_y[threadIdx.x] = yi;
+    s_z[threadIdx.x] = zi;
   }
   const int count = block_compact<FB>(take, s_list, s_cnt);
+  const unsigned far_hi = __reduce_max_sync(
+      0xffffffffu, take ? (unsigned)__double2hiint(norm1(xi, yi, zi)) : 0u);
+  if ((threadIdx.x & 31) == 0) s_far[threadIdx.x >> 5] = far_hi;
   const int share = threads_per_atom<FB>(count);
   const int slot = (int)threadIdx.x / share, part = (int)threadIdx.x % share;
   const bool mine = slot < count;
   const int own = mine ? s_list[slot] : 0;
-  const double ux = s_x[own], uy = s_y[own], uz = s_z[own];
+  const double xo = s_x[own], yo = s_y[own], zo = s_z[own];
   double fx = 0, fy = 0, fz = 0;
   for (int k0 = 0; k0 < p && count > 0; k0 += FRC_TABLE) {
     const int kn = min(FRC_TABLE, p - k0);
     __syncthreads();
+    unsigned rmax_hi = 0;
+    for (int w = 0; w < FB / 32; ++w) rmax_hi = max(rmax_hi, s_far[w]);
+    const double rmax = bound_of_hi(rmax_hi);
+    bool large = false;
     for (int s = threadIdx.x; s < kn; s += FB) {
       const KTab& t = tab[k0 + s];
-      s_tab[s] = KTabD{t.md[0], t.md[1], t.md[2], t.a, t.b};
+      s_tab[s] = KTabD{t.kx, t.ky, t.kz, t.a, t.b};
+      large |= !(norm1(t.kx, t.ky, t.kz) * rmax <= PHASE_MAX);
     }
-    __syncthreads();
-    if (mine) {
-      auto add = [&](int s) {
-        const KTabD t = s_tab[s];
-        double sn, cs;
-        sincos_quarter(t.mx * ux + t.my * uy + t.mz * uz, &sn, &cs);
-        const double f = cs * t.b - sn * t.a;
-        fx += f * t.mx;
-        fy += f * t.my;
-        fz += f * t.mz;
-      };
+    large = __syncthreads_or(large);
+    auto add = [&](int s, auto phase) {
+      const KTabD t = s_tab[s];
+      double sn, cs;
+      phase(t.kx * xo + t.ky * yo + t.kz * zo, &sn, &cs);
+      const double f = cs * t.b - sn * t.a;
+      fx += f * t.kx;
+      fy += f * t.ky;
+      fz += f * t.kz;
+    };
+    auto phase = [](double t, double* s, double* c) { sincos_phase(t, s, c); };
+    if (mine && !large) {
       if (share == 1)
-        for (int s = 0; s < kn; ++s) add(s);
+        for (int s = 0; s < kn; ++s) add(s, phase);
       else
-        for (int s = part; s < kn; s += share) add(s);
+        for (int s = part; s < kn; s += share) add(s, phase);
+    } else if (mine) {
+      for (int s = part; s < kn; s += share)
+        add(s, [](double t, double* s, double* c) { sincos(t, s, c); });
     }
   }
   for (int o = share >> 1; o > 0; o >>= 1) {  // a share never crosses a warp
@@ -737,10 +768,10 @@ k_rbe_force_f64(int n, int p, double Lx, double Ly, double Lz, const KTab* __res
     fz += __shfl_xor_sync(0xffffffffu, fz, o);
   }
   __syncthreads();  // every position has been read
-  if (mine && part == 0) {  // k = 2 pi m / L
-    s_x[own] = fx * (2 * RBX_PI / Lx);
-    s_y[own] = fy * (2 * RBX_PI / Ly);
-    s_z[own] = fz * (2 * RBX_PI / Lz);
+  if (mine && part == 0) {
+    s_x[own] = fx;
+    s_y[own] = fy;
+    s_z[own] = fz;
   }
   __syncthreads();
   if (live)
@@ -939,7 +970,8 @@ k_ewald_rho(int n, int nk, int kx_max, int ky_max, int kz_max, double Lx, double
   // k index -> (i, j, l) in ExecuteOnKmax order, skipping the origin.
   const int ny = 2 * ky_max + 1, nz = 2 * kz_max + 1;
   const int center = kx_max * ny * nz + ky_max * nz + kz_max;
-  double m0[EW_KPT], m1[EW_KPT], m2[EW_KPT], sr[EW_KPT], si[EW_KPT];
+  int m0[EW_KPT], m1[EW_KPT], m2[EW_KPT];
+  double kx[EW_KPT], ky[EW_KPT], kz[EW_KPT], sr[EW_KPT], si[EW_KPT], kmax = 0.0;
 #pragma unroll
   for (int t = 0; t < EW_KPT; ++t) {
     const int k = min(k0 + t, nk - 1);
@@ -947,7 +979,11 @@ k_ewald_rho(int n, int nk, int kx_max, int ky_max, int kz_max, double Lx, double
     m0[t] = flat / (ny * nz) - kx_max;
     m1[t] = (flat / nz) % ny - ky_max;
     m2[t] = flat % nz - kz_max;
+    kx[t] = 2 * RBX_PI * m0[t] / Lx;
+    ky[t] = 2 * RBX_PI * m1[t] / Ly;
+    kz[t] = 2 * RBX_PI * m2[t] / Lz;
     sr[t] = si[t] = 0.0;
+    kmax = fmax(kmax, norm1(kx[t], ky[t], kz[t]));
   }
   for (int base = 0; base < n; base += EW_BLOCK) {
     const int j = base + threadIdx.x;
@@ -957,22 +993,28 @@ k_ewald_rho(int n, int nk, int kx_max, int ky_max, int kz_max, double Lx, double
     const bool take = live && kspace_atom(qj, xj, yj, zj);
     __syncthreads();  // the previous tile has been read
     if (take) {
-      s_x[threadIdx.x] = 4.0 * (xj / Lx);
-      s_y[threadIdx.x] = 4.0 * (yj / Ly);
-      s_z[threadIdx.x] = 4.0 * (zj / Lz);
+      s_x[threadIdx.x] = xj;
+      s_y[threadIdx.x] = yj;
+      s_z[threadIdx.x] = zj;
       s_q[threadIdx.x] = qj;
     }
     const int count = block_compact<EW_BLOCK>(take, s_list, s_cnt);
     for (int a = lane; a < count; a += 32) {
       const int o = s_list[a];
-      const double ux = s_x[o], uy = s_y[o], uz = s_z[o], c = s_q[o];
+      const double xo = s_x[o], yo = s_y[o], zo = s_z[o], c = s_q[o];
+      auto add = [&](auto phase) {
 #pragma unroll
-      for (int t = 0; t < EW_KPT; ++t) {
-        double sn, cs;
-        sincos_quarter(m0[t] * ux + m1[t] * uy + m2[t] * uz, &sn, &cs);
-        sr[t] += c * cs;
-        si[t] += c * sn;
-      }
+        for (int t = 0; t < EW_KPT; ++t) {
+          double sn, cs;
+          phase(kx[t] * xo + ky[t] * yo + kz[t] * zo, &sn, &cs);
+          sr[t] += c * cs;
+          si[t] += c * sn;
+        }
+      };
+      if (norm1(xo, yo, zo) * kmax <= PHASE_MAX)
+        add([](double t, double* s, double* c) { sincos_phase(t, s, c); });
+      else
+        add([](double t, double* s, double* c) { sincos(t, s, c); });
     }
   }
 #pragma unroll
@@ -984,29 +1026,24 @@ k_ewald_rho(int n, int nk, int kx_max, int ky_max, int kz_max, double Lx, double
     }
     const int k = k0 + t;
     if (lane == 0 && k < nk) {
-      const double kx = 2 * RBX_PI * m0[t] / Lx, ky = 2 * RBX_PI * m1[t] / Ly,
-                   kz = 2 * RBX_PI * m2[t] / Lz;
       re[k] = sr[t];
       im[k] = si[t];
-      kvec[3 * k] = kx;
-      kvec[3 * k + 1] = ky;
-      kvec[3 * k + 2] = kz;
+      kvec[3 * k] = kx[t];
+      kvec[3 * k + 1] = ky[t];
+      kvec[3 * k + 2] = kz[t];
       if (tab) {
-        const double k2 = kx * kx + ky * ky + kz * kz;
+        const double k2 = kx[t] * kx[t] + ky[t] * ky[t] + kz[t] * kz[t];
         const double f = coef / k2 * exp(-0.25 * k2 / alpha);
         KTab e;
-        e.kx = kx;
-        e.ky = ky;
-        e.kz = kz;
+        e.kx = kx[t];
+        e.ky = ky[t];
+        e.kz = kz[t];
         e.a = f * sr[t];
         e.b = f * si[t];
-        e.m[0] = (int)m0[t];
-        e.m[1] = (int)m1[t];
-        e.m[2] = (int)m2[t];
+        e.m[0] = m0[t];
+        e.m[1] = m1[t];
+        e.m[2] = m2[t];
         e.m[3] = 0;
-        e.md[0] = m0[t];
-        e.md[1] = m1[t];
-        e.md[2] = m2[t];
         tab[k] = e;
       }
     }
@@ -1189,17 +1226,16 @@ static ForceEpilogue make_ep(const RbeForceOut& o) {
 }
 
 // block: atoms per block (128, 256 or 512); the forces do not depend on it.
-int launch_rbe_force_f64(const DBox& b, int n, int p, const KTab* tab, const double* q,
-                         const double* x, const double* y, const double* z,
-                         const RbeForceOut& out, cudaStream_t st, int block) {
+int launch_rbe_force_f64(int n, int p, const KTab* tab, const double* q, const double* x,
+                         const double* y, const double* z, const RbeForceOut& out,
+                         cudaStream_t st, int block) {
   const int extra = out.job.kind != EnergyJob::NONE;  // the energy's block
   if (n <= 0) return extra ? launch_energy_sum(out.job, st) : RBX_OK;
   const ForceEpilogue ep = make_ep(out);
   if (block != 128 && block != 512) block = 256;
   const auto kern = block == 128 ? k_rbe_force_f64<128>
                                  : (block == 512 ? k_rbe_force_f64<512> : k_rbe_force_f64<256>);
-  kern<<<(n + block - 1) / block + extra, block, 0, st>>>(n, p, b.len[0], b.len[1], b.len[2], tab,
-                                                          q, x, y, z, ep);
+  kern<<<(n + block - 1) / block + extra, block, 0, st>>>(n, p, tab, q, x, y, z, ep);
   count_launch();
   return check_launch("rbe_force_f64");
 }
@@ -1320,7 +1356,7 @@ int launch_ewald(const DBox& b, int n, const int kmax[3], double alpha, double q
     o.f_out_x = fx;
     o.f_out_y = fy;
     o.f_out_z = fz;
-    rc = launch_rbe_force_f64(b, n, nk, tab, q, x, y, z, o, st, 256);
+    rc = launch_rbe_force_f64(n, nk, tab, q, x, y, z, o, st, 256);
     if (rc) return rc;
   }
   if (energy) {

@@ -220,9 +220,6 @@ k_rbsog_finalize(int p, int nparts, const double* __restrict__ part_re,
     t.m[1] = (int)my[k];
     t.m[2] = (int)mz[k];
     t.m[3] = 0;
-    t.md[0] = mx[k];
-    t.md[1] = my[k];
-    t.md[2] = mz[k];
     tab[k] = t;
   }
 }

@@ -90,6 +90,65 @@ def test_kspace_fractional_k_and_far_positions(cuda, rbx):
     _close(np.stack([a.cpu().numpy() for a in F], 1), f, 1e-10)
 
 
+def test_kspace_rounding(cuda, rbx):
+    """Rounding of the FP64 functors beyond that of the phase k.r itself, which
+    both sides form alike (k = 2 pi m / L, then fused multiply-adds): sine and
+    cosine within an ulp and the sums' order, a few 2^-53 of the norm.  The
+    reference takes the sines and sums in 80 bits.  (A phase from m and r / L,
+    rounded otherwise, is 2.8e-15 away at this size.)"""
+    rng = np.random.default_rng(4)
+    n, p, L, S = 40000, 100, 36.84, 50.0
+    pos, q = rng.uniform(0, L, (n, 3)), np.where(np.arange(n) % 4, 0.0, rng.choice([-1.0, 1.0], n))
+    m = rng.integers(-9, 10, (3, p)).astype(float)
+    m[0, (m == 0).all(0)] = 1.0
+    ld = np.longdouble
+    fma = lambda a, b, c: (ld(a) * ld(b) + ld(c)).astype(np.float64)  # noqa: E731
+    k = 2 * np.pi * m / L
+    c = -4 * np.pi * S / (p * L ** 3 * (k * k).sum(0))
+    w = np.nonzero(q)[0]
+    re, im, f = np.zeros(p), np.zeros(p), np.zeros((n, 3), dtype=ld)
+    for a in range(p):
+        ph = fma(k[2, a], pos[w, 2], fma(k[0, a], pos[w, 0], k[1, a] * pos[w, 1])).astype(ld)
+        cs, sn = np.cos(ph), np.sin(ph)
+        re[a], im[a] = (q[w] * cs).sum(), (q[w] * sn).sum()
+        f[w] += (c[a] * (cs * im[a] - sn * re[a]) * q[w])[:, None] * k[:, a]
+    dev = lambda a: cuda.as_tensor(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    box = rbx.Box.make([0] * 3, [L] * 3)
+    T = [dev(q), *(dev(v) for v in m), *(dev(pos[:, d]) for d in range(3))]
+    rho, F = [dev(np.zeros(p)) for _ in range(2)], [dev(np.zeros(n)) for _ in range(3)]
+    rbx.rbe_structure_factor(box, *T, *rho)
+    rbx.rbe_force(box, 0.16, S, 1.0, dev(re), dev(im), *T, *F)
+    cuda.cuda.synchronize()
+    err = lambda a, b: float(np.sqrt(((a - b) ** 2).sum() / (b ** 2).sum()))  # noqa: E731
+    assert err(np.stack([v.cpu().numpy() for v in rho]), np.stack([re, im])) < 8e-16
+    assert err(np.stack([v.cpu().numpy() for v in F], 1), f) < 8e-16
+
+
+def test_kspace_any_phase(cuda, rbx):
+    """Phases of 2^45 radians and far more still have a sine (positions are
+    taken as they come)."""
+    lo, hi, _, _, _ = _system(2, 1, 1.0, 0)
+    L, mx = hi - lo, 3.0
+    x = np.array([0.3, 1e13, -3e14, 7e15, 1e18, -1e30, 5e300])
+    k = 2 * np.pi * mx / L[0]
+    n, zero = len(x), np.zeros(len(x))
+    dev = lambda a: cuda.as_tensor(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    m = [dev(np.array([v])) for v in (mx, 0.0, 0.0)]
+    box = rbx.Box.make(lo, hi)
+    for i in range(n):
+        rho = [dev(np.zeros(1)) for _ in range(2)]
+        rbx.rbe_structure_factor(box, dev(np.ones(1)), *m, dev(x[i:i + 1]), dev(zero[:1]),
+                                 dev(zero[:1]), *rho)
+        assert abs(rho[0].item() - np.cos(k * x[i])) < 4e-16
+        assert abs(rho[1].item() - np.sin(k * x[i])) < 4e-16
+    F = [dev(zero) for _ in range(3)]
+    rbx.rbe_force(box, 0.16, 1.0, 1.0, dev(np.array([2.0])), dev(np.array([-1.0])),
+                  dev(np.ones(n)), *m, dev(x), dev(zero), dev(zero), *F)
+    c = -4 * np.pi / (np.prod(L) * k * k)
+    want = c * (-np.cos(k * x) - 2.0 * np.sin(k * x)) * k
+    assert np.abs(F[0].cpu().numpy() - want).max() < 1e-15 * abs(c * k) * 3
+
+
 @pytest.mark.parametrize("n,kmax,share", [(300, (1, 1, 1), 1.0), (2000, (3, 2, 1), 0.1),
                                           (70, (0, 4, 2), 0.0)])
 def test_ewald_blocks(cuda, rbx, oracle, n, kmax, share):
