@@ -18,6 +18,8 @@
 // TwoSum-compensated pair; the cross-block reduction, energy and virial are FP64.
 #include <math.h>
 
+#include <type_traits>
+
 #include "rbx_common.cuh"
 #include "rbx_kernels.h"
 #include "rbx_phase.cuh"
@@ -603,9 +605,13 @@ __device__ void rbe_finalize_one(int k, int p, int nparts, const double* __restr
 // ---------------------------------------------------------------------------
 // Force scatter over the charged atoms of a block, compacted onto its first
 // threads.  FP64: where few are charged, the idle threads share the atoms'
-// k-vectors (partial sums meet in shuffles).  Mixed: one thread an atom, k in
-// increasing order, since FP32 sums in another order move a force by 1e-7.  The
-// k table is staged in shared memory.
+// k-vectors.  An atom's k-vectors fall into eight classes (k modulo 8), each
+// summed in increasing k, and the eight sums meet in one tree, in a thread's
+// registers or in shuffles: the force is the same to the bit however many
+// threads share it, so it depends neither on the block size nor on the charges
+// around the atom.  Mixed: one thread an atom, k in increasing order, since FP32
+// sums in another order move a force by 1e-7.  The k table is staged in shared
+// memory.
 // Epilogue variants: plain store of F_k, or the fused combine
 // F = F_pair - mean + F_k with the second velocity-Verlet half kick.
 // ---------------------------------------------------------------------------
@@ -681,12 +687,12 @@ __device__ __forceinline__ int block_compact(bool take, unsigned short* s_list, 
 }
 
 // Threads that share one charged atom's k-vectors: the largest power of two
-// (at most a warp) that the block has threads for.  With most of the block
-// charged that is one thread an atom, k in increasing order.
+// (at most the number of classes) that the block has threads for.
+constexpr int K_CLASSES = 8;
 template <int FB>
 __device__ __forceinline__ int threads_per_atom(int count) {
   int s = 1;
-  while (s < 32 && 2 * s * count <= FB) s *= 2;
+  while (s < K_CLASSES && 2 * s * count <= FB) s *= 2;
   return s;
 }
 
@@ -728,41 +734,74 @@ k_rbe_force_f64(int n, int p, const KTab* __restrict__ tab, const double* __rest
   const bool mine = slot < count;
   const int own = mine ? s_list[slot] : 0;
   const double xo = s_x[own], yo = s_y[own], zo = s_z[own];
-  double fx = 0, fy = 0, fz = 0;
-  for (int k0 = 0; k0 < p && count > 0; k0 += FRC_TABLE) {
-    const int kn = min(FRC_TABLE, p - k0);
-    __syncthreads();
-    unsigned rmax_hi = 0;
-    for (int w = 0; w < FB / 32; ++w) rmax_hi = max(rmax_hi, s_far[w]);
-    const double rmax = bound_of_hi(rmax_hi);
-    bool large = false;
-    for (int s = threadIdx.x; s < kn; s += FB) {
-      const KTab& t = tab[k0 + s];
-      s_tab[s] = KTabD{t.kx, t.ky, t.kz, t.a, t.b};
-      large |= !(norm1(t.kx, t.ky, t.kz) * rmax <= PHASE_MAX);
+  // a thread that has its atom to itself does what two would, one after the
+  // other: half the accumulators, twice the resident blocks
+  double fx = 0.0, fy = 0.0, fz = 0.0;
+  for (int half = 0; half < (share == 1 ? 2 : 1); ++half) {
+    const int first = share == 1 ? half : part;
+    double f[K_CLASSES / 2][3];  // classes first + max(share, 2) c
+#pragma unroll
+    for (int c = 0; c < K_CLASSES / 2; ++c) f[c][0] = f[c][1] = f[c][2] = 0.0;
+    for (int k0 = 0; k0 < p && count > 0; k0 += FRC_TABLE) {
+      const int kn = min(FRC_TABLE, p - k0);
+      const int kpad = (kn + K_CLASSES - 1) / K_CLASSES * K_CLASSES;
+      __syncthreads();
+      unsigned rmax_hi = 0;
+      for (int w = 0; w < FB / 32; ++w) rmax_hi = max(rmax_hi, s_far[w]);
+      const double rmax = bound_of_hi(rmax_hi);
+      bool large = false;
+      for (int s = threadIdx.x; s < kpad; s += FB) {
+        if (s < kn) {
+          const KTab& t = tab[k0 + s];
+          s_tab[s] = KTabD{t.kx, t.ky, t.kz, t.a, t.b};
+          large |= !(norm1(t.kx, t.ky, t.kz) * rmax <= PHASE_MAX);
+        } else {
+          s_tab[s] = KTabD{0.0, 0.0, 0.0, 0.0, 0.0};  // adds 0 to its class
+        }
+      }
+      large = __syncthreads_or(large);
+      auto add = [&](int s, double* fc, auto phase) {
+        const KTabD t = s_tab[s];
+        double sn, cs;
+        phase(t.kx * xo + t.ky * yo + t.kz * zo, &sn, &cs);
+        const double g = cs * t.b - sn * t.a;
+        fc[0] += g * t.kx;
+        fc[1] += g * t.ky;
+        fc[2] += g * t.kz;
+      };
+      auto classes = [&](auto step, auto phase) {
+        constexpr int STEP = decltype(step)::value;
+#pragma unroll 2
+        for (int s = first; s < kpad; s += K_CLASSES)
+#pragma unroll
+          for (int c = 0; c < K_CLASSES / STEP; ++c) add(s + STEP * c, f[c], phase);
+      };
+      auto all = [&](auto phase) {
+        if (share <= 2)
+          classes(std::integral_constant<int, 2>(), phase);
+        else if (share == 4)
+          classes(std::integral_constant<int, 4>(), phase);
+        else
+          classes(std::integral_constant<int, 8>(), phase);
+      };
+      if (mine && !large)
+        all([](double t, double* s, double* c) { sincos_phase(t, s, c); });
+      else if (mine)
+        all([](double t, double* s, double* c) { sincos(t, s, c); });
     }
-    large = __syncthreads_or(large);
-    auto add = [&](int s, auto phase) {
-      const KTabD t = s_tab[s];
-      double sn, cs;
-      phase(t.kx * xo + t.ky * yo + t.kz * zo, &sn, &cs);
-      const double f = cs * t.b - sn * t.a;
-      fx += f * t.kx;
-      fy += f * t.ky;
-      fz += f * t.kz;
-    };
-    auto phase = [](double t, double* s, double* c) { sincos_phase(t, s, c); };
-    if (mine && !large) {
-      if (share == 1)
-        for (int s = 0; s < kn; ++s) add(s, phase);
-      else
-        for (int s = part; s < kn; s += share) add(s, phase);
-    } else if (mine) {
-      for (int s = part; s < kn; s += share)
-        add(s, [](double t, double* s, double* c) { sincos(t, s, c); });
-    }
+    // the tree: classes c and c + 4, then c + 2, then c + 1, first those that a
+    // thread holds, then those of its neighbours (a share never crosses a warp)
+#pragma unroll
+    for (int h = K_CLASSES / 4; h > 0; h >>= 1)
+      if (share * h < K_CLASSES)
+#pragma unroll
+        for (int c = 0; c < h; ++c)
+          for (int d = 0; d < 3; ++d) f[c][d] += f[c + h][d];
+    fx += f[0][0];
+    fy += f[0][1];
+    fz += f[0][2];
   }
-  for (int o = share >> 1; o > 0; o >>= 1) {  // a share never crosses a warp
+  for (int o = share >> 1; o > 0; o >>= 1) {
     fx += __shfl_xor_sync(0xffffffffu, fx, o);
     fy += __shfl_xor_sync(0xffffffffu, fy, o);
     fz += __shfl_xor_sync(0xffffffffu, fz, o);

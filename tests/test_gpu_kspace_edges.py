@@ -124,6 +124,31 @@ def test_kspace_rounding(cuda, rbx):
     assert err(np.stack([v.cpu().numpy() for v in F], 1), f) < 8e-16
 
 
+@pytest.mark.parametrize("p", [7, 100, 1030])
+def test_force_does_not_depend_on_the_block(cuda, rbx, p):
+    """An atom's FP64 force is the same to the bit whatever shares its block:
+    the charged atoms alone, among as many neutral atoms, and with 1 in 3, 6,
+    12 and 40 charged (one to eight threads sum an atom's k-vectors)."""
+    lo, hi, pos, _, m = _system(500, p, 1.0, p)
+    q = np.random.default_rng(p).choice([-1.0, 0.5, 2.0], 500)
+    rng = np.random.default_rng(1)
+    dev = lambda a: cuda.as_tensor(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    box, rho = rbx.Box.make(lo, hi), [dev(rng.normal(size=p)) for _ in range(2)]
+    ref = None
+    for every in (1, 2, 3, 6, 12, 40):
+        n = 500 * every
+        at = np.sort(rng.choice(n, 500, replace=False))
+        x, c = rng.uniform(0, 20, (n, 3)), np.zeros(n)
+        x[at], c[at] = pos, q
+        F = [dev(np.ones(n)) for _ in range(3)]
+        rbx.rbe_force(box, 0.16, 50.0, 1.0, *rho, dev(c), *(dev(v) for v in m),
+                      *(dev(x[:, d]) for d in range(3)), *F)
+        f = np.stack([a.cpu().numpy() for a in F], 1)
+        assert (np.delete(f, at, 0) == 0).all()
+        ref = f[at] if ref is None else ref
+        assert np.array_equal(f[at], ref), every
+
+
 def test_kspace_any_phase(cuda, rbx):
     """Phases of 2^45 radians and far more still have a sine (positions are
     taken as they come)."""
