@@ -638,9 +638,9 @@ k_full_list(DBox b, int dimx, int dimy, int dimz, double cut2, float cut2_up, fl
 // A warp takes SL_C centre atoms; a block stages the fixed-point records of all
 // atoms tile by tile.  Their wrapped differences are the minimum image, and
 // |d|^2 in FP32 decides every pair outside a guard band (the RBL kernels'
-// bound); the FP64 predicate settles the rest.  Hits are appended in index order
-// through a ballot prefix, far pairs (certainly at least r_near, see FarSplit)
-// to the back.  Measured, B200, 1,000 / 1,500 / 3,000 atoms: 10.8 / 14.9 / 36.0 us;
+// bound) around the cutoff and around r_near; the FP64 distance settles the
+// rest.  Hits are appended in index order through a ballot prefix, far pairs (at
+// least r_near, see FarSplit) to the back.  Measured, B200, 1,000 / 1,500 / 3,000 atoms: 10.8 / 14.9 / 36.0 us;
 // 16.5 / 23.6 / 43.0 us with a warp an atom and FP64 distances.
 // ---------------------------------------------------------------------------
 constexpr int SL_WARPS = 8;
@@ -648,13 +648,14 @@ constexpr int SL_C = 2;       // centre atoms of a warp
 constexpr int SL_TILE = 1024; // atoms staged at a time
 
 struct SmallScreen {
-  float lo, hi, far;  // thresholds of the fixed-point |d|^2: cutoff band, certainly far
-  float w[3];         // L_d / L_max
+  IntScreen cut, near;  // of the fixed-point |d|^2: list cutoff, near and far segment
+  double cut2, near2;   // the same in FP64
+  float w[3];           // L_d / L_max
 };
 
 template <bool SPLIT>
 __global__ void __launch_bounds__(32 * SL_WARPS)
-k_full_list_small(DBox b, double cut2, SmallScreen sc, int n, const uint4* __restrict__ atoms,
+k_full_list_small(DBox b, SmallScreen sc, int n, const uint4* __restrict__ atoms,
                   const double* __restrict__ x, const double* __restrict__ y,
                   const double* __restrict__ z, int cap, int* __restrict__ count,
                   int* __restrict__ nbrs, int* __restrict__ overflow, int* __restrict__ far,
@@ -689,17 +690,25 @@ k_full_list_small(DBox b, double cut2, SmallScreen sc, int n, const uint4* __res
                     dy = (float)(int)(v.y - u[q].y) * sc.w[1],
                     dz = (float)(int)(v.z - u[q].z) * sc.w[2];
         d2[q] = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-        odd |= (d2[q] >= sc.lo) & (d2[q] < sc.hi);
+        odd |= (d2[q] >= sc.cut.lo) & (d2[q] < sc.cut.hi);
+        if (SPLIT) odd |= (d2[q] >= sc.near.lo) & (d2[q] < sc.near.hi);
       }
       const bool settle = __any_sync(0xffffffffu, odd & there);
 #pragma unroll
       for (int q = 0; q < SL_C; ++q) {
         const int i = i0 + q;
-        bool in = d2[q] < sc.lo;
-        if (settle && d2[q] >= sc.lo && d2[q] < sc.hi && there && i < n)
-          in = dist2_list(b, x[i], y[i], z[i], x[j], y[j], z[j]) < cut2;
+        bool in = d2[q] < sc.cut.lo, bk = SPLIT & (d2[q] >= sc.near.hi);
+        if (settle && there && i < n) {
+          const bool c = d2[q] >= sc.cut.lo && d2[q] < sc.cut.hi,
+                     f = SPLIT && d2[q] >= sc.near.lo && d2[q] < sc.near.hi;
+          if (c || f) {
+            const double r2 = dist2_list(b, x[i], y[i], z[i], x[j], y[j], z[j]);
+            if (c) in = r2 < sc.cut2;
+            if (f) bk = !(r2 < sc.near2);
+          }
+        }
         in = in & there & (j != i) & (i < n);
-        const bool bk = SPLIT & in & (d2[q] >= sc.far);
+        bk = bk & in;
         const unsigned mb = SPLIT ? __ballot_sync(0xffffffffu, bk) : 0u;
         const unsigned mf = __ballot_sync(0xffffffffu, in) ^ mb;
         const int pos = (bk ? nb[q] : nf[q]) + __popc((bk ? mb : mf) & lt);
@@ -734,21 +743,18 @@ int launch_full_list_small(const DBox& b, double cutoff, int n, const uint4* ato
   double L = 0.0;
   for (int d = 0; d < 3; ++d) L = fmax(L, b.len[d]);
   const double qerr = 64.0 * (L / 4294967296.0) * (cutoff + 1.0);
-  const double cut2 = cutoff * cutoff;
-  const IntScreen c = make_screen(cut2, L, 1e-4 + 8e-6 * cut2 + qerr);
   SmallScreen sc;
-  sc.lo = c.lo;
-  sc.hi = c.hi;
-  sc.far = INFINITY;
-  if (split) {
-    const double near2 = split->r_near * split->r_near;
-    sc.far = make_screen(near2, L, 1e-4 + 8e-6 * near2 + qerr).hi;
-  }
+  sc.cut2 = cutoff * cutoff;
+  sc.cut = make_screen(sc.cut2, L, 1e-4 + 8e-6 * sc.cut2 + qerr);
+  // the near threshold is raised by 1e-9 relative: FP64 rounding never moves a
+  // pair that could come within r_core before the next rebuild to the far segment
+  sc.near2 = split ? split->r_near * split->r_near * (1.0 + 1e-9) : 0.0;
+  sc.near = make_screen(sc.near2, L, 1e-4 + 8e-6 * sc.near2 + qerr);
   for (int d = 0; d < 3; ++d) sc.w[d] = (float)(b.len[d] / L);
   const int per_block = SL_WARPS * SL_C;
   const auto kern = split ? k_full_list_small<true> : k_full_list_small<false>;
   kern<<<(n + per_block - 1) / per_block, 32 * SL_WARPS, 0, st>>>(
-      b, cut2, sc, n, atoms, x, y, z, cap, count, nbrs, overflow, split ? split->far : nullptr,
+      b, sc, n, atoms, x, y, z, cap, count, nbrs, overflow, split ? split->far : nullptr,
       total);
   count_launch();
   return check_launch("full_list_small");

@@ -57,6 +57,31 @@ def test_small_box_forces_and_pairs(cuda, rbx, oracle, name, n, scale):
         e.close()
 
 
+def test_small_box_near_segment_is_exact(cuda, rbx):
+    """The near segment of a (mixed form's) row holds the pairs whose FP64
+    distance lies below r_near = r_core + skin and no others, also where r^2 is
+    within the fixed-point screen's guard band of r_near^2 (a lattice puts 24 pairs
+    an atom there).  The pair lists give the near segment first, as the rows do."""
+    a, side = 1.2, 11
+    r_near = a * 5 ** 0.5 * (1 - 2e-6)
+    s = systems.lj_electrolyte(side ** 3, seed=2, r_core=r_near - 0.3, skin=0.3,
+                               neighbor_sample_num=100000)
+    g = (np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3) + 0.5) * a
+    s = dict(s, pos=g, hi=np.full(3, side * a))
+    e = rbx.Engine(s, precision=rbx.MIXED)
+    e.compute_forces(0)
+    assert e.stats().selection_frequency == 1
+    _, shell = e.rbl_pairs()
+    e.close()
+    d = g[shell[:, 0] - 1] - g[shell[:, 1] - 1]
+    d -= side * a * np.round(d / (side * a))
+    far = (d ** 2).sum(1) > (r_near * (1 + 1e-6)) ** 2
+    order = np.argsort(shell[:, 0], kind="stable")
+    rows = np.split(far[order], np.searchsorted(shell[order, 0], s["gid"][1:]))
+    for r in rows:  # 6 pairs at 2 a, then the 24 at sqrt(5) a and all others
+        assert not r[:6].any() and r[6:].all() and r.sum() > 24
+
+
 def test_small_box_steps_keep_exact_pairs(cuda, rbx, oracle):
     """Velocity-Verlet steps with list rebuilds: after each block of steps the
     engine's RBL pairs equal the oracle's lists on the engine's own positions."""
