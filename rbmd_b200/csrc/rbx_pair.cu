@@ -736,28 +736,34 @@ RefLen<T> ref_len(const DBox& b) {
 
 // FilterRBLNeighborCandidates semantics (rbl_full_neighbor_list_op.hip.cu:237-304).
 // A warp an atom: lanes take consecutive candidates and append their hits
-// through ballot prefixes, so both lists keep the candidates' order.  (One
-// thread an atom walked 485 candidates in series with uncoalesced reads.)
-// Bound by the latency of the gathers, then the integer work of the hash; every
-// candidate is hashed (no branch) and eight blocks an SM are resident.  The float
-// build's 50,000 atoms x 485 candidates: 598 us serial; 177, 153, 146, 144 us at
-// the compiler's own choice of registers and at five, six and eight blocks.
+// through ballot prefixes, so both lists keep the candidates' order.  Bound by the
+// latency of the gathers, then the integer work of the hash; every candidate is
+// hashed (no branch) and eight blocks an SM are resident.
+// Short rows are a warp's latency and not its work: where 32 atoms in a row have
+// at most FILTER_SHORT candidates each, one of their four blocks does them all,
+// eight lanes an atom, and the other three return.  The largest shell count is one
+// atomic a block (one an atom, all at the same address, is 0.8 ns each).
+// Measured, B200, 50,000 atoms, us for rows of 4 / 16 / 32 / 64 / 485 candidates:
+// float 14 / 15 / 21 / 29 / 128, double 15 / 17 / 24 / 33 / 140; a thread an atom,
+// its row in series, 9 / 17 / 33 / 60 / 539 and 7 / 14 / 23 / 43 / 404; a warp an atom
+// and an atomic an atom throughout, 39 for every row up to 64, 128 and 132.
 // FREQ_LOW2: freq is 1, 2 or 4 and the batch test needs two bits of the hash.
-template <typename T, bool FREQ_LOW2>
-__global__ void __launch_bounds__(PAIR_BLOCK, 8)
-k_ref_rbl_filter(T core2, T force2, int n, const int* __restrict__ gid,
-                 const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ z,
-                 const int* __restrict__ cstart, const int* __restrict__ cend,
-                 const int* __restrict__ cand, const int* __restrict__ core_cap,
-                 const int* __restrict__ core_start, int* __restrict__ core_end,
-                 int* __restrict__ core, int shell_cap, int* __restrict__ shell,
-                 int* __restrict__ shell_num, int* __restrict__ required, RefLen<T> b,
-                 int* __restrict__ realloc, DivTest div, int epoch) {
+constexpr int FILTER_SHORT = 32;
+
+// Atom i's row by W neighbouring lanes (W = 32 or 8; the warp runs to the longest
+// of its rows); returns the shell count.
+template <typename T, bool FREQ_LOW2, int W>
+__device__ __forceinline__ int filter_row(
+    bool live, int i, T core2, T force2, int n, const int* __restrict__ gid,
+    const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ z,
+    const int* __restrict__ cstart, const int* __restrict__ cend, const int* __restrict__ cand,
+    const int* __restrict__ core_cap, const int* __restrict__ core_start,
+    int* __restrict__ core_end, int* __restrict__ core, int shell_cap, int* __restrict__ shell,
+    int* __restrict__ shell_num, const RefLen<T>& b, int* __restrict__ realloc,
+    const DivTest& div, int epoch) {
   constexpr int U = 2;  // candidates a lane takes per iteration
-  const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * PAIR_WARPS + (int)__shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
-  if (i >= n) return;
-  const unsigned lt = lanemask_lt();
+  const int lane = threadIdx.x & 31, sub = lane % W;
+  const unsigned lt = (1u << sub) - 1u, group = W == 32 ? 0xffffffffu : (1u << (W & 31)) - 1u;
   const unsigned mask = (1u << div.shift) - 1u;
   const T band_core = (T)4e-6 * (T)fabs(core2), band_force = (T)4e-6 * (T)fabs(force2);
   const unsigned long long ea = rbl_key_a(gid[i]) ^ (unsigned long long)(long long)epoch;
@@ -767,14 +773,15 @@ k_ref_rbl_filter(T core2, T force2, int n, const int* __restrict__ gid,
   // positions count from the row's start, unsigned: stepping past the end of a
   // row that ends near INT_MAX does not wrap
   const int c0 = cstart[i], c1 = cend[i];
-  const unsigned cnt = c1 > c0 ? (unsigned)c1 - (unsigned)c0 : 0u;
+  const unsigned cnt = live && c1 > c0 ? (unsigned)c1 - (unsigned)c0 : 0u;
+  const unsigned end = W == 32 ? cnt : __reduce_max_sync(0xffffffffu, cnt);
   const int* const row = cand + c0;
-  for (unsigned pos = 0; pos < cnt; pos += 32 * U) {
+  for (unsigned pos = 0; pos < end; pos += W * U) {
     int j[U], g[U];
     T d2[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const unsigned k = pos + 32 * u + lane;
+      const unsigned k = pos + W * u + sub;
       j[u] = k < cnt ? row[k] : i;
     }
 #pragma unroll
@@ -797,8 +804,12 @@ k_ref_rbl_filter(T core2, T force2, int n, const int* __restrict__ gid,
       const bool in_shell =
           other & !in_core & (d2[u] < force2) &
           (FREQ_LOW2 ? rbl_selected_low2(ea ^ kb, mask) : rbl_selected(ea, kb, div));
-      const unsigned mc = __ballot_sync(0xffffffffu, in_core);
-      const unsigned ms = __ballot_sync(0xffffffffu, in_shell);
+      unsigned mc = __ballot_sync(0xffffffffu, in_core);
+      unsigned ms = __ballot_sync(0xffffffffu, in_shell);
+      if (W < 32) {  // the atom's own lanes
+        mc = (mc >> (lane - sub)) & group;
+        ms = (ms >> (lane - sub)) & group;
+      }
       if (in_core) {
         const int o = nc + __popc(mc & lt);
         if (o < ccap) core[out0 + o] = j[u];
@@ -811,12 +822,57 @@ k_ref_rbl_filter(T core2, T force2, int n, const int* __restrict__ gid,
       ns += __popc(ms);
     }
   }
-  if (lane == 0) {
+  if (sub == 0 && live) {
     if (nc > ccap) atomicOr(realloc, 1);
     core_end[i] = out0 + (nc < ccap ? nc : ccap);
     shell_num[i] = ns < shell_cap ? ns : shell_cap;
+  }
+  return ns;
+}
+
+// The block's largest shell count into *required.
+__device__ __forceinline__ void filter_need(int ns, int* __restrict__ required) {
+  __shared__ int s_need[PAIR_WARPS];
+  if ((threadIdx.x & 31) == 0) s_need[threadIdx.x >> 5] = ns;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < PAIR_WARPS; ++w) ns = max(ns, s_need[w]);
     atomicMax(required, ns);
   }
+}
+
+template <typename T, bool FREQ_LOW2>
+__global__ void __launch_bounds__(PAIR_BLOCK, 8)
+k_ref_rbl_filter(T core2, T force2, int n, const int* __restrict__ gid,
+                 const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ z,
+                 const int* __restrict__ cstart, const int* __restrict__ cend,
+                 const int* __restrict__ cand, const int* __restrict__ core_cap,
+                 const int* __restrict__ core_start, int* __restrict__ core_end,
+                 int* __restrict__ core, int shell_cap, int* __restrict__ shell,
+                 int* __restrict__ shell_num, int* __restrict__ required, RefLen<T> b,
+                 int* __restrict__ realloc, DivTest div, int epoch) {
+  static_assert(PAIR_WARPS == 8, "four blocks of eight warps share 32 atoms");
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+  {
+    const int lane = threadIdx.x & 31, first = (int)(blockIdx.x / 4) * 32;
+    const int any = min(first + lane, n - 1);
+    if (__all_sync(0xffffffffu, (long long)cend[any] - cstart[any] <= FILTER_SHORT)) {
+      if (blockIdx.x % 4 != 0) return;  // the same for the whole block
+      const int i = first + 4 * warp + lane / 8;
+      const int ns = filter_row<T, FREQ_LOW2, 8>(
+          i < n, min(i, n - 1), core2, force2, n, gid, x, y, z, cstart, cend, cand, core_cap,
+          core_start, core_end, core, shell_cap, shell, shell_num, b, realloc, div, epoch);
+      filter_need((int)__reduce_max_sync(0xffffffffu, (unsigned)ns), required);
+      return;
+    }
+  }
+  const bool live = blockIdx.x * PAIR_WARPS + warp < n;
+  const int i = live ? blockIdx.x * PAIR_WARPS + warp : n - 1;
+  filter_need(filter_row<T, FREQ_LOW2, 32>(live, i, core2, force2, n, gid, x, y, z, cstart, cend,
+                                           cand, core_cap, core_start, core_end, core, shell_cap,
+                                           shell, shell_num, b, realloc, div, epoch),
+              required);
 }
 
 __device__ __forceinline__ double pow6(double v) {
@@ -1212,8 +1268,8 @@ int launch_ref_rbl_filter_t(T core2, T force2, int n, const int* gid, const T* x
   if (n <= 0) return RBX_OK;
   // freq = 1, 2 or 4 (DivTest of a power of two: inverse 1, shift log2)
   const bool low2 = div.trivial || (div.inv == 1ULL && div.shift <= 2);
-  auto kern = low2 ? k_ref_rbl_filter<T, true> : k_ref_rbl_filter<T, false>;
-  kern<<<(n + PAIR_WARPS - 1) / PAIR_WARPS, PAIR_BLOCK, 0, st>>>(
+  const auto kern = low2 ? k_ref_rbl_filter<T, true> : k_ref_rbl_filter<T, false>;
+  kern<<<(n + 31) / 32 * 4, PAIR_BLOCK, 0, st>>>(
       core2, force2, n, gid, x, y, z, cstart, cend, cand, core_cap, core_start, core_end, core,
       shell_cap, shell, shell_num, required, ref_len<T>(b), realloc, div, epoch);
   count_launch();

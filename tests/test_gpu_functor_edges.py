@@ -24,14 +24,15 @@ def _mix(v):
 
 @pytest.mark.parametrize("freq", [1, 2, 3, 4, 8])
 @pytest.mark.parametrize("caps", [(128, 192), (7, 5), (0, 0)])
-def test_filter_capacities(cuda, rbx, freq, caps):
+@pytest.mark.parametrize("lengths", [(0, 1, 31, 32, 63, 64, 65, 128, 200),
+                                     (32, 0, 1, 7, 8, 15, 16, 17, 31)])  # all short
+def test_filter_capacities(cuda, rbx, freq, caps, lengths):
     rng = np.random.default_rng(freq)
-    n, L, epoch = 300, 20.0, 9
+    n, L, epoch = 300, 20.0 if max(lengths) > 32 else 12.0, 9
     pos = rng.uniform(0, L, (n, 3))
     gid = rng.permutation(n).astype(np.int32) + 1
-    # 0, 1, 63, 64, 65, ... candidates (an atom may meet itself)
-    cand = [rng.choice(n, k, replace=False) for k in
-            [(0, 1, 31, 32, 63, 64, 65, 128, 200)[i % 9] for i in range(n)]]
+    # an atom may meet itself; the last rows are long again
+    cand = [rng.choice(n, lengths[i % 9] if i < 290 else 70, replace=False) for i in range(n)]
     count = np.array([len(c) for c in cand])
     start = np.concatenate([[0], np.cumsum(count)[:-1]]).astype(np.int32)
     ccap, scap = caps
@@ -69,6 +70,7 @@ def test_filter_capacities(cuda, rbx, freq, caps):
                 assert hshell[:int(snum[i]), i].tolist() == want[:scap].tolist()
     assert need.item() == most
     assert realloc.item() == (1 if most_core > ccap else 0)
+    assert most_core > 0 and most > 0
 
 
 @pytest.mark.parametrize("real", ["f64", "f32"])
