@@ -327,8 +327,9 @@ int rbx_ewald_force(const rbx_box* box, int num_atoms, const int kmax[3], double
   if (nk <= 0) return RBX_OK;
   double *re = nullptr, *im = nullptr, *kv = nullptr;
   KTab* tab = nullptr;
-  RBX_TRY(async_alloc(&re, nk, st));
-  RBX_TRY(async_alloc(&im, nk, st));
+  const size_t parts = ewald_parts(num_atoms, nk);
+  RBX_TRY(async_alloc(&re, parts * nk, st));
+  RBX_TRY(async_alloc(&im, parts * nk, st));
   RBX_TRY(async_alloc(&kv, (size_t)3 * nk, st));
   RBX_TRY(async_alloc(&tab, nk, st));
   double qsq = 0.0;

@@ -1369,19 +1369,20 @@ int rbx_engine::kspace_energy_exact(const int kmax[3], double* energy) {
     *energy = -prm.qqr2e * sqrt(prm.alpha / RBX_PI) * qsq;
     return RBX_OK;
   }
-  double* buf = nullptr;  // re, im, k vectors, one energy
-  if (cudaMallocAsync((void**)&buf, sizeof(double) * (5 * (size_t)nk + 1), st) != cudaSuccess) {
+  const size_t sums = (size_t)ewald_parts(n, nk) * nk;
+  double* buf = nullptr;  // partial re, im, k vectors, one energy
+  if (cudaMallocAsync((void**)&buf, sizeof(double) * (2 * sums + 3 * (size_t)nk + 1), st) !=
+      cudaSuccess) {
     cudaGetLastError();
     set_error("kspace_energy_exact: cudaMallocAsync failed");
     return RBX_ERR_NOMEM;
   }
-  int rc = launch_ewald(dbox, n, kmax, prm.alpha, prm.qqr2e, qsq, q, x, y, z, buf, buf + nk,
-                        buf + 2 * (size_t)nk, nullptr, nullptr, nullptr, nullptr,
-                        buf + 5 * (size_t)nk, st);
+  double* const kvec = buf + 2 * sums;
+  double* const e_out = kvec + 3 * (size_t)nk;
+  int rc = launch_ewald(dbox, n, kmax, prm.alpha, prm.qqr2e, qsq, q, x, y, z, buf, buf + sums, kvec,
+                        nullptr, nullptr, nullptr, nullptr, e_out, st);
   if (!rc)
-    rc = cuda_ok(cudaMemcpyAsync(energy, buf + 5 * (size_t)nk, sizeof(double),
-                                 cudaMemcpyDeviceToHost, st),
-                 "D2H");
+    rc = cuda_ok(cudaMemcpyAsync(energy, e_out, sizeof(double), cudaMemcpyDeviceToHost, st), "D2H");
   cudaFreeAsync(buf, st);
   if (!rc) rc = cuda_ok(cudaStreamSynchronize(st), "kspace energy sync");
   return rc;

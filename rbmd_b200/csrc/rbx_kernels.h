@@ -100,7 +100,9 @@ int launch_rbe_sample(int p, const double* tables, const int cnt[3], const doubl
                       double* mz, int* mi, int* status, cudaStream_t st);
 int launch_m_to_int(int p, const double* mx, const double* my, const double* mz, int* mi,
                     cudaStream_t st);
+// re, im: ewald_parts(n, nk) * nk entries of scratch, rho(k) in the first nk.
 // Forces only with tab (nk entries of scratch).
+int ewald_parts(int n, int nk);
 int launch_ewald(const DBox& b, int n, const int kmax[3], double alpha, double qqr2e,
                  double qsq, const double* q, const double* x, const double* y, const double* z,
                  double* re, double* im, double* kvec, KTab* tab, double* fx, double* fy,

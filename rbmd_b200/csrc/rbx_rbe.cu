@@ -987,18 +987,63 @@ __global__ void k_m_to_int(int p, const double* __restrict__ mx, const double* _
 // ---------------------------------------------------------------------------
 // A warp owns EW_KPT k-vectors, a block EW_BLOCK / 32 warps: the block streams
 // the atoms once for its 32 k-vectors, keeping the charged ones of each
-// tile in shared memory, and lanes take atoms.  (One block a k-vector read
-// every atom nk times: bound by L2, 300 us for 4,912 vectors x 20,011 atoms of
-// which 10 % are charged; 114 us now, the tile loop's two barriers a tile.)
-// Writes rho(k), the integer vector and, with tab, the force table entry of
-// coef exp(-k^2 / 4 alpha) / k^2.
+// tile in shared memory, and lanes take atoms.  (One block a k-vector reads every
+// atom nk times and is bound by L2.)  Where the k-vectors make fewer blocks than
+// fit the chip, the atoms are split over blockIdx.y as well: without that, 26
+// vectors are one block's work, and 200,000 atoms took it 3.4 ms.
+// Measured, B200, rho, force and energy (with the charges' copy to the host, some
+// 75 us) of 20,000 all-charged atoms, kmax 1 / 2 / 4 / 8: 115 / 129 / 237 / 939 us;
+// a block a k-vector 144 / 182 / 479 / 2,600, without the split 390 / 404 / 484 / 1,190.
+// Part blockIdx.y writes its sums to re, im[blockIdx.y][nk]; with one part they
+// are rho(k), and the k-vectors and the table are written too.
 constexpr int EW_BLOCK = 256;
 constexpr int EW_KPT = 4;
 constexpr int EW_PER_BLOCK = EW_BLOCK / 32 * EW_KPT;
 
+struct EwaldBox {
+  int nk, kmax[3];
+  double L[3], alpha, coef;
+  // k index -> (i, j, l) in ExecuteOnKmax order, skipping the origin
+  __device__ __forceinline__ void vector(int k, int m[3], double kv[3]) const {
+    const int ny = 2 * kmax[1] + 1, nz = 2 * kmax[2] + 1;
+    const int center = kmax[0] * ny * nz + kmax[1] * nz + kmax[2];
+    const int flat = k < center ? k : k + 1;
+    m[0] = flat / (ny * nz) - kmax[0];
+    m[1] = (flat / nz) % ny - kmax[1];
+    m[2] = flat % nz - kmax[2];
+    for (int d = 0; d < 3; ++d) kv[d] = 2 * RBX_PI * m[d] / L[d];
+  }
+  // k-vector k and, with tab, the force table entry of coef exp(-k^2 / 4 alpha) / k^2
+  __device__ __forceinline__ void entry(int k, double re, double im, double* __restrict__ kvec,
+                                        KTab* __restrict__ tab) const {
+    int m[3];
+    double kv[3];
+    vector(k, m, kv);
+    for (int d = 0; d < 3; ++d) kvec[3 * k + d] = kv[d];
+    if (!tab) return;
+    const double k2 = kv[0] * kv[0] + kv[1] * kv[1] + kv[2] * kv[2];
+    const double f = coef / k2 * exp(-0.25 * k2 / alpha);
+    KTab e;
+    e.kx = kv[0];
+    e.ky = kv[1];
+    e.kz = kv[2];
+    e.a = f * re;
+    e.b = f * im;
+    for (int d = 0; d < 3; ++d) e.m[d] = m[d];
+    e.m[3] = 0;
+    tab[k] = e;
+  }
+};
+
+int ewald_parts(int n, int nk) {
+  const int blocks = (nk + EW_PER_BLOCK - 1) / EW_PER_BLOCK, tiles = (n + EW_BLOCK - 1) / EW_BLOCK;
+  const int fit = 2 * sm_count();  // resident blocks
+  const int parts = blocks > 0 ? (fit + blocks - 1) / blocks : 1;
+  return parts < tiles ? parts : (tiles > 0 ? tiles : 1);
+}
+
 __global__ void __launch_bounds__(EW_BLOCK)
-k_ewald_rho(int n, int nk, int kx_max, int ky_max, int kz_max, double Lx, double Ly, double Lz,
-            double alpha, double coef, const double* __restrict__ q, const double* __restrict__ x,
+k_ewald_rho(int n, EwaldBox E, const double* __restrict__ q, const double* __restrict__ x,
             const double* __restrict__ y, const double* __restrict__ z, double* __restrict__ re,
             double* __restrict__ im, double* __restrict__ kvec, KTab* __restrict__ tab) {
   __shared__ double s_x[EW_BLOCK], s_y[EW_BLOCK], s_z[EW_BLOCK], s_q[EW_BLOCK];
@@ -1006,26 +1051,21 @@ k_ewald_rho(int n, int nk, int kx_max, int ky_max, int kz_max, double Lx, double
   __shared__ int s_cnt[EW_BLOCK / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int k0 = blockIdx.x * EW_PER_BLOCK + warp * EW_KPT;
-  // k index -> (i, j, l) in ExecuteOnKmax order, skipping the origin.
-  const int ny = 2 * ky_max + 1, nz = 2 * kz_max + 1;
-  const int center = kx_max * ny * nz + ky_max * nz + kz_max;
-  int m0[EW_KPT], m1[EW_KPT], m2[EW_KPT];
   double kx[EW_KPT], ky[EW_KPT], kz[EW_KPT], sr[EW_KPT], si[EW_KPT], kmax = 0.0;
 #pragma unroll
   for (int t = 0; t < EW_KPT; ++t) {
-    const int k = min(k0 + t, nk - 1);
-    const int flat = k < center ? k : k + 1;
-    m0[t] = flat / (ny * nz) - kx_max;
-    m1[t] = (flat / nz) % ny - ky_max;
-    m2[t] = flat % nz - kz_max;
-    kx[t] = 2 * RBX_PI * m0[t] / Lx;
-    ky[t] = 2 * RBX_PI * m1[t] / Ly;
-    kz[t] = 2 * RBX_PI * m2[t] / Lz;
+    int m[3];
+    double kv[3];
+    E.vector(min(k0 + t, E.nk - 1), m, kv);
+    kx[t] = kv[0];
+    ky[t] = kv[1];
+    kz[t] = kv[2];
     sr[t] = si[t] = 0.0;
     kmax = fmax(kmax, norm1(kx[t], ky[t], kz[t]));
   }
-  for (int base = 0; base < n; base += EW_BLOCK) {
-    const int j = base + threadIdx.x;
+  const int tiles = (n + EW_BLOCK - 1) / EW_BLOCK;
+  for (int tile = blockIdx.y; tile < tiles; tile += gridDim.y) {
+    const int j = tile * EW_BLOCK + threadIdx.x;
     const bool live = j < n;
     const double xj = live ? x[j] : 0.0, yj = live ? y[j] : 0.0, zj = live ? z[j] : 0.0;
     const double qj = live ? q[j] : 0.0;
@@ -1064,29 +1104,29 @@ k_ewald_rho(int n, int nk, int kx_max, int ky_max, int kz_max, double Lx, double
       si[t] += __shfl_xor_sync(0xffffffffu, si[t], o);
     }
     const int k = k0 + t;
-    if (lane == 0 && k < nk) {
-      re[k] = sr[t];
-      im[k] = si[t];
-      kvec[3 * k] = kx[t];
-      kvec[3 * k + 1] = ky[t];
-      kvec[3 * k + 2] = kz[t];
-      if (tab) {
-        const double k2 = kx[t] * kx[t] + ky[t] * ky[t] + kz[t] * kz[t];
-        const double f = coef / k2 * exp(-0.25 * k2 / alpha);
-        KTab e;
-        e.kx = kx[t];
-        e.ky = ky[t];
-        e.kz = kz[t];
-        e.a = f * sr[t];
-        e.b = f * si[t];
-        e.m[0] = m0[t];
-        e.m[1] = m1[t];
-        e.m[2] = m2[t];
-        e.m[3] = 0;
-        tab[k] = e;
-      }
+    if (lane == 0 && k < E.nk) {
+      re[(size_t)blockIdx.y * E.nk + k] = sr[t];
+      im[(size_t)blockIdx.y * E.nk + k] = si[t];
+      if (gridDim.y == 1) E.entry(k, sr[t], si[t], kvec, tab);
     }
   }
+}
+
+// rho(k) = the sum over the parts, left in part 0.
+__global__ void __launch_bounds__(128)
+k_ewald_parts(int parts, EwaldBox E, double* __restrict__ re, double* __restrict__ im,
+              double* __restrict__ kvec, KTab* __restrict__ tab) {
+  const int k = blockIdx.x * 128 + threadIdx.x;
+  if (k >= E.nk) return;
+  double r = 0.0, i = 0.0;
+#pragma unroll 8
+  for (int b = 0; b < parts; ++b) {
+    r += re[(size_t)b * E.nk + k];
+    i += im[(size_t)b * E.nk + k];
+  }
+  re[k] = r;
+  im[k] = i;
+  E.entry(k, r, i, kvec, tab);
 }
 
 __global__ void k_ewald_energy(int nk, double V, double alpha, double qqr2e, double qsq,
@@ -1384,12 +1424,26 @@ int launch_ewald(const DBox& b, int n, const int kmax[3], double alpha, double q
   const int nk = (2 * kmax[0] + 1) * (2 * kmax[1] + 1) * (2 * kmax[2] + 1) - 1;
   if (nk <= 0) return RBX_OK;
   const double V = b.len[0] * b.len[1] * b.len[2];
-  k_ewald_rho<<<(nk + EW_PER_BLOCK - 1) / EW_PER_BLOCK, EW_BLOCK, 0, st>>>(
-      n, nk, kmax[0], kmax[1], kmax[2], b.len[0], b.len[1], b.len[2], alpha,
-      -4.0 * RBX_PI * qqr2e / V, q, x, y, z, re, im, kvec, tab);
+  EwaldBox E;
+  E.nk = nk;
+  for (int d = 0; d < 3; ++d) {
+    E.kmax[d] = kmax[d];
+    E.L[d] = b.len[d];
+  }
+  E.alpha = alpha;
+  E.coef = -4.0 * RBX_PI * qqr2e / V;
+  const int parts = ewald_parts(n, nk);
+  k_ewald_rho<<<dim3((nk + EW_PER_BLOCK - 1) / EW_PER_BLOCK, parts), EW_BLOCK, 0, st>>>(
+      n, E, q, x, y, z, re, im, kvec, tab);
   count_launch();
   int rc = check_launch("ewald_rho");
   if (rc) return rc;
+  if (parts > 1) {
+    k_ewald_parts<<<(nk + 127) / 128, 128, 0, st>>>(parts, E, re, im, kvec, tab);
+    count_launch();
+    rc = check_launch("ewald_parts");
+    if (rc) return rc;
+  }
   if (n > 0 && tab) {
     RbeForceOut o;
     o.f_out_x = fx;

@@ -175,7 +175,9 @@ def test_kspace_any_phase(cuda, rbx):
 
 
 @pytest.mark.parametrize("n,kmax,share", [(300, (1, 1, 1), 1.0), (2000, (3, 2, 1), 0.1),
-                                          (70, (0, 4, 2), 0.0)])
+                                          (70, (0, 4, 2), 0.0),
+                                          (2, (0, 0, 1), 1.0),  # one ion's force is rounding only
+                                          (5000, (2, 3, 4), 0.5), (600, (11, 11, 11), 1.0)])
 def test_ewald_blocks(cuda, rbx, oracle, n, kmax, share):
     lo, hi, pos, q, _ = _system(n, 1, share, n)
     dev = lambda a: cuda.as_tensor(np.ascontiguousarray(a)).cuda()  # noqa: E731
