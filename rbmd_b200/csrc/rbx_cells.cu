@@ -19,6 +19,8 @@
 // then in cell order.
 #include <math.h>
 
+#include <algorithm>
+
 #include "rbx_common.cuh"
 #include "rbx_kernels.h"
 
@@ -254,24 +256,42 @@ k_cell_segsort(int ncell, int n, const int* __restrict__ start, const unsigned* 
 // 466 us (split rows 915 and 614), 20,000 atoms split 214 and 92, 4,000 atoms
 // split 171 and 42.
 // ---------------------------------------------------------------------------
-constexpr int NL_WARPS = 8;                // warps of a block
-constexpr int NL_BLOCK = 32 * NL_WARPS;
-constexpr int NL_CH = 4;                   // atoms of a chunk, centre atoms of a warp
-constexpr int NL_GROUP = NL_CH * NL_WARPS; // centre atoms of a block
-constexpr int NL_BATCH = 448;              // chunks staged at a time
-constexpr int NL_WORDS = 256;              // 32-chunk cull words handled at a time
+// W, the warps of a block (centre atoms 4 W): eight, or one where cells hold a few
+// atoms, whose blocks would leave most of eight warps idle.
+constexpr int NL_CH = 4;  // atoms of a chunk, centre atoms of a warp
+template <int W>
+struct ListShape {
+  static constexpr int GROUP = NL_CH * W;            // centre atoms of a block
+  static constexpr int BATCH = W == 8 ? 448 : 64;    // chunks staged at a time
+  static constexpr int WORDS = W == 8 ? 256 : 64;    // 32-chunk cull words handled at a time
+  static constexpr int RESIDENT = W == 8 ? 4 : 24;   // blocks of an SM
+};
 
 __device__ __forceinline__ int chunk_base(int c, int cs) { return cs / NL_CH + c; }
-__device__ __forceinline__ int group_base(int c, int cs) { return cs / NL_GROUP + c; }
+__device__ __forceinline__ int group_base(int c, int cs, int group) { return cs / group + c; }
 
-static size_t full_list_groups(int n, int ncell) { return (size_t)(n / NL_GROUP) + ncell; }
+static size_t full_list_groups(int n, int ncell, int group) { return (size_t)(n / group) + ncell; }
 static size_t full_list_chunks(int n, int ncell) { return (size_t)(n / NL_CH) + ncell; }
+// With fewer than LIST_DILUTE atoms a cell on average the cells of at most LIST_FEW
+// atoms go to one-warp blocks (a second launch), the others to the eight-warp
+// blocks, as all do in a denser box: a gas and a droplet in a large box each get
+// the blocks that suit them.  The indices of the eight-warp groups are then
+// gathered first: a block that finds none costs 1 ns, and most would.  Measured, B200, us, eight warps / one for all cells:
+// 200,000 atoms of 0.3, 1, 3, 6 and 12 a cell 1779 / 545, 1252 / 556, 809 / 529,
+// 475 / 469, 314 / 508; 4,000 atoms of 1, 2, 3 and 6 32 / 20, 28 / 24, 22 / 25, 18 / 27.
+constexpr long long LIST_DILUTE = 3;
+constexpr int LIST_FEW = 6;
+static bool list_dilute(int n, int ncell) { return n < LIST_DILUTE * ncell; }
+// Most groups that cells of more than LIST_FEW atoms can make.
+static int list_many(int n) { return n / ListShape<8>::GROUP + n / (LIST_FEW + 1) + 1; }
 
 // Device scratch of one list build.
 struct ListTables {
   float4* rel;      // plain rows: an atom's FP32 position relative to its cell's centre
   float4 *lo, *hi;  // per chunk: its box relative to its cell's centre, rounded outwards
-  int* group_cell;  // per group: its cell, -1 for an index between two cells
+  int* group_cell;  // per group: its cell, -1 for an index without a group
+  int* few_cell;    // the same for the one-warp blocks, null where there are none
+  int* many;        // then: how many groups group_cell has, and their indices
 };
 
 __global__ void __launch_bounds__(128)
@@ -311,9 +331,37 @@ k_chunk_boxes(DBox b, int dimx, int dimy, int dimz, const double* __restrict__ x
       T.hi[k] = make_float4(hi[0], hi[1], hi[2], 0.f);
     }
   }
-  const int g0 = group_base(c, cs), ng = (ce - cs + NL_GROUP - 1) / NL_GROUP;
-  const int g1 = group_base(c + 1, ce);  // first index of the next cell
-  for (int g = g0 + threadIdx.x; g < g1; g += blockDim.x) T.group_cell[g] = g < g0 + ng ? c : -1;
+  const bool few = T.few_cell && ce - cs <= LIST_FEW;
+  auto groups = [&](int* __restrict__ of, int size, bool taken) {
+    const int g0 = group_base(c, cs, size), ng = taken ? (ce - cs + size - 1) / size : 0;
+    const int g1 = group_base(c + 1, ce, size);  // first index of the next cell
+    for (int g = g0 + threadIdx.x; g < g1; g += blockDim.x) of[g] = g < g0 + ng ? c : -1;
+  };
+  groups(T.group_cell, ListShape<8>::GROUP, !few);
+  if (T.few_cell) groups(T.few_cell, ListShape<1>::GROUP, few);
+  if (T.few_cell && c == 0 && threadIdx.x == 0) T.many[0] = 0;
+}
+
+// The indices of the groups in group_cell, in any order (rows do not depend on it).
+__global__ void __launch_bounds__(256) k_many_groups(int groups, ListTables T) {
+  __shared__ int s_at[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = blockIdx.x * 256 + threadIdx.x;
+  const bool live = g < groups && T.group_cell[g] >= 0;
+  const unsigned m = __ballot_sync(0xffffffffu, live);
+  if (lane == 0) s_at[warp] = __popc(m);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int sum = 0;
+    for (int w = 0; w < 8; ++w) {
+      const int k = s_at[w];
+      s_at[w] = sum;
+      sum += k;
+    }
+    const int first = sum ? atomicAdd(T.many, sum) : 0;
+    for (int w = 0; w < 8; ++w) s_at[w] += first;
+  }
+  __syncthreads();
+  if (live) T.many[1 + s_at[warp] + __popc(m & ((1u << lane) - 1u))] = g;
 }
 
 // A store under a predicate, without a branch around it.
@@ -325,40 +373,49 @@ __device__ __forceinline__ void store_if(bool take, int* p, int v) {
       : "memory");
 }
 
+template <int W>
 struct FullListSmem {
-  float4 atom[(NL_BATCH + 1) * NL_CH];  // staged chunks; the last one is empty
-  float2 bx[NL_BATCH], by[NL_BATCH], bz[NL_BATCH];  // {lo, hi} of a staged chunk
-  int first[NL_BATCH + 1];              // its first atom
-  unsigned short meta[NL_BATCH];        // stencil cell | atoms << 8
-  unsigned short pick[NL_WARPS][NL_BATCH + 8];  // a warp's surviving chunks
+  static constexpr int BATCH = ListShape<W>::BATCH, WORDS = ListShape<W>::WORDS;
+  float4 atom[(BATCH + 1) * NL_CH];  // staged chunks; the last one is empty
+  float2 bx[BATCH], by[BATCH], bz[BATCH];  // {lo, hi} of a staged chunk
+  int first[BATCH + 1];              // its first atom
+  unsigned short meta[BATCH];        // stencil cell | atoms << 8
+  unsigned short pick[W][BATCH + 8];  // a warp's surviving chunks
   float4 edge[27];                      // centre of a stencil cell's image, relative to the
   float shl[27][3], shh[27][3];         // centre cell's; and rounded down and up
   double shift[27][3];                  // its periodic image minus the centre cell's centre
   int cs[27], ce[27], cb[27];           // atom range and first chunk index of a stencil cell
   int word0[28];                        // first cull word of a stencil cell
-  unsigned mask[NL_WORDS];              // surviving chunks of a word
-  int off[NL_WORDS + 1];                // survivors before it
+  unsigned mask[WORDS];              // surviving chunks of a word
+  int off[WORDS + 1];                // survivors before it
 };
 
 // SPLIT: RBL rows with a far segment; without it (Verlet lists) no far test.
-template <bool SPLIT>
-__global__ void __launch_bounds__(NL_BLOCK, 4)
+template <bool SPLIT, int W>
+__global__ void __launch_bounds__(32 * W, ListShape<W>::RESIDENT)
 k_full_list(DBox b, int dimx, int dimy, int dimz, double cut2, float cut2_up, float lo_band,
             float hi_band, const double* __restrict__ x, const double* __restrict__ y,
             const double* __restrict__ z, const int* __restrict__ cell_start, ListTables T,
             int cap, int* __restrict__ count, int* __restrict__ nbrs, int* __restrict__ overflow,
             float near2, int* __restrict__ far, long long* __restrict__ total) {
+  constexpr int BLOCK = 32 * W, GROUP = ListShape<W>::GROUP;
+  constexpr int BATCH = ListShape<W>::BATCH, WORDS = ListShape<W>::WORDS;
   extern __shared__ __align__(16) unsigned char s_list[];
-  FullListSmem& S = *reinterpret_cast<FullListSmem*>(s_list);
-  const int c = T.group_cell[blockIdx.x];
-  if (c < 0) return;  // an index between two cells
+  FullListSmem<W>& S = *reinterpret_cast<FullListSmem<W>*>(s_list);
+  int block = blockIdx.x;
+  if (W == 8 && T.few_cell) {
+    if (block >= T.many[0]) return;
+    block = T.many[1 + block];
+  }
+  const int c = (W == 1 ? T.few_cell : T.group_cell)[block];
+  if (c < 0) return;  // an index without a group
   // the warp's index through a shuffle, so that the compiler knows the loops
   // below to be uniform over the warp
   const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const unsigned lt = (1u << lane) - 1u;
   const int cs = cell_start[c], ce = cell_start[c + 1];
-  const int g = (int)blockIdx.x - group_base(c, cs);
-  const int i0 = cs + NL_GROUP * g + NL_CH * warp;  // this warp's first centre atom
+  const int g = block - group_base(c, cs, GROUP);
+  const int i0 = cs + GROUP * g + NL_CH * warp;  // this warp's first centre atom
   const int cz = c / (dimx * dimy), cy = (c / dimx) % dimy, cx = c % dimx;
   const double ox = b.lo[0] + (cx + 0.5) * (b.len[0] / dimx);  // the centre cell's centre
   const double oy = b.lo[1] + (cy + 0.5) * (b.len[1] / dimy);
@@ -403,9 +460,9 @@ k_full_list(DBox b, int dimx, int dimy, int dimz, double cut2, float cut2_up, fl
     if (lane < 27) S.word0[lane + 1] = incl;
     if (lane == 0) S.word0[0] = 0;
   }
-  if (threadIdx.x < NL_CH) S.atom[NL_BATCH * NL_CH + threadIdx.x] =
+  if (threadIdx.x < NL_CH) S.atom[BATCH * NL_CH + threadIdx.x] =
       make_float4(0.f, 0.f, 0.f, INFINITY);  // an empty slot: never a hit
-  if (threadIdx.x == NL_CH) S.first[NL_BATCH] = 0;
+  if (threadIdx.x == NL_CH) S.first[BATCH] = 0;
   // this warp's centres i0 + q: their tests and their box (it is their chunk's)
   float ax[NL_CH], ay[NL_CH], az[NL_CH], lo_i[NL_CH], hi_i[NL_CH], near_i[NL_CH];
 #pragma unroll
@@ -421,10 +478,10 @@ k_full_list(DBox b, int dimx, int dimy, int dimz, double cut2, float cut2_up, fl
     hi_i[q] = live ? hi_band - uu : -INFINITY;
     near_i[q] = near2 - uu;  // far pairs: d above this
   }
-  const int own = chunk_base(c, cs) + (int)NL_WARPS * g;  // the group's first chunk
+  const int own = chunk_base(c, cs) + W * g;  // the group's first chunk
   float ulo[3], uhi[3], glo[3], ghi[3];                   // boxes of the group, of the warp
   {
-    const bool ok = lane < NL_WARPS && cs + NL_GROUP * g + NL_CH * lane < ce;
+    const bool ok = lane < W && cs + GROUP * g + NL_CH * lane < ce;
     const float4 l = T.lo[ok ? own + lane : own], h = T.hi[ok ? own + lane : own];
     const float ll[3] = {l.x, l.y, l.z}, hh[3] = {h.x, h.y, h.z};
 #pragma unroll
@@ -434,7 +491,7 @@ k_full_list(DBox b, int dimx, int dimy, int dimz, double cut2, float cut2_up, fl
       ulo[d] = ll[d];  // lanes without a chunk repeat the first
       uhi[d] = hh[d];
 #pragma unroll
-      for (int s = 1; s < NL_WARPS; s <<= 1) {
+      for (int s = 1; s < W; s <<= 1) {
         ulo[d] = fminf(ulo[d], __shfl_xor_sync(0xffffffffu, ulo[d], s));
         uhi[d] = fmaxf(uhi[d], __shfl_xor_sync(0xffffffffu, uhi[d], s));
       }
@@ -473,9 +530,9 @@ k_full_list(DBox b, int dimx, int dimy, int dimz, double cut2, float cut2_up, fl
   };
 
   const int nwords = S.word0[27];
-  for (int wb = 0; wb < nwords; wb += NL_WORDS) {
-    const int nw = min(NL_WORDS, nwords - wb);
-    for (int w = warp; w < nw; w += NL_WARPS) {  // level 1
+  for (int wb = 0; wb < nwords; wb += WORDS) {
+    const int nw = min(WORDS, nwords - wb);
+    for (int w = warp; w < nw; w += W) {  // level 1
       const int s = word_cell(wb + w);
       const int k = (wb + w - S.word0[s]) * 32 + lane;
       bool near = false;
@@ -505,14 +562,14 @@ k_full_list(DBox b, int dimx, int dimy, int dimz, double cut2, float cut2_up, fl
     }
     __syncthreads();
     const int found = S.off[nw];
-    for (int b0 = 0; b0 < found; b0 += NL_BATCH) {
-      const int nb = min(NL_BATCH, found - b0);
-      for (int w = warp; w < nw; w += NL_WARPS) {  // the batch's chunks
-        if (S.off[w + 1] <= b0 || S.off[w] >= b0 + NL_BATCH) continue;
+    for (int b0 = 0; b0 < found; b0 += BATCH) {
+      const int nb = min(BATCH, found - b0);
+      for (int w = warp; w < nw; w += W) {  // the batch's chunks
+        if (S.off[w + 1] <= b0 || S.off[w] >= b0 + BATCH) continue;
         const int s = word_cell(wb + w);
         const unsigned m = S.mask[w];
         const int slot = S.off[w] + __popc(m & lt) - b0;
-        if (((m >> lane) & 1u) && slot >= 0 && slot < NL_BATCH) {
+        if (((m >> lane) & 1u) && slot >= 0 && slot < BATCH) {
           const int k = (wb + w - S.word0[s]) * 32 + lane;
           float rl[3], rh[3];
           chunk_box(s, k, rl, rh);
@@ -526,7 +583,7 @@ k_full_list(DBox b, int dimx, int dimy, int dimz, double cut2, float cut2_up, fl
       }
       __syncthreads();
 #pragma unroll 4
-      for (int t = threadIdx.x; t < nb * NL_CH; t += NL_BLOCK) {  // its atoms
+      for (int t = threadIdx.x; t < nb * NL_CH; t += BLOCK) {  // its atoms
         const int slot = t / NL_CH, u = t % NL_CH;
         const int meta = S.meta[slot];
         const double* const sh = S.shift[meta & 255];
@@ -560,7 +617,7 @@ k_full_list(DBox b, int dimx, int dimy, int dimz, double cut2, float cut2_up, fl
           if (near) pick[np + __popc(m & lt)] = (unsigned short)k;
           np += __popc(m);
         }
-        if (lane < 8) pick[np + lane] = NL_BATCH;  // pad with the empty chunk
+        if (lane < 8) pick[np + lane] = BATCH;  // pad with the empty chunk
         __syncwarp();
         const int u = lane % NL_CH;
         for (int t = 0; t < np; t += 32 / NL_CH) {
@@ -1052,16 +1109,20 @@ int launch_cells_sort(const DBox& b, const int dims[3], int n, const double* x, 
   return check_launch("cells_sort");
 }
 
-static size_t list_pieces(int n, int ncell, size_t piece[4]) {
+static size_t list_pieces(int n, int ncell, size_t piece[6]) {
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
   piece[0] = al(sizeof(float4) * (size_t)n);
   piece[1] = piece[2] = al(sizeof(float4) * full_list_chunks(n, ncell));
-  piece[3] = al(sizeof(int) * full_list_groups(n, ncell));
-  return piece[0] + piece[1] + piece[2] + piece[3];
+  piece[3] = al(sizeof(int) * full_list_groups(n, ncell, ListShape<8>::GROUP));
+  piece[4] = list_dilute(n, ncell)
+                 ? al(sizeof(int) * full_list_groups(n, ncell, ListShape<1>::GROUP))
+                 : 0;
+  piece[5] = list_dilute(n, ncell) ? al(sizeof(int) * (1 + (size_t)list_many(n))) : 0;
+  return piece[0] + piece[1] + piece[2] + piece[3] + piece[4] + piece[5];
 }
 
 size_t full_list_scratch_bytes(int n, int ncell) {
-  size_t piece[4];
+  size_t piece[6];
   return list_pieces(n, ncell, piece);
 }
 
@@ -1099,7 +1160,7 @@ int launch_full_list(const DBox& b, const int dims[3], double cutoff, int n, con
   const float lo_band = (float)(cut2 - band), hi_band = (float)(cut2 + band);
   float cut2_up = (float)cut2;  // rounded up
   if ((double)cut2_up < cut2) cut2_up = nextafterf(cut2_up, INFINITY);
-  size_t piece[4];
+  size_t piece[6];
   list_pieces(n, ncell, piece);
   char* p = (char*)scratch;
   ListTables T;
@@ -1107,19 +1168,37 @@ int launch_full_list(const DBox& b, const int dims[3], double cutoff, int n, con
   T.lo = (float4*)(p + piece[0]);
   T.hi = (float4*)(p + piece[0] + piece[1]);
   T.group_cell = (int*)(p + piece[0] + piece[1] + piece[2]);
-  k_chunk_boxes<<<ncell, 128, 0, st>>>(b, dims[0], dims[1], dims[2], x, y, z, cell_start, T);
+  T.few_cell = piece[4] ? (int*)(p + piece[0] + piece[1] + piece[2] + piece[3]) : nullptr;
+  T.many = T.few_cell ? (int*)((char*)T.few_cell + piece[4]) : nullptr;
+  // a thread an atom: 32 threads a cell up to some 60 atoms (200,000 atoms of 1 / 16 /
+  // 120 a cell: 103 / 9 / 7 us, 128 threads 190 / 15 / 5)
+  k_chunk_boxes<<<ncell, n < 60LL * ncell ? 32 : 128, 0, st>>>(b, dims[0], dims[1], dims[2], x, y, z,
+                                                              cell_start, T);
   count_launch();
   // far threshold in r^2, raised by the FP32 error of the test value
   const float near2 = split ? (float)(split->r_near * split->r_near + band) : INFINITY;
-  const auto kern = split ? k_full_list<true> : k_full_list<false>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sizeof(FullListSmem)) != cudaSuccess)
-    return check_launch("full_list (shared memory)");
-  kern<<<(unsigned)full_list_groups(n, ncell), NL_BLOCK, sizeof(FullListSmem), st>>>(
-      b, dims[0], dims[1], dims[2], cut2, cut2_up, lo_band, hi_band, x, y, z, cell_start, T, cap,
-      count, nbrs, overflow, near2, split ? split->far : nullptr, total);
-  count_launch();
-  return check_launch("full_list");
+  const int many = (int)full_list_groups(n, ncell, ListShape<8>::GROUP);
+  auto build = [&](auto kern, unsigned blocks, int warps, int smem) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+        cudaSuccess)
+      return check_launch("full_list (shared memory)");
+    kern<<<blocks, 32 * warps, smem, st>>>(
+        b, dims[0], dims[1], dims[2], cut2, cut2_up, lo_band, hi_band, x, y, z, cell_start, T,
+        cap, count, nbrs, overflow, near2, split ? split->far : nullptr, total);
+    count_launch();
+    return check_launch("full_list");
+  };
+  if (T.few_cell) {
+    k_many_groups<<<(many + 255) / 256, 256, 0, st>>>(many, T);
+    count_launch();
+    const int rc = build(split ? k_full_list<true, 1> : k_full_list<false, 1>,
+                         (unsigned)full_list_groups(n, ncell, ListShape<1>::GROUP), 1,
+                         (int)sizeof(FullListSmem<1>));
+    if (rc) return rc;
+  }
+  return build(split ? k_full_list<true, 8> : k_full_list<false, 8>,
+               (unsigned)(T.few_cell ? std::min(many, list_many(n)) : many), 8,
+               (int)sizeof(FullListSmem<8>));
 }
 
 // dst[a][idx[i]] = src[a][i] for every array of the set (one launch).

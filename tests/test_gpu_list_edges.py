@@ -1,6 +1,7 @@
 """The stencil list builder where its tiles end: groups and chunks with
 remainders, cells of several cull words, more surviving chunks than one
-staged batch, more cull words than one pass, cells with one atom or none, an
+staged batch, more cull words than one pass, cells with one atom or none, dense
+cells in a mostly empty box (whose cells of few atoms take other blocks), an
 orthorhombic box away from the origin.
 
 Rows must equal, in order, the FP64 predicate (minimum image, squares summed
@@ -20,19 +21,32 @@ def _uniform(n, lo, hi, seed):
     return lo, hi, lo + rng.uniform(0.0, 1.0, (n, 3)) * (hi - lo)
 
 
-def _clusters(per_cell, seed):
-    """27 unit cells, each with per_cell atoms within 0.004 of its centre."""
+def _clusters(per_cell, seed, side=3.0):
+    """27 unit cells, each with per_cell atoms within 0.004 of its centre, in a
+    box of side^3 such cells."""
     rng = np.random.default_rng(seed)
     k = np.arange(27)
     cen = np.stack([k % 3, (k // 3) % 3, k // 9], 1) + 0.5
     pos = np.repeat(cen, per_cell, 0) + rng.uniform(-0.002, 0.002, (27 * per_cell, 3))
-    return np.zeros(3), np.full(3, 3.0), pos
+    return np.zeros(3), np.full(3, side), pos
+
+
+def _gas_and_drops(seed):
+    """Clusters of 300 atoms in one corner of 16^3 cells, every other cell with
+    none to a dozen atoms."""
+    lo, hi, pos = _clusters(300, seed, 16.0)
+    rng = np.random.default_rng(seed + 1)
+    gas = rng.uniform(0.0, 16.0, (4000, 3))
+    near = rng.uniform(0.0, 4.0, (200, 3)) + 6.0
+    return lo, hi, np.concatenate([pos, gas, near])
 
 
 CASES = {
     "three_cells_n3300": (lambda: _uniform(3300, [0] * 3, [16.1] * 3, 1), 5.3),
     "dense_batches": (lambda: _uniform(20000, [0] * 3, [12.0] * 3, 2), 3.0),
     "many_cull_words": (lambda: _clusters(1300, 3), 0.99),
+    "gas_and_drops": (lambda: _gas_and_drops(7), 0.99),
+    "drops_in_a_void": (lambda: _clusters(1300, 3, 24.0), 0.99),
     "sparse_n40": (lambda: _uniform(40, [0] * 3, [30.0] * 3, 4), 5.0),
     "orthorhombic_offset": (lambda: _uniform(5003, [-7, 3, 100], [13, 20, 123], 5), 4.1),
 }

@@ -18,6 +18,7 @@ CASES = {
     "almost_all_far": (0.8, 0.9, 5.0, 0.3, 100),
     "wide_skin": (0.8, 2.5, 4.0, 1.5, 60),
     "short_rows": (0.02, 2.5, 5.0, 0.3, 2),
+    "dilute": (0.01, 2.5, 5.0, 0.3, 2),
     "ragged_far": (0.3, 2.0, 4.4, 0.45, 20),
 }
 
@@ -39,3 +40,19 @@ def test_rbl_segments(cuda, rbx, oracle, name):
         assert systems.rel_rms(f, want["force"]) < tol, (prec, name)
         assert np.isfinite(f).all()
         e.close()
+
+
+def test_dilute_steps_in_the_graph(cuda, rbx):
+    """A box of two atoms a cell (its list is built by two launches): steps from
+    the captured graph, rebuilds included, equal the launch-by-launch engine's."""
+    s = systems.lj_electrolyte(3000, seed=8, density=0.01, temperature=40.0)
+    out = []
+    for graph in (True, False):
+        e = rbx.Engine(s, precision=rbx.MIXED, seed=4)
+        e.set_step_graph(graph)
+        e.step(60)
+        assert e.stats().rebuilds >= 2
+        out.append(e.get_state())
+        e.close()
+    for k in ("pos", "vel", "force"):
+        assert np.array_equal(out[0][k], out[1][k])
