@@ -169,11 +169,17 @@ __global__ void k_cell_scatter(int n, const int* __restrict__ cell,
   tmp[base + __popc(same & ((1u << lane) - 1u))] = (sub[i] << SUB_SHIFT) | (unsigned)i;
 }
 
-// One block per cell: bitonic sort of the cell's keys (sub-cell, old index).  A
-// cell of edge cut_off + skin holds some 120 atoms: 128 threads a block let every
-// cell's block be resident at once (200,000 atoms: 21 us at 512 threads, 12 us).
-constexpr int SORT_BLOCK = 128;
-__global__ void __launch_bounds__(SORT_BLOCK)
+// One block per cell: bitonic sort of the cell's keys (sub-cell, old index).  128
+// threads a block let many cells be resident at once; 512 shorten the passes over
+// full cells.  Measured, B200, 200,000 atoms of 120 / 200 / 300 / 400 / 600 / 1,200 a
+// cell: 13 / 11 / 18 / 18 / 35 / 75 us with 128, 21 / 16 / 19 / 15 / 21 / 30 with 512;
+// 27 cells of 120 8.3 and 6.2, where all are resident either way.
+constexpr int SORT_BLOCK = 128, SORT_BLOCK_FULL = 512;
+static int sort_block(int n, int ncell) {
+  const long long full = ncell <= 2 * sm_count() ? 100 : 350;  // atoms a cell
+  return n < full * ncell ? SORT_BLOCK : SORT_BLOCK_FULL;
+}
+__global__ void __launch_bounds__(SORT_BLOCK_FULL)
 k_cell_segsort(int ncell, int n, const int* __restrict__ start, const unsigned* __restrict__ tmp,
                int* __restrict__ perm, int* __restrict__ cell_of_sorted, int* __restrict__ status) {
   __shared__ unsigned s[SEG_MAX];
@@ -1103,8 +1109,8 @@ int launch_cells_sort(const DBox& b, const int dims[3], int n, const double* x, 
     k_cell_scatter<<<(n + 255) / 256, 256, 0, st>>>(n, cell, sub, fill, tmp);
     count_launch();
   }
-  k_cell_segsort<<<ncell, SORT_BLOCK, 0, st>>>(ncell, n, cell_start, tmp, perm, cell_of_sorted,
-                                               status);
+  k_cell_segsort<<<ncell, sort_block(n, ncell), 0, st>>>(
+      ncell, n, cell_start, tmp, perm, cell_of_sorted, status);
   count_launch();
   return check_launch("cells_sort");
 }

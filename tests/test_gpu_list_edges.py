@@ -43,6 +43,7 @@ def _gas_and_drops(seed):
 
 CASES = {
     "three_cells_n3300": (lambda: _uniform(3300, [0] * 3, [16.1] * 3, 1), 5.3),
+    "full_cells": (lambda: _uniform(27000, [0] * 3, [3.0] * 3, 8), 0.99),
     "dense_batches": (lambda: _uniform(20000, [0] * 3, [12.0] * 3, 2), 3.0),
     "many_cull_words": (lambda: _clusters(1300, 3), 0.99),
     "gas_and_drops": (lambda: _gas_and_drops(7), 0.99),
