@@ -756,10 +756,11 @@ int rbx_lammps_write_charge(const char* path, const rbx_box* box, int n, int nty
  *     For RBL engines in the mixed form with RBE k-space, NVE, no SHAKE and
  *     no special bonds;
  *   RBX_BATCH_BRANCHES: every replica's own step graph as a parallel branch.
- * RBX_BATCH_AUTO (the default) takes the phased design for replicas of fewer
- * than 5,000 atoms on average when every replica allows it, else the
- * branches.  The engines stay owned by the caller and
- * must outlive the batch; each must have skin > 0 and profiling off.  Results
+ * RBX_BATCH_AUTO (the default) takes the branches for replicas of 5,000 atoms or
+ * more on average, for six or more smaller ones of at least 50 atoms per replica
+ * of the batch (24 of 1,200 atoms, 80 of 4,000), and where a replica does not
+ * allow the phased design; else the phased design.  The engines stay owned by
+ * the caller and must outlive the batch; each must have skin > 0 and profiling off.  Results
  * equal stepping each engine alone, in either design.  No counterpart in the
  * reference (one system per process). */
 #define RBX_BATCH_AUTO 0

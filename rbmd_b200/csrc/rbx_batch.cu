@@ -218,22 +218,27 @@ struct rbx_batch {
     return RBX_OK;
   }
 
-  // AUTO: the branches for replicas of kPhasedMeanAtoms atoms or more on
-  // average (the phased force launches wait for every replica's rebuild) and
-  // for nine to kBranchReplicas smaller ones; else the phased graph: one launch
-  // per phase pays off over many small replicas, whose graph of branches is
-  // bound by node scheduling, and a handful makes a small graph either way.
-  // Measured, us per step, phased and branches: 192 x 1,753 atoms 1864 / 3414,
-  // 96 x 2,095 1214 / 1314, 48 x 4,448 940 / 843, 24 x 1,990 367 / 337,
-  // 12 x 4,393 350 / 318, 8 x 1,364 136 / 122, 64 x 5,120 1523 / 1410;
-  // 910 x 2,000 atoms 5.1x in favour of phased.
-  static constexpr int kPhasedMeanAtoms = 5000;
-  static constexpr size_t kBranchReplicas = 64;
+  // AUTO: the branches for replicas of kBranchMean atoms or more on average, where
+  // the phased force launches wait for every replica's rebuild, and for smaller
+  // ones of kBranchRatio atoms or more per replica of the batch: a graph of many
+  // small branches is bound by node scheduling, and its launches overlap best
+  // where each is long and they are few.  Batches of up to kAlwaysPhased small
+  // replicas keep the phased graph, which is what they have always had, although
+  // the branches are some 8 % faster there.  Measured, B200, us a step, phased /
+  // branches, sizes within 30 % of the mean:
+  //   replicas    4         8         16        24        32        48         64         96
+  //   1,000     81/75   113/98    155/152   204/209   255/279   343/434    423/597    584/1038
+  //   2,000    100/90   143/123   241/212   320/294   392/375   520/535    680/717    972/1150
+  //   4,000   132/124   218/183   361/308   476/425   598/538   845/765   1077/1003
+  // and 910 x 2,000 5.1x in favour of phased, 91 x 20,000 1.2x in favour of branches.
+  static constexpr int kBranchMean = 5000;
+  static constexpr int kBranchRatio = 50;
+  static constexpr long long kAlwaysPhased = 5;
   int capture() {
     long long atoms = 0;
     for (rbx_engine* e : eng) atoms += e->n;
-    const bool small = atoms < (long long)kPhasedMeanAtoms * (long long)eng.size() &&
-                       (eng.size() <= 8 || eng.size() > kBranchReplicas);
+    const long long k = (long long)eng.size();
+    const bool small = atoms < kBranchMean * k && (k <= kAlwaysPhased || atoms < kBranchRatio * k * k);
     if (mode == RBX_BATCH_PHASED || (mode == RBX_BATCH_AUTO && small)) {
       const int rc = capture_phased();
       if (rc == RBX_OK || mode == RBX_BATCH_PHASED) return rc;
