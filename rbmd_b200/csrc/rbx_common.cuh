@@ -205,4 +205,11 @@ void count_launch(int n = 1);
 int check_launch(const char* what);
 int grid_for(long long work, int per_block, int max_blocks = 1 << 30);
 int sm_count();
+// a / b from rb, an approximation of 1 / b good to a few ulp: one step with the
+// exact residual (Markstein 1990) leaves the quotient's own rounding.
+__device__ __forceinline__ double quotient(double a, double b, double rb) {
+  const double q = a * rb;
+  return fma(fma(-q, b, a), rb, q);
+}
+
 }  // namespace rbx

@@ -37,21 +37,16 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 }
 
 
-// LJ 12-6 force/r (lj126_rs, src/force/src/lj_op/rocm/lj_op.hip.cu:40-54) in FP64.
-__device__ __forceinline__ double lj_f64(double eps_ij, double s6, double d2) {
-  const double r2i = 1.0 / d2;
-  const double sd6 = s6 * (r2i * r2i * r2i);
-  return -24.0 * eps_ij * ((2.0 * sd6 - 1.0) * sd6) * r2i;
-}
-// erfc-Coulomb force/r (CoulCutForce_rs_fix, lj_cut_coul_kspace_op.hip.cu:134-161).
+// erfc-Coulomb force/r (CoulCutForce_rs_fix, lj_cut_coul_kspace_op.hip.cu:134-161),
+// r2i = 1 / d2.
 __device__ __forceinline__ double coul_f64(double alpha, double sqrt_alpha, double qqr2e,
-                                           double qq, double d2) {
+                                           double qq, double d2, double r2i) {
   const double rinv = rsqrt(d2), dis = d2 * rinv;
   // erfc(x) = erfcx(x) exp(-x^2): one exponential serves both terms
   const double ex = exp(-alpha * d2);
   const double g = ex * (erfcx(sqrt_alpha * dis) * rinv +
                          (2.0 / 1.7724538509055160273) * sqrt_alpha);
-  return -qqr2e * qq * g * (rinv * rinv);
+  return quotient(-qqr2e * qq * g, d2, r2i);
 }
 __device__ __forceinline__ float lj_f32(float eps_ij, float s6, float d2) {
   const float d6 = d2 * d2 * d2;
@@ -321,10 +316,11 @@ __device__ __forceinline__ void rbl_fused_body(
         const double d2 =
             __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
         const bool ok = !(c & QF_CHECK) || classify_exact(d2, pp).shell_window;
-        double f = lj_f64(tt.eps[ti * nt + tj], tt.s6[ti * nt + tj], d2);
+        const double r2i = 1.0 / d2;
+        double f = lj_term(tt.eps[ti * nt + tj], tt.s6[ti * nt + tj], d2, r2i).f;
         if (qi != (T)0) {  // the whole warp works on atom i
           const double qq = (double)qi * __ldg(q + j);
-          if (qq != 0.0) f += coul_f64(pp.alpha, pp.sqrt_alpha, pp.qqr2e, qq, d2);
+          if (qq != 0.0) f += coul_f64(pp.alpha, pp.sqrt_alpha, pp.qqr2e, qq, d2, r2i);
         }
         if (c < 0) f *= (double)freq_t;
         f = ok ? f : 0.0;
@@ -557,14 +553,16 @@ k_verlet_fused_f64(PairParams pp, int n, const uint4* __restrict__ atoms,
       const double qq = qi * __ldg(q + j);
       const double e_ij = tt.eps[pt];
       const double r2i = 1.0 / d2;
-      const double sd6 = tt.s6[pt] * (r2i * r2i * r2i);
-      double f = -24.0 * e_ij * ((2.0 * sd6 - 1.0) * sd6) * r2i;
-      e_lj += 0.5 * (4.0 * e_ij * (sd6 - 1.0) * sd6);
+      const LjTerm lj = lj_term(e_ij, tt.s6[pt], d2, r2i);
+      double f = lj.f;
+      e_lj += 0.5 * (4.0 * e_ij * (lj.sd6 - 1.0) * lj.sd6);
       if (qq != 0.0) {
-        const double rinv = rsqrt(d2), ec = erfc(pp.sqrt_alpha * (d2 * rinv));
+        // erfc(x) = erfcx(x) exp(-x^2), whose error does not grow with the
+        // argument's as erfc's own does; coincident atoms keep their infinite energy
+        const double rinv = rsqrt(d2), ex = exp(-pp.alpha * d2);
+        const double ec = ex * erfcx(pp.sqrt_alpha * (d2 == 0.0 ? 0.0 : d2 * rinv));
         f += -pp.qqr2e * qq *
-             (ec * rinv + (2.0 / 1.7724538509055160273) * pp.sqrt_alpha * exp(-pp.alpha * d2)) *
-             (rinv * rinv);
+             (ec * rinv + (2.0 / 1.7724538509055160273) * pp.sqrt_alpha * ex) * r2i;
         e_c += pp.qqr2e * (0.5 * qq * ec * rinv);
       }
       const double gx = f * dx, gy = f * dy, gz = f * dz;
@@ -875,9 +873,11 @@ k_ref_rbl_filter(T core2, T force2, int n, const int* __restrict__ gid,
               required);
 }
 
+// v^6; the rounding of v^2, which the cube would triple, is put back (exact for
+// floats, whose squares are).
 __device__ __forceinline__ double pow6(double v) {
-  const double v2 = v * v;
-  return v2 * v2 * v2;
+  const double v2 = v * v, v4 = v2 * v2;
+  return fma(3.0 * fma(v, v, -v2), v4, v4 * v2);
 }
 
 // Pair vector r_j - r_i in T with the minimum image, and its r^2 as the
@@ -924,9 +924,10 @@ k_ref_pair_rbl(RefLen<T> b, T rs, T rc, int n, int pice, double alpha, double sq
     if (p.d2 < rs2 && p.d2 > eps_t) {
       const double dx = p.dx, dy = p.dy, dz = p.dz, d2 = dx * dx + dy * dy + dz * dz;
       const double sij = (si + (double)sigma[type[j]]) / 2, eij = sqrt(ei * (double)eps[type[j]]);
-      double f = lj_f64(eij, pow6(sij), d2);
+      const double r2i = 1.0 / d2;
+      double f = lj_term(eij, pow6(sij), d2, r2i).f;
       const double qq = qi * (double)q[j];
-      if (qq != 0.0) f += coul_f64(alpha, sqa, qqr2e, qq, d2);
+      if (qq != 0.0) f += coul_f64(alpha, sqa, qqr2e, qq, d2, r2i);
       s[0] += f * dx;
       s[1] += f * dy;
       s[2] += f * dz;
@@ -938,9 +939,10 @@ k_ref_pair_rbl(RefLen<T> b, T rs, T rc, int n, int pice, double alpha, double sq
     if (p.d2 < rc2 && p.d2 > rs2) {
       const double dx = p.dx, dy = p.dy, dz = p.dz, d2 = dx * dx + dy * dy + dz * dz;
       const double sij = (si + (double)sigma[type[j]]) / 2, eij = sqrt(ei * (double)eps[type[j]]);
-      double f = lj_f64(eij, pow6(sij), d2);
+      const double r2i = 1.0 / d2;
+      double f = lj_term(eij, pow6(sij), d2, r2i).f;
       const double qq = qi * (double)q[j];
-      if (qq != 0.0) f += coul_f64(alpha, sqa, qqr2e, qq, d2);
+      if (qq != 0.0) f += coul_f64(alpha, sqa, qqr2e, qq, d2, r2i);
       f *= (double)pice;
       c[0] += f * dx;
       c[1] += f * dy;

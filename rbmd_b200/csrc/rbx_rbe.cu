@@ -127,7 +127,8 @@ __device__ __forceinline__ void rbe_group_samples(const SampleArgs& sa, int p, i
 
 template <int KPT>
 __global__ void __launch_bounds__(RBE_BLOCK)
-k_rbe_rho_partial_f64(int n, int p, int chunk, double Lx, double Ly, double Lz,
+k_rbe_rho_partial_f64(int n, int p, int chunk, double Lx, double Ly, double Lz, double rLx,
+                      double rLy, double rLz,
                       const double* __restrict__ mx, const double* __restrict__ my,
                       const double* __restrict__ mz, const double* __restrict__ q,
                       const double* __restrict__ x, const double* __restrict__ y,
@@ -141,13 +142,14 @@ k_rbe_rho_partial_f64(int n, int p, int chunk, double Lx, double Ly, double Lz,
   const int kbase = blockIdx.y * (32 * KPT);
   if (sa.tables) rbe_group_samples<KPT>(sa, p, kbase, s_m, blockIdx.x == 0);
   // the block's k-vectors, k = 2 pi m / L evaluated as (2 pi * m) / L like the
-  // reference: a division a thread or two, where each warp's own took a fifth of
-  // the kernel at 400 vectors
+  // reference (rL = 1 / L): formed once, since every warp's own took a fifth of the
+  // kernel at 400 vectors
   for (int t = threadIdx.x; t < 96 * KPT; t += RBE_BLOCK) {
     const int d = t / (32 * KPT), s = t % (32 * KPT);
     const double* const m = d == 0 ? mx : (d == 1 ? my : mz);
     const double md = sa.tables ? (double)s_m[d][s] : (kbase + s < p ? m[kbase + s] : 0.0);
-    s_k[d][s] = (2 * RBX_PI * md) / (d == 0 ? Lx : (d == 1 ? Ly : Lz));
+    s_k[d][s] = quotient(2 * RBX_PI * md, d == 0 ? Lx : (d == 1 ? Ly : Lz),
+                         d == 0 ? rLx : (d == 1 ? rLy : rLz));
   }
   __syncthreads();
   double kx[KPT], ky[KPT], kz[KPT], sr[KPT], si[KPT];
@@ -1166,9 +1168,9 @@ int launch_rbe_rho_partial_f64(const DBox& b, int n, int p, const double* mx, co
   dim3 grid(nblocks, (p + 32 * kpt - 1) / (32 * kpt));
   const SampleArgs sa = sample ? *sample : SampleArgs{};
 #define RHO_F64(K)                                                                             \
-  k_rbe_rho_partial_f64<K><<<grid, RBE_BLOCK, 0, st>>>(n, p, chunk, b.len[0], b.len[1],       \
-                                                       b.len[2], mx, my, mz, q, x, y, z,       \
-                                                       part_re, part_im, sa)
+  k_rbe_rho_partial_f64<K><<<grid, RBE_BLOCK, 0, st>>>(                                        \
+      n, p, chunk, b.len[0], b.len[1], b.len[2], 1.0 / b.len[0], 1.0 / b.len[1],               \
+      1.0 / b.len[2], mx, my, mz, q, x, y, z, part_re, part_im, sa)
   switch (kpt) {
     case 1: RHO_F64(1); break;
     case 2: RHO_F64(2); break;

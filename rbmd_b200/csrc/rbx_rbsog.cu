@@ -261,15 +261,14 @@ k_verlet_sog(SogPairParams sp, int n, const double* __restrict__ x, const double
       const int pt = ti * sp.ntypes + type[j];
       const double eps = sp.lj_eps[pt], s6 = sp.lj_s6[pt];
       const double r2inv = 1.0 / d2, rinv = rsqrt(d2), r3inv = rinv * r2inv;
-      const double sd6 = s6 * (r2inv * r2inv * r2inv);
-      const double flj = -24 * eps * ((2 * sd6 - 1) * sd6) * r2inv;
+      const LjTerm lj = lj_term(eps, s6, d2, r2inv);
       const double pre = sp.qqr2e * qi * q[j];
       const double poly =
           sp.taylor[0] +
           d2 * (sp.taylor[1] +
                 d2 * (sp.taylor[2] + d2 * (sp.taylor[3] + d2 * (sp.taylor[4] + d2 * sp.taylor[5]))));
       const double fcl = -pre * (r3inv + poly);
-      const double fp = flj + fcl;
+      const double fp = lj.f + fcl;
       f[0] += fp * dx;
       f[1] += fp * dy;
       f[2] += fp * dz;
@@ -282,7 +281,7 @@ k_verlet_sog(SogPairParams sp, int n, const double* __restrict__ x, const double
         v[5] += -0.5 * dy * dz * fp;
       }
       if (ENERGY) {
-        elj += 0.5 * (4 * eps * (sd6 - 1) * sd6);
+        elj += 0.5 * (4 * eps * (lj.sd6 - 1) * lj.sd6);
         double sume = sp.norm * sp.w0 * exp(-d2 / (2.0 * sp.sigma * sp.sigma));
         double bl = 1.0;
         for (int l = 1; l < sp.mmax; ++l) {
@@ -323,8 +322,10 @@ k_verlet_sog(SogPairParams sp, int n, const double* __restrict__ x, const double
 // and short-range SOG terms are FP32 (cut decided on the FP32 r^2), each lane
 // sums its pairs in FP32 and the warp reduces in FP64.  Four candidates a lane
 // are loaded before any is used, and the reciprocal is the fast one with a
-// Newton step (the division's slow path kept the loop from overlapping): 134 ->
-// 76 us at 50,021 atoms, 485 candidates an atom (twelve blocks an SM; 78 at ten).
+// Newton step (the division's slow path kept the loop from overlapping): the
+// correctly rounded one for every float from 2^-20 to 2^20, all of them compared
+// on the device.  134 -> 76 us at 50,021 atoms, 485 candidates an atom (twelve
+// blocks an SM; 78 at ten).
 __global__ void __launch_bounds__(SOG_PAIR_BLOCK, 12)
 k_verlet_sog_mixed(SogPairParams sp, float sfx, float sfy, float sfz, int n,
                    const uint4* __restrict__ atoms, const int* __restrict__ type,
