@@ -205,6 +205,16 @@ void count_launch(int n = 1);
 int check_launch(const char* what);
 int grid_for(long long work, int per_block, int max_blocks = 1 << 30);
 int sm_count();
+// 1 / x to an ulp for x whose reciprocal is a normal number: the hardware's 20-bit
+// approximation and one third-order Newton step.  A division's slow path would cost
+// the pair kernels registers; what needs a rounded quotient corrects it (quotient).
+__device__ __forceinline__ double reciprocal(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
 // a / b from rb, an approximation of 1 / b good to a few ulp: one step with the
 // exact residual (Markstein 1990) leaves the quotient's own rounding.
 __device__ __forceinline__ double quotient(double a, double b, double rb) {

@@ -316,7 +316,7 @@ __device__ __forceinline__ void rbl_fused_body(
         const double d2 =
             __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
         const bool ok = !(c & QF_CHECK) || classify_exact(d2, pp).shell_window;
-        const double r2i = 1.0 / d2;
+        const double r2i = reciprocal(d2);
         double f = lj_term(tt.eps[ti * nt + tj], tt.s6[ti * nt + tj], d2, r2i).f;
         if (qi != (T)0) {  // the whole warp works on atom i
           const double qq = (double)qi * __ldg(q + j);
@@ -552,7 +552,7 @@ k_verlet_fused_f64(PairParams pp, int n, const uint4* __restrict__ atoms,
       const int pt = ti * nt + __ldg(type + j);
       const double qq = qi * __ldg(q + j);
       const double e_ij = tt.eps[pt];
-      const double r2i = 1.0 / d2;
+      const double r2i = reciprocal(d2);
       const LjTerm lj = lj_term(e_ij, tt.s6[pt], d2, r2i);
       double f = lj.f;
       e_lj += 0.5 * (4.0 * e_ij * (lj.sd6 - 1.0) * lj.sd6);
@@ -924,7 +924,7 @@ k_ref_pair_rbl(RefLen<T> b, T rs, T rc, int n, int pice, double alpha, double sq
     if (p.d2 < rs2 && p.d2 > eps_t) {
       const double dx = p.dx, dy = p.dy, dz = p.dz, d2 = dx * dx + dy * dy + dz * dz;
       const double sij = (si + (double)sigma[type[j]]) / 2, eij = sqrt(ei * (double)eps[type[j]]);
-      const double r2i = 1.0 / d2;
+      const double r2i = reciprocal(d2);
       double f = lj_term(eij, pow6(sij), d2, r2i).f;
       const double qq = qi * (double)q[j];
       if (qq != 0.0) f += coul_f64(alpha, sqa, qqr2e, qq, d2, r2i);
@@ -939,7 +939,7 @@ k_ref_pair_rbl(RefLen<T> b, T rs, T rc, int n, int pice, double alpha, double sq
     if (p.d2 < rc2 && p.d2 > rs2) {
       const double dx = p.dx, dy = p.dy, dz = p.dz, d2 = dx * dx + dy * dy + dz * dz;
       const double sij = (si + (double)sigma[type[j]]) / 2, eij = sqrt(ei * (double)eps[type[j]]);
-      const double r2i = 1.0 / d2;
+      const double r2i = reciprocal(d2);
       double f = lj_term(eij, pow6(sij), d2, r2i).f;
       const double qq = qi * (double)q[j];
       if (qq != 0.0) f += coul_f64(alpha, sqa, qqr2e, qq, d2, r2i);
