@@ -50,11 +50,11 @@ sys.path.insert(0, ROOT)
 METRIC = "RBE+LJ atom-steps/s @200k atoms: mixed vs FP64 plain at <=1e-5 rel force err"
 UNIT = "atom-steps/s"
 # DRAM bytes (read + written) per atom of one mixed k_rbl_fused launch, from an ncu
-# capture of the same workload at N = 100,000 (215.1 MB per launch: the split candidate
+# capture of the same workload at N = 100,003 (212.0 MB per launch: the split candidate
 # rows streamed once, plus neighbour-record and key gathers that miss L2).  Rows and
 # gathers grow with N, so the traffic is scaled by N.
-RBL_TRAFFIC_BYTES_PER_ATOM = 2151.0
-# Warp instructions per 32 candidates of one launch (175.7 M for 47.8 M candidates in a
+RBL_TRAFFIC_BYTES_PER_ATOM = 2120.0
+# Warp instructions per 32 candidates of one launch (175.6 M for 47.8 M candidates in a
 # capture at N = 100,003), and the SM issue limit they are compared with: one warp
 # instruction per cycle per SM sub-partition, four per SM.
 RBL_WARP_INSTR_PER_32_CAND = 117.5

@@ -238,7 +238,8 @@ struct rbx_batch {
     long long atoms = 0;
     for (rbx_engine* e : eng) atoms += e->n;
     const long long k = (long long)eng.size();
-    const bool small = atoms < kBranchMean * k && (k <= kAlwaysPhased || atoms < kBranchRatio * k * k);
+    const bool small =
+        atoms < kBranchMean * k && (k <= kAlwaysPhased || atoms < kBranchRatio * k * k);
     if (mode == RBX_BATCH_PHASED || (mode == RBX_BATCH_AUTO && small)) {
       const int rc = capture_phased();
       if (rc == RBX_OK || mode == RBX_BATCH_PHASED) return rc;

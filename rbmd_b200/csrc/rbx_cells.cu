@@ -253,14 +253,17 @@ k_cell_segsort(int ncell, int n, const int* __restrict__ start, const unsigned* 
 // count[i] is the number of candidates (above cap: overflow), far[i] the
 // number of far ones; a row that overflows holds some cap of its candidates.
 //
-// Bound by instruction issue.  Four centres a warp and four-atom chunks leave
-// about 1,400 tested slots an atom at rho* = 0.8, cutoff 5.3 (499 hits),
-// against 3,700 when one warp tests 32-atom chunks against 32 centres, one a
-// lane, as an earlier builder did; and a small box fills the chip (that
-// builder ran one warp per 32 atoms through all 27 cells).  Measured, B200,
-// rho* = 0.8, cutoff 5.3, that builder and this one: 200,000 atoms 660 and
-// 466 us (split rows 915 and 614), 20,000 atoms split 214 and 92, 4,000 atoms
-// split 171 and 42.
+// Bound by issue and by the barriers between a block's phases: 70 % of the issue
+// slots are taken (split rows 74 %) with half of the warp slots (64 registers,
+// 52 KB: four blocks an SM), and of the ten cycles a warp spends on an instruction
+// 2.3 are waits at a barrier, the largest share.  An append in half its
+// instructions was no faster.  Four centres a warp and four-atom chunks leave
+// about 1,400 tested slots an atom at rho* = 0.8, cutoff 5.3 (499 hits; 1,860 warp
+// instructions, 2,350 with split rows), against 3,700 slots when one warp tests
+// 32-atom chunks against 32 centres, one a lane; and a small box fills the chip.
+// Measured, B200, rho* = 0.8, cutoff 5.3, one warp per 32 centres and this:
+// 200,000 atoms 660 and 466 us (split rows 915 and 614), 20,000 atoms split 214
+// and 92, 4,000 atoms split 171 and 42.
 // ---------------------------------------------------------------------------
 // W, the warps of a block (centre atoms 4 W): eight, or one where cells hold a few
 // atoms, whose blocks would leave most of eight warps idle.
@@ -282,9 +285,10 @@ static size_t full_list_chunks(int n, int ncell) { return (size_t)(n / NL_CH) + 
 // atoms go to one-warp blocks (a second launch), the others to the eight-warp
 // blocks, as all do in a denser box: a gas and a droplet in a large box each get
 // the blocks that suit them.  The indices of the eight-warp groups are then
-// gathered first: a block that finds none costs 1 ns, and most would.  Measured, B200, us, eight warps / one for all cells:
-// 200,000 atoms of 0.3, 1, 3, 6 and 12 a cell 1779 / 545, 1252 / 556, 809 / 529,
-// 475 / 469, 314 / 508; 4,000 atoms of 1, 2, 3 and 6 32 / 20, 28 / 24, 22 / 25, 18 / 27.
+// gathered first: a block that finds none costs 1 ns, and most would.  Measured,
+// B200, us, eight warps / one for all cells: 200,000 atoms of 0.3, 1, 3, 6 and 12 a
+// cell 1779 / 545, 1252 / 556, 809 / 529, 475 / 469, 314 / 508; 4,000 atoms of 1, 2,
+// 3 and 6 32 / 20, 28 / 24, 22 / 25, 18 / 27.
 constexpr long long LIST_DILUTE = 3;
 constexpr int LIST_FEW = 6;
 static bool list_dilute(int n, int ncell) { return n < LIST_DILUTE * ncell; }
@@ -703,8 +707,9 @@ k_full_list(DBox b, int dimx, int dimy, int dimz, double cut2, float cut2_up, fl
 // |d|^2 in FP32 decides every pair outside a guard band (the RBL kernels'
 // bound) around the cutoff and around r_near; the FP64 distance settles the
 // rest.  Hits are appended in index order through a ballot prefix, far pairs (at
-// least r_near, see FarSplit) to the back.  Measured, B200, 1,000 / 1,500 / 3,000 atoms: 10.8 / 14.9 / 36.0 us;
-// 16.5 / 23.6 / 43.0 us with a warp an atom and FP64 distances.
+// least r_near, see FarSplit) to the back.  Measured, B200, 1,000 / 1,500 / 3,000
+// atoms: 10.8 / 14.9 / 36.0 us; 16.5 / 23.6 / 43.0 us with a warp an atom and FP64
+// distances.
 // ---------------------------------------------------------------------------
 constexpr int SL_WARPS = 8;
 constexpr int SL_C = 2;       // centre atoms of a warp
@@ -1178,8 +1183,8 @@ int launch_full_list(const DBox& b, const int dims[3], double cutoff, int n, con
   T.many = T.few_cell ? (int*)((char*)T.few_cell + piece[4]) : nullptr;
   // a thread an atom: 32 threads a cell up to some 60 atoms (200,000 atoms of 1 / 16 /
   // 120 a cell: 103 / 9 / 7 us, 128 threads 190 / 15 / 5)
-  k_chunk_boxes<<<ncell, n < 60LL * ncell ? 32 : 128, 0, st>>>(b, dims[0], dims[1], dims[2], x, y, z,
-                                                              cell_start, T);
+  k_chunk_boxes<<<ncell, n < 60LL * ncell ? 32 : 128, 0, st>>>(b, dims[0], dims[1], dims[2], x, y,
+                                                              z, cell_start, T);
   count_launch();
   // far threshold in r^2, raised by the FP32 error of the test value
   const float near2 = split ? (float)(split->r_near * split->r_near + band) : INFINITY;

@@ -151,17 +151,17 @@ __device__ __forceinline__ void write_block_partial(double (*s_acc)[3], double* 
 // pairs at a time from its tail.
 //
 // Bound by the latency of the gathers until the warp slots are full, then by
-// integer issue (mixed, 100,000 atoms: 95 % of the slots, 76 % issue), so resident
-// warps count more than registers: the mixed form fits eight blocks an SM (32
-// registers, no spills), the FP64 form six (40, a few spilled words that
+// integer issue (100,000 atoms, mixed: 95 % of the slots, 79 % issue; FP64 73 and
+// 77 %), so resident warps count more than registers: the mixed form fits eight blocks an SM (32
+// registers, no spills), the FP64 form six (40, some spilled words that
 // stay in L1).  What keeps the registers down is that the warp index comes
 // through a shuffle: atom, row and loop state are then uniform.  Queue pushes
 // are predicated stores at ballot prefixes.  Measured, B200, 200,000-atom LJ
 // electrolyte: mixed 464 -> 390 us (four blocks of 64 registers, per-thread
 // state before; 415, 397, 389, 381, 378 at four to eight blocks with the far
-// segment queued in another order, below), FP64 697 -> 552 us (three blocks
-// before; 608, 568 at four and five); water, 73,000 atoms: 271 -> 247 and
-// 523 -> 370 us.
+// segment queued in another order, below), FP64 697 -> 565 us (three blocks
+// before; six take as long as five since the quotients' residual steps, 553 to
+// 565 us for those); water, 73,000 atoms: mixed 271 -> 247 us.
 //
 // The queue holds the pairs in row order: a lane's FP32 sums, and with them the
 // mixed form's forces, then depend on the row alone.  Batches from the row's end

@@ -20,8 +20,8 @@ __device__ __forceinline__ double norm1(double x, double y, double z) {
 // rounded once.  Then polynomials in r^2 on |r| <= pi/4: the interpolants of
 // (sin(r) / r - 1) / r^2 and (cos(r) - 1) / r^2 at the six and seven Chebyshev
 // nodes of r^2 in [0, pi^2/16], computed in 60-digit arithmetic (truncation
-// 1.3e-17 and 1.2e-19 relative).  Some 20 FP64 instructions, where the library's sincos takes about 85, and FP64
-// issue bounds the passes that call it.
+// 1.3e-17 and 1.2e-19 relative).  Some 20 FP64 instructions, where the library's
+// sincos takes about 85, and FP64 issue bounds the passes that call it.
 __device__ __forceinline__ void sincos_phase(double t, double* s, double* c) {
   const double kShift = 6755399441055744.0;                 // 1.5 * 2^52
   const double b = fma(t, 0.6366197723675814, kShift);      // 2 / pi
