@@ -718,6 +718,7 @@ constexpr int SL_TILE = 1024; // atoms staged at a time
 struct SmallScreen {
   IntScreen cut, near;  // of the fixed-point |d|^2: list cutoff, near and far segment
   double cut2, near2;   // the same in FP64
+  float cut_mid, cut_half, near_mid, near_half;  // intervals that contain the bands
   float w[3];           // L_d / L_max
 };
 
@@ -758,8 +759,9 @@ k_full_list_small(DBox b, SmallScreen sc, int n, const uint4* __restrict__ atoms
                     dy = (float)(int)(v.y - u[q].y) * sc.w[1],
                     dz = (float)(int)(v.z - u[q].z) * sc.w[2];
         d2[q] = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-        odd |= (d2[q] >= sc.cut.lo) & (d2[q] < sc.cut.hi);
-        if (SPLIT) odd |= (d2[q] >= sc.near.lo) & (d2[q] < sc.near.hi);
+        // either guard band (written as two subtractions: fewer predicates)
+        odd |= fabsf(d2[q] - sc.cut_mid) <= sc.cut_half;
+        if (SPLIT) odd |= fabsf(d2[q] - sc.near_mid) <= sc.near_half;
       }
       const bool settle = __any_sync(0xffffffffu, odd & there);
 #pragma unroll
@@ -818,6 +820,13 @@ int launch_full_list_small(const DBox& b, double cutoff, int n, const uint4* ato
   // pair that could come within r_core before the next rebuild to the far segment
   sc.near2 = split ? split->r_near * split->r_near * (1.0 + 1e-9) : 0.0;
   sc.near = make_screen(sc.near2, L, 1e-4 + 8e-6 * sc.near2 + qerr);
+  // a little wider than the bands, which decide
+  auto around = [](const IntScreen& s, float* mid, float* half) {
+    *mid = 0.5f * (s.lo + s.hi);
+    *half = 0.5f * (s.hi - s.lo) + 1e-6f * s.hi;
+  };
+  around(sc.cut, &sc.cut_mid, &sc.cut_half);
+  around(sc.near, &sc.near_mid, &sc.near_half);
   for (int d = 0; d < 3; ++d) sc.w[d] = (float)(b.len[d] / L);
   const int per_block = SL_WARPS * SL_C;
   const auto kern = split ? k_full_list_small<true> : k_full_list_small<false>;
